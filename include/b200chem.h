@@ -350,10 +350,11 @@ int b200chem_selftest_bounded_wait(int* err, int polls, void* stream);
 enum {
   B200CHEM_PROF_START = 0,       /* rk_start: load, validate, initialise   */
   B200CHEM_PROF_RHS = 1,         /* rk_rhs: right-hand sides               */
-  B200CHEM_PROF_CTRL = 2,        /* rk_ctrl after the right-hand sides     */
+  B200CHEM_PROF_CTRL = 2,        /* rk_step after the right-hand sides     */
   B200CHEM_PROF_JAC = 3,         /* rk_jac: analytic Jacobians             */
   B200CHEM_PROF_GJ = 4,          /* rk_gj: Newton-matrix inverses          */
-  B200CHEM_PROF_CTRL_SETUP = 5,  /* rk_ctrl after a setup                  */
+  B200CHEM_PROF_CTRL_SETUP = 5,  /* rk_step after a setup                  */
+  B200CHEM_PROF_CTRL_RARE = 6,   /* rk_ctrl: starts, failures, ends        */
   B200CHEM_PROF_KINDS = 8
 };
 typedef struct b200chem_kernel_profile {

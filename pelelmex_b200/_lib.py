@@ -79,7 +79,7 @@ class Tuning(ctypes.Structure):
                 ("reserved", ctypes.c_int32)]
 
 
-PROF_KINDS = ("start", "rhs", "ctrl", "jac", "gj", "ctrl_setup")
+PROF_KINDS = ("start", "rhs", "ctrl", "jac", "gj", "ctrl_setup", "ctrl_rare")
 
 
 class KernelProfile(ctypes.Structure):

@@ -416,10 +416,6 @@ int tuned_grid(int max_grid, int sm_count, int per_sm) {
   return std::max(sm_count, std::min(max_grid, per_sm * sm_count));
 }
 
-// One round of the integrator: right-hand sides of the cells in list_in,
-// step control (Newton update, error test, next prediction) appending to
-// list_out and to the setup list, Jacobian and iteration-matrix inversion of
-// the setup list, step control of the cells back from their setup.
 constexpr int kProfCountSlots = 1 << 16;
 
 cudaEvent_t prof_event(b200chem_reactor* h) {
@@ -435,15 +431,15 @@ cudaEvent_t prof_event(b200chem_reactor* h) {
 // bracketed by two events and the count of the list it processes is copied
 // to the host first (stream-ordered, so it is the count the kernel sees).
 int launch_kernel(b200chem_reactor* h, int lut, int what, int prof_kind, const RoundsParams& R, const RoundsGrids& G,
-                  int after_rhs, const int* cnt, long long host_cells, cudaStream_t st) {
+                  int setup_pass, const int* cnt, long long host_cells, cudaStream_t st) {
   if (!h->prof_on || h->prof_overflow) {
-    CK(rounds_launch(h->N, lut, what, R, G, after_rhs, st));
+    CK(rounds_launch(h->N, lut, what, R, G, setup_pass, st));
     return 0;
   }
   b200chem_reactor::ProfRec rec{prof_kind, -1, host_cells, prof_event(h), prof_event(h)};
   if (!rec.e0 || !rec.e1 || (cnt && h->pcnt_used >= kProfCountSlots)) {
     h->prof_overflow = true;
-    CK(rounds_launch(h->N, lut, what, R, G, after_rhs, st));
+    CK(rounds_launch(h->N, lut, what, R, G, setup_pass, st));
     return 0;
   }
   if (cnt) {
@@ -451,52 +447,48 @@ int launch_kernel(b200chem_reactor* h, int lut, int what, int prof_kind, const R
     CK(cudaMemcpyAsync(h->h_pcnt + rec.slot, cnt, sizeof(int), cudaMemcpyDeviceToHost, st));
   }
   CK(cudaEventRecord(rec.e0, st));
-  CK(rounds_launch(h->N, lut, what, R, G, after_rhs, st));
+  CK(rounds_launch(h->N, lut, what, R, G, setup_pass, st));
   CK(cudaEventRecord(rec.e1, st));
   h->prof.push_back(rec);
   return 0;
 }
 
-// The slot lists of one chunk: A and B (cells needing a right-hand side,
-// swapped every round), S (cells needing a Newton-matrix setup) and its
-// subset SJ (setups that recompute the Jacobian).
+// The slot lists of one chunk and their counters (the kRl* indices): two sets
+// of those a round reads and the next one gets, swapped every round, and the
+// control kernel's list, whose counter lies in the set written.
 struct RoundLists {
-  int* lst[2];
+  int* lst[2][kRoundLists];
   int* cnt[2];
-  int* setup;
-  int* cnt_setup;
-  int* jac;
-  int* cnt_jac;
 };
 
+// One round of the integrator: right-hand sides of the live cells (list A);
+// Newton correction and step of those that keep their Newton matrix; Jacobian
+// and inverse of the others, then their step; the control kernel for whatever
+// the step kernel passed on.  Every kernel appends to the lists of the next
+// round, whose counters the right-hand-side kernel clears.
 int enqueue_round(b200chem_reactor* h, int lut, RoundsParams R, const RoundsGrids& G, const RoundLists& Ls, int cur,
                   cudaStream_t st) {
-  R.list_in = Ls.lst[cur];
-  R.cnt_in = Ls.cnt[cur];
-  R.list_out = Ls.lst[1 - cur];
-  R.cnt_out = Ls.cnt[1 - cur];
-  R.list_setup = Ls.setup;
-  R.cnt_setup = Ls.cnt_setup;
-  R.list_jac = Ls.jac;
-  R.cnt_jac = Ls.cnt_jac;
-  int err = launch_kernel(h, lut, kRoundsRhs, B200CHEM_PROF_RHS, R, G, 0, R.cnt_in, 0, st);
-  if (err) return err;
-  CK(cudaMemsetAsync(R.cnt_out, 0, sizeof(int), st));
-  CK(cudaMemsetAsync(Ls.cnt_setup, 0, sizeof(int), st));
-  CK(cudaMemsetAsync(Ls.cnt_jac, 0, sizeof(int), st));
-  if ((err = launch_kernel(h, lut, kRoundsCtrl, B200CHEM_PROF_CTRL, R, G, 1, R.cnt_in, 0, st))) return err;
-  R.list_in = Ls.jac;
-  R.cnt_in = Ls.cnt_jac;
-  if ((err = launch_kernel(h, lut, kRoundsJac, B200CHEM_PROF_JAC, R, G, 0, Ls.cnt_jac, 0, st))) return err;
-  R.list_in = Ls.setup;
-  R.cnt_in = Ls.cnt_setup;
-  if ((err = launch_kernel(h, lut, kRoundsGj, B200CHEM_PROF_GJ, R, G, 0, Ls.cnt_setup, 0, st))) return err;
-  // cells coming back from a setup always ask for a right-hand side next
-  return launch_kernel(h, lut, kRoundsCtrl, B200CHEM_PROF_CTRL_SETUP, R, G, 0, Ls.cnt_setup, 0, st);
+  const int* cnt = Ls.cnt[cur];
+  R.cnt_next = Ls.cnt[1 - cur];
+  for (int k = 0; k < kRoundLists; ++k) R.list[k] = Ls.lst[1 - cur][k];
+  const struct { int what, kind, setup_pass, in; const int* c; const int* list; } seq[6] = {
+      {kRoundsRhs, B200CHEM_PROF_RHS, 0, kRlRhs, cnt, Ls.lst[cur][kRlRhs]},
+      {kRoundsStep, B200CHEM_PROF_CTRL, 0, kRlRhs, cnt, Ls.lst[cur][kRlRhs]},
+      {kRoundsJac, B200CHEM_PROF_JAC, 0, kRlJac, cnt, Ls.lst[cur][kRlJac]},
+      {kRoundsGj, B200CHEM_PROF_GJ, 0, kRlSetup, cnt, Ls.lst[cur][kRlSetup]},
+      {kRoundsStep, B200CHEM_PROF_CTRL_SETUP, 1, kRlSetup, cnt, Ls.lst[cur][kRlSetup]},
+      {kRoundsCtrl, B200CHEM_PROF_CTRL_RARE, 0, kRlCtrl, R.cnt_next, Ls.lst[1 - cur][kRlCtrl]}};
+  for (const auto& k : seq) {
+    R.list_in = k.list;
+    R.cnt_in = k.c + k.in;
+    const int err = launch_kernel(h, lut, k.what, k.kind, R, G, k.setup_pass, R.cnt_in, 0, st);
+    if (err) return err;
+  }
+  return 0;
 }
 
-// Captures `rounds` rounds (an even number: the two slot lists swap roles
-// every round, so the graph starts and ends on list A) into h->rgraph,
+// Captures `rounds` rounds (an even number: the two sets of lists swap roles
+// every round, so the graph starts and ends on the same one) into h->rgraph,
 // updating the executable graph in place when only kernel parameters
 // changed.
 int capture_rounds(b200chem_reactor* h, int lut, const RoundsParams& R, const RoundsGrids& G, int rounds,
@@ -551,6 +543,7 @@ int launch_rounds(b200chem_reactor* h, const ReactParams& P, cudaStream_t st, in
   const b200chem_tuning& T = h->tune;
   RoundsGrids G = h->rgrid;
   G.rhs = tuned_grid(h->rgrid.rhs, h->sm_count, T.rhs_ctas_per_sm);
+  G.step = tuned_grid(h->rgrid.step, h->sm_count, T.ctrl_ctas_per_sm);
   G.ctrl = tuned_grid(h->rgrid.ctrl, h->sm_count, T.ctrl_ctas_per_sm);
   G.jac = tuned_grid(h->rgrid.jac, h->sm_count, T.jac_ctas_per_sm);
   G.gj = tuned_grid(h->rgrid.gj, h->sm_count, T.gj_ctas_per_sm);
@@ -571,27 +564,24 @@ int launch_rounds(b200chem_reactor* h, const ReactParams& P, cudaStream_t st, in
                       "setup scratch");
   if (err) return err;
   if (!h->d_rcnt) {
-    CK(cudaMalloc(&h->d_rcnt, 4 * sizeof(int)));
+    CK(cudaMalloc(&h->d_rcnt, 2 * kRoundLists * sizeof(int)));
     CK(cudaMallocHost(&h->h_rcnt, sizeof(int)));
   }
   RoundsParams R;
   R.P = P;
   R.SL = SL;
   R.S = rounds_carve(h->d_rounds, cap, h->N, lut);
-  // the four slot lists follow the cell records
+  // the slot lists follow the cell records
   const size_t rec_bytes = (size_t)R.S.L.stride * cap;
-  if (rec_bytes + 16ull * cap > h->rounds_bytes)
+  if (rec_bytes + 4ull * kRoundSlotLists * cap > h->rounds_bytes)
     return set_err(B200CHEM_ECUDA, "round-integrator state layout overflows its buffer");
   int* lists = reinterpret_cast<int*>(static_cast<unsigned char*>(h->d_rounds) + rec_bytes);
   RoundLists Ls;
-  Ls.lst[0] = lists;
-  Ls.lst[1] = lists + cap;
-  Ls.setup = lists + 2 * cap;
-  Ls.jac = lists + 3 * cap;
-  Ls.cnt[0] = h->d_rcnt;
-  Ls.cnt[1] = h->d_rcnt + 1;
-  Ls.cnt_setup = h->d_rcnt + 2;
-  Ls.cnt_jac = h->d_rcnt + 3;
+  for (int b = 0; b < 2; ++b) {
+    for (int k = 0; k < kRlCtrl; ++k) Ls.lst[b][k] = lists + (b * kRlCtrl + k) * cap;
+    Ls.lst[b][kRlCtrl] = lists + 2 * kRlCtrl * cap;
+    Ls.cnt[b] = h->d_rcnt + b * kRoundLists;
+  }
   R.wscratch = static_cast<unsigned char*>(h->d_rwarp);
   // right-hand-side form: generated mechanism code, the constant bank or the
   // global tables
@@ -602,15 +592,11 @@ int launch_rounds(b200chem_reactor* h, const ReactParams& P, cudaStream_t st, in
   for (long long chunk0 = 0; chunk0 < P.total; chunk0 += cap) {
     R.chunk0 = chunk0;
     R.nchunk = std::min<long long>(cap, P.total - chunk0);
-    CK(cudaMemsetAsync(h->d_rcnt, 0, 4 * sizeof(int), st));
+    CK(cudaMemsetAsync(h->d_rcnt, 0, 2 * kRoundLists * sizeof(int), st));
     R.list_in = nullptr;
     R.cnt_in = nullptr;
-    R.list_out = Ls.lst[0];
-    R.cnt_out = Ls.cnt[0];
-    R.list_setup = Ls.setup;
-    R.cnt_setup = Ls.cnt_setup;
-    R.list_jac = Ls.jac;
-    R.cnt_jac = Ls.cnt_jac;
+    R.cnt_next = Ls.cnt[0];
+    for (int k = 0; k < kRoundLists; ++k) R.list[k] = Ls.lst[0][k];
     err = launch_kernel(h, lut, kRoundsStart, B200CHEM_PROF_START, R, G, 0, nullptr, R.nchunk, st);
     if (err) return err;
     h->launches++;
@@ -628,9 +614,9 @@ int launch_rounds(b200chem_reactor* h, const ReactParams& P, cudaStream_t st, in
           if (err) return err;
         }
       }
-      h->launches += 5LL * per_check;
-      // per_check is even: the live cells are back in list A
-      CK(cudaMemcpyAsync(h->h_rcnt, Ls.cnt[0], sizeof(int), cudaMemcpyDeviceToHost, st));
+      h->launches += 6LL * per_check;
+      // per_check is even: the live cells are back in the first list
+      CK(cudaMemcpyAsync(h->h_rcnt, Ls.cnt[0] + kRlRhs, sizeof(int), cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));
       if (*h->h_rcnt == 0) break;
     }

@@ -39,22 +39,11 @@ struct CellCounters {
   int nst, nfe, nje, nlu, netf, ncfn, nni;
 };
 
-// In-place Gauss-Jordan inverse of A = D (I - gamma J) D^-1 (FP32, D = Dsc)
-// or A = I - gamma J (FP64).  J is column-major (J[col*ldj + row]); A is
-// row-major in shared memory.  Returns 0, or k+1 when pivot k is zero.
+// In-place Gauss-Jordan inverse of the matrix A, row-major in shared memory.
+// Returns 0, or k+1 when pivot k is zero.
 template <int G, typename LUT>
-__device__ __noinline__ int grp_gj_inverse(const double* J, int ldj, LUT* A, int ldl, int* ipiv, LUT* fcol,
-                                           const double* Dsc, int n, double gamma, int lane) {
+__device__ __noinline__ int grp_gj_eliminate(LUT* A, int ldl, int* ipiv, LUT* fcol, int n, int lane) {
   const Grp<G> g(lane);
-  constexpr bool kScaled = sizeof(LUT) == 4;
-  for (int j = g.gl; j < n; j += G) {
-    const double dj = kScaled ? Dsc[j] : 1.0;
-    for (int i = 0; i < n; ++i) {
-      const double mij = ((i == j) ? 1.0 : 0.0) - gamma * J[j * ldj + i];
-      A[i * ldl + j] = (LUT)(kScaled ? mij * Dsc[i] / dj : mij);
-    }
-  }
-  g.sync();
   for (int k = 0; k < n; ++k) {
     LUT best = (LUT)-1;
     int bi = k;
@@ -110,6 +99,24 @@ __device__ __noinline__ int grp_gj_inverse(const double* J, int ldj, LUT* A, int
     g.sync();
   }
   return 0;
+}
+
+// Inverse of A = D (I - gamma J) D^-1 (FP32, D = Dsc) or A = I - gamma J
+// (FP64).  J is column-major (J[col*ldj + row]); A as above.
+template <int G, typename LUT>
+__device__ __forceinline__ int grp_gj_inverse(const double* J, int ldj, LUT* A, int ldl, int* ipiv, LUT* fcol,
+                                              const double* Dsc, int n, double gamma, int lane) {
+  const Grp<G> g(lane);
+  constexpr bool kScaled = sizeof(LUT) == 4;
+  for (int j = g.gl; j < n; j += G) {
+    const double dj = kScaled ? Dsc[j] : 1.0;
+    for (int i = 0; i < n; ++i) {
+      const double mij = ((i == j) ? 1.0 : 0.0) - gamma * J[j * ldj + i];
+      A[i * ldl + j] = (LUT)(kScaled ? mij * Dsc[i] / dj : mij);
+    }
+  }
+  g.sync();
+  return grp_gj_eliminate<G, LUT>(A, ldl, ipiv, fcol, n, lane);
 }
 
 // x := D^-1 A D x  (A = scaled inverse; bvec is per-group shared scratch)

@@ -10,20 +10,24 @@
 //
 //   rhs kernel    one THREAD per cell: f(y) for every cell of the list (all
 //                 lanes walk the same reaction at the same time);
-//   ctrl kernel   one THREAD per cell: resumes the state machine below with
-//                 that f until the cell needs its next f, a setup, or is done;
-//   setup kernel  one WARP per cell: analytic Jacobian (FP64) and the
-//                 Gauss-Jordan inverse of D (I - gamma J) D^-1 (FP32);
-//   ctrl kernel   again for the cells that were set up.
+//   step kernel   8 or 16 lanes per cell: the Newton correction with that f
+//                 and, when it converges and passes the error test, the whole
+//                 way to the next prediction (g_newton, g_finish_step);
+//   jac, gj       one WARP per cell: analytic Jacobian (FP64) and the
+//                 Gauss-Jordan inverse of D (I - gamma J) D^-1 (FP32) for the
+//                 cells whose matrix is rebuilt (known since their prediction:
+//                 the step kernel passes over them), then the step kernel for
+//                 those cells;
+//   ctrl kernel   everything rarer (start of a cell, failures, its end): the
+//                 state machine r_advance.
 //
 // Each cell ("slot") owns one contiguous record in device memory: its
 // step-control scalars (RCell), its vectors (Nordsieck array, ewt, acor, ...)
 // and its two matrices (FP64 Jacobian and the scaled inverse of the Newton
-// matrix), both column-major.  A thread streams its own record sequentially,
-// so every 32-byte sector it touches is used whole whatever the order of the
-// cells in the work lists; a warp working on one cell reads a matrix column
-// as one coalesced transaction.
+// matrix) in the lanes' order (mat_idx).
 #pragma once
+#include <type_traits>
+
 #include "bdf_group.cuh"
 
 namespace b200 {
@@ -33,18 +37,19 @@ namespace rounds {
 enum Label : int {
   kLAfterF0 = 0,   // f(y0) evaluated
   kLAfterHin,      // f(y0 + hg y0') evaluated (initial step estimate)
-  kLAfterNStart,   // f(predicted y) evaluated: maybe setup, then Newton
+  kLAfterNStart,   // f(predicted y) evaluated: Newton
   kLAfterNIter,    // f(current Newton iterate) evaluated
   kLAfterRestart,  // f(y) after an order-1 restart
-  kLAfterSetup,    // Newton matrix rebuilt (setup_ier holds its status)
+  kLAfterSetup,    // f(predicted y) evaluated and Newton matrix rebuilt (setup_ier holds its status)
   // internal labels
-  kLStart, kLBeginStep, kLAttempt, kLNlsAttempt, kLNewtonIter, kLNlsRecover, kLNlsFail1, kLNlsFail2,
-  kLNlsSuccess
+  kLStart, kLBeginStep, kLAttempt, kLNlsAttempt, kLNlsRecover, kLNlsFail1, kLNlsFail2, kLNlsSuccess,
+  kLStall
 };
 
 // What the cell needs next.
-// kNeedSetupJac: a setup whose Jacobian is stale (CVODE's jbad rule) and is
-// recomputed first; kNeedSetup: a setup that reuses the stored Jacobian.
+// kNeedRhs: a right-hand side; kNeedSetup: that and a new Newton matrix from
+// the stored Jacobian; kNeedSetupJac: the same with a stale Jacobian (CVODE's
+// jbad rule), which is recomputed first.
 enum Need : int { kNeedRhs = 0, kNeedSetup = 1, kDone = 2, kNeedSetupJac = 3 };
 
 // Step-control record of one cell (doubles first, then ints), padded to a
@@ -62,24 +67,55 @@ struct alignas(16) RCell {
 };
 static_assert(sizeof(RCell) % 16 == 0, "RCell moves as 16-byte vectors");
 
+// Lanes per cell of the step and control kernels.
+#ifndef B200_CTRL_LANES
+#define B200_CTRL_LANES 8
+#endif
+__host__ __device__ constexpr int ctrl_group(int n) { return n <= 32 ? B200_CTRL_LANES : 16; }
+
+// A matrix of the record for lane groups of G: lane g owns rows g, g + G, ...
+// and reads V consecutive columns of one of its rows as one 16-byte vector;
+// the lanes of a group read consecutive vectors.  Rows come in blocks of G
+// (the last one as many as are left, so no row is padded), columns are padded
+// to a multiple of V.
+// mat_vec: offset of the vector of columns jb V .. jb V + V - 1 of row
+// cc G + g; mat_idx: offset of element (i, j).
+template <int n, int G, int V>
+__host__ __device__ __forceinline__ constexpr int mat_vec(int cc, int g, int jb) {
+  constexpr int JB = (n + V - 1) / V;
+  const int rows = (n - cc * G < G) ? n - cc * G : G;
+  return (cc * G * JB + jb * rows + g) * V;
+}
+template <int n, int G, int V>
+__host__ __device__ __forceinline__ constexpr int mat_idx(int i, int j) {
+  return mat_vec<n, G, V>(i / G, i % G, j / V) + j % V;
+}
+// columns per 16-byte vector of the Jacobian and of the inverse
+constexpr int kVJ = 2;
+template <typename LUT>
+__host__ __device__ constexpr int vec_of() { return 16 / (int)sizeof(LUT); }
+
+// Vectors of a record, in this order: what the step kernel reads (dsc, fv,
+// ewt, acor, the Nordsieck columns) directly after the scalars, then the
+// evaluation point and the forcing.
+enum RVecSlot : int { kVDsc = 0, kVFv, kVEwt, kVAcor, kVZn, kVYev = kVZn + kZn, kVF, kVecs };
+constexpr int kVecsRead = kVZn + kZn;
+
 // Byte layout of one cell record for n components and inverse type of
-// lut_bytes: [RCell][vectors (kZn + 7) n doubles][J: n columns of ldj
-// doubles][A: n columns of lda LUT], each part 16-byte aligned, the record
-// padded to 128 bytes.
+// lut_bytes: [RCell][kVecs vectors of n doubles][J][A], each part 16-byte
+// aligned, the record padded to 128 bytes.
 struct RLayout {
-  int ldj, lda;          // column strides (elements) of J and A
   int off_vec, off_j, off_a;
   long long stride;      // bytes per record
 };
 
 __host__ __device__ inline RLayout rounds_record_layout(int n, int lut_bytes) {
   RLayout L;
-  L.ldj = (n + 1) & ~1;                                  // 16-byte columns
-  L.lda = (lut_bytes == 4) ? ((n + 3) & ~3) : L.ldj;     // 16-byte columns
+  const int vj = (n + kVJ - 1) / kVJ * kVJ, v = 16 / lut_bytes, va = (n + v - 1) / v * v;
   L.off_vec = (int)sizeof(RCell);
-  L.off_j = L.off_vec + ((8 * (kZn + 7) * n + 15) & ~15);
-  L.off_a = L.off_j + 8 * L.ldj * n;
-  L.stride = ((long long)L.off_a + (long long)lut_bytes * L.lda * n + 127) & ~127LL;
+  L.off_j = L.off_vec + ((8 * kVecs * n + 15) & ~15);
+  L.off_a = L.off_j + 8 * vj * n;
+  L.stride = ((long long)L.off_a + (long long)lut_bytes * va * n + 127) & ~127LL;
   return L;
 }
 
@@ -94,14 +130,13 @@ struct RState {
 template <int n>
 struct RVec {
   double* b;
-  __device__ __forceinline__ double& zn(int j, int i) const { return b[j * n + i]; }
-  __device__ __forceinline__ double& ewt(int i) const { return b[(kZn + 0) * n + i]; }
-  __device__ __forceinline__ double& acor(int i) const { return b[(kZn + 1) * n + i]; }
-  __device__ __forceinline__ double& ftemp(int i) const { return b[(kZn + 2) * n + i]; }
-  __device__ __forceinline__ double& fv(int i) const { return b[(kZn + 3) * n + i]; }
-  __device__ __forceinline__ double& F(int i) const { return b[(kZn + 4) * n + i]; }
-  __device__ __forceinline__ double& dsc(int i) const { return b[(kZn + 5) * n + i]; }
-  __device__ __forceinline__ double& yev(int i) const { return b[(kZn + 6) * n + i]; }
+  __device__ __forceinline__ double& zn(int j, int i) const { return b[(kVZn + j) * n + i]; }
+  __device__ __forceinline__ double& ewt(int i) const { return b[kVEwt * n + i]; }
+  __device__ __forceinline__ double& acor(int i) const { return b[kVAcor * n + i]; }
+  __device__ __forceinline__ double& fv(int i) const { return b[kVFv * n + i]; }
+  __device__ __forceinline__ double& F(int i) const { return b[kVF * n + i]; }
+  __device__ __forceinline__ double& dsc(int i) const { return b[kVDsc * n + i]; }
+  __device__ __forceinline__ double& yev(int i) const { return b[kVYev * n + i]; }
 };
 
 __device__ __forceinline__ unsigned char* rec_of(const RState& S, long long slot) {
@@ -423,57 +458,47 @@ __device__ __forceinline__ void r_prepare_next(RCell& c, const RVec<n>& v, doubl
   }
 }
 
-// 16-byte vector loads / stores of an n-vector (n even, p 16-byte aligned).
-template <int n>
-__device__ __forceinline__ void vld(const double* p, double (&r)[n]) {
-  static_assert(n % 2 == 0, "records hold even-length vectors");
-  const double2* q = reinterpret_cast<const double2*>(p);
-#pragma unroll
-  for (int i = 0; i < n / 2; ++i) {
-    const double2 t = q[i];
-    r[2 * i] = t.x;
-    r[2 * i + 1] = t.y;
-  }
-}
+// Internal status of a cell stopped for the FP64 retry (never reported).
+constexpr int kStatusRefineStall = -100;
+// refine_ratio of a cell whose current matrix has not been measured yet
+constexpr float kRefineUnknown = 3.0e38f;
 
-template <int n>
-__device__ __forceinline__ void vst(double* p, const double (&r)[n]) {
-  double2* q = reinterpret_cast<double2*>(p);
-#pragma unroll
-  for (int i = 0; i < n / 2; ++i) q[i] = make_double2(r[2 * i], r[2 * i + 1]);
-}
-
-// Column stride of the inverse for n components (the record layout's lda).
-template <int n, typename LUT>
-constexpr int inv_ld() {
-  return sizeof(LUT) == 4 ? (n + 3) / 4 * 4 : (n + 1) / 2 * 2;
-}
-
-// x := D^-1 A D x for the group's cell: A is the scaled inverse
-// (column-major, 16-byte columns of inv_ld<n, LUT>() elements), D = dsc;
-// LUT = double: A is the plain inverse.  Lane gl holds components gl + G cc
-// of x and dsc; the multiplier of column j comes from its owner lane by
-// shuffle and lanes read consecutive elements of the column.
+// x := D^-1 A D x for the group's cell: A is the scaled inverse (mat_idx
+// order), D = dsc; LUT = double: A is the plain inverse.  Lane gl holds
+// components gl + G cc of x and dsc; the multipliers go through xs (n entries
+// of the group's shared scratch, 16-byte aligned and padded).
 template <int n, int G, typename LUT>
-__device__ __forceinline__ void g_apply_inverse(const LUT* A, const double (&dsc)[(n + G - 1) / G],
-                                                double (&x)[(n + G - 1) / G], int gl, unsigned gm) {
+__device__ __forceinline__ void g_apply_inverse(const LUT* __restrict__ A, const double (&dsc)[(n + G - 1) / G],
+                                                double (&x)[(n + G - 1) / G], LUT* xs, int gl, unsigned gm) {
   constexpr int CPL = (n + G - 1) / G;
   constexpr bool kScaled = sizeof(LUT) == 4;
-  constexpr int LD = inv_ld<n, LUT>();
-  LUT acc[CPL], bs[CPL];
+  constexpr int V = vec_of<LUT>(), JB = (n + V - 1) / V;
+  using Vec16 = typename std::conditional<kScaled, float4, double2>::type;
+  __syncwarp(gm);
 #pragma unroll
   for (int cc = 0; cc < CPL; ++cc) {
-    acc[cc] = (LUT)0;
-    bs[cc] = (LUT)(kScaled ? x[cc] * dsc[cc] : x[cc]);
+    const int i = gl + G * cc;
+    if (i < n) xs[i] = (LUT)(kScaled ? x[cc] * dsc[cc] : x[cc]);
   }
+  if (JB * V > n && gl < JB * V - n) xs[n + gl] = (LUT)0;
+  __syncwarp(gm);
+  LUT acc[CPL];
 #pragma unroll
-  for (int j = 0; j < n; ++j) {
-    const LUT bj = __shfl_sync(gm, bs[j / G], j % G, G);
-    const LUT* col = A + j * LD;
+  for (int cc = 0; cc < CPL; ++cc) acc[cc] = (LUT)0;
+#pragma unroll
+  for (int jb = 0; jb < JB; ++jb) {
+    const Vec16 bv = *reinterpret_cast<const Vec16*>(xs + jb * V);
+    const LUT* b = reinterpret_cast<const LUT*>(&bv);
 #pragma unroll
     for (int cc = 0; cc < CPL; ++cc) {
       const int i = gl + G * cc;
-      if (i < n) acc[cc] += col[i] * bj;
+      if (i < n) {
+        const Vec16 av = *reinterpret_cast<const Vec16*>(A + mat_vec<n, G, V>(cc, gl, jb));
+        const LUT* a = reinterpret_cast<const LUT*>(&av);
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+          if (jb * V + v < n) acc[cc] += a[v] * b[v];
+      }
     }
   }
 #pragma unroll
@@ -481,50 +506,57 @@ __device__ __forceinline__ void g_apply_inverse(const LUT* A, const double (&dsc
 }
 
 // One Newton correction: x = (I - gamma_lu J)^-1 dl with
-// dl = -(rl1 zn[1] + acor - gamma ftemp) (FP32 inverse, then, when `refine`,
+// dl = -(rl1 zn[1] + acor - gamma f) (FP32 inverse, then, when `refine`,
 // one FP64 refinement step r = dl - (x - gamma_lu J x), x += A r, whose WRMS
 // relative to x goes to *ratio; FP64 inverse: no refinement), scaled by
-// 2 / (1 + gamrat) when gamma has moved since the setup; then acor += x.
-// Returns the WRMS norms of x (*del) and of the new acor (*anrm).
-// Internal status of a cell stopped for the FP64 retry (never reported).
-constexpr int kStatusRefineStall = -100;
-// refine_ratio of a cell whose current matrix has not been measured yet
-constexpr float kRefineUnknown = 3.0e38f;
-
+// 2 / (1 + gamrat) when gamma has moved since the setup; then ac += x.
+// v: the record's vectors (shared-memory copy); ac: this lane's components of
+// acor.  Returns the WRMS norms of x (*del) and of the new acor (*anrm).
 template <int n, int G, typename LUT>
-__device__ __forceinline__ void g_newton(const RVec<n>& v, const double* J, const LUT* A, double rl1, double gamma,
-                                         double gamma_lu, double gamrat, int gl, unsigned gm, double* del,
-                                         double* anrm, double stall_ratio, bool* stall, bool refine,
-                                         float* ratio) {
+__device__ __forceinline__ void g_newton(const RVec<n>& v, const double* __restrict__ J, const LUT* __restrict__ A,
+                                         double* xs, double rl1, double gamma, double gamma_lu, double gamrat,
+                                         int gl, unsigned gm, double (&ac)[(n + G - 1) / G], double* del,
+                                         double* anrm, double stall_ratio, bool* stall, bool refine, float* ratio) {
   constexpr int CPL = (n + G - 1) / G;
   double dl[CPL], x[CPL], dsc[CPL];
 #pragma unroll
   for (int cc = 0; cc < CPL; ++cc) {
     const int i = gl + G * cc;
-    dl[cc] = (i < n) ? -(rl1 * v.zn(1, i) + v.acor(i) - gamma * v.ftemp(i)) : 0.0;
+    dl[cc] = (i < n) ? -(rl1 * v.zn(1, i) + ac[cc] - gamma * v.fv(i)) : 0.0;
     dsc[cc] = (i < n) ? v.dsc(i) : 1.0;
     x[cc] = dl[cc];
   }
-  g_apply_inverse<n, G, LUT>(A, dsc, x, gl, gm);
+  g_apply_inverse<n, G, LUT>(A, dsc, x, reinterpret_cast<LUT*>(xs), gl, gm);
   if constexpr (sizeof(LUT) == 4) {
     if (refine) {
-      constexpr int LDJ = (n + 1) / 2 * 2;
+      constexpr int JB = (n + kVJ - 1) / kVJ;
+      static_assert(n % kVJ == 0, "no column padding in J");
+      __syncwarp(gm);
+#pragma unroll
+      for (int cc = 0; cc < CPL; ++cc) {
+        const int i = gl + G * cc;
+        if (i < n) xs[i] = x[cc];
+      }
+      __syncwarp(gm);
       double r[CPL];
 #pragma unroll
       for (int cc = 0; cc < CPL; ++cc) r[cc] = 0.0;
 #pragma unroll
-      for (int j = 0; j < n; ++j) {
-        const double xj = __shfl_sync(gm, x[j / G], j % G, G);
-        const double* col = J + j * LDJ;
+      for (int jb = 0; jb < JB; ++jb) {
+        const double2 xv = *reinterpret_cast<const double2*>(xs + jb * kVJ);
 #pragma unroll
         for (int cc = 0; cc < CPL; ++cc) {
           const int i = gl + G * cc;
-          if (i < n) r[cc] += col[i] * xj;
+          if (i < n) {
+            const double2 a = *reinterpret_cast<const double2*>(J + mat_vec<n, G, kVJ>(cc, gl, jb));
+            r[cc] += a.x * xv.x;
+            r[cc] += a.y * xv.y;
+          }
         }
       }
 #pragma unroll
       for (int cc = 0; cc < CPL; ++cc) r[cc] = dl[cc] - (x[cc] - gamma_lu * r[cc]);
-      g_apply_inverse<n, G, LUT>(A, dsc, r, gl, gm);
+      g_apply_inverse<n, G, LUT>(A, dsc, r, reinterpret_cast<LUT*>(xs), gl, gm);
       double r2 = 0.0, x2 = 0.0;
 #pragma unroll
       for (int cc = 0; cc < CPL; ++cc) {
@@ -550,25 +582,285 @@ __device__ __forceinline__ void g_newton(const RVec<n>& v, const double* J, cons
     const int i = gl + G * cc;
     if (i < n) {
       const double xi = x[cc] * sc;
-      const double ac = v.acor(i) + xi;
-      v.acor(i) = ac;
+      ac[cc] += xi;
       const double w = v.ewt(i);
       s2 += (xi * w) * (xi * w);
-      a2 += (ac * w) * (ac * w);
+      a2 += (ac[cc] * w) * (ac[cc] * w);
     }
   }
   *del = sqrt(gsum<G>(s2, gm) / n);
   *anrm = sqrt(gsum<G>(a2, gm) / n);
 }
 
+// The next f of a cell is at its new prediction: whether its Newton matrix is
+// rebuilt before that f is consumed, and whether with a new Jacobian (CVODE's
+// jbad rule: on the first step, every msbj steps, or after a convergence
+// failure with a stale Jacobian or with gamma little changed).
+__device__ __forceinline__ int r_ask_attempt(RCell& c) {
+  if (!c.callSetup) {
+    c.label = kLAfterNStart;
+    return kNeedRhs;
+  }
+  c.label = kLAfterSetup;
+  c.setup_conv = c.jbad ? kFailBadJ : c.convfail;
+  const double dgamma = fabs(c.gamma / c.gammap - 1.0);
+  const bool jbad = (c.cnt.nst == 0) || (c.cnt.nst >= c.nstlj + kMSBJ) ||
+                    (c.setup_conv == kFailBadJ && dgamma < kDGMAX_JBAD) || (c.setup_conv == kFailOther);
+  c.jcur = jbad ? 1 : 0;
+  if (!jbad) return kNeedSetup;
+  c.cnt.nje++;
+  c.nstlj = c.cnt.nst;
+  return kNeedSetupJac;
+}
+
+// The step of a converged Newton iteration that passed its error test
+// (dsm <= 1, not the last of the cell): completes it, chooses the next order
+// and step size, and predicts, with the Nordsieck columns in registers from
+// one load to one store (r_prepare_next, r_set_ewt, r_increase, r_decrease,
+// r_rescale, r_predict and r_set_bdf in one pass).  s: the record's vectors
+// and c its scalars in shared memory (read only); g: the record's vectors in
+// device memory, written; o: the scalars that change.  Returns the need.
+template <int n, int G>
+__device__ __forceinline__ int g_finish_step(const RCell& c, RCell& o, const RVec<n>& s, const RVec<n>& g,
+                                             const double (&ac)[(n + G - 1) / G], double dsm, const double* atolv,
+                                             double rtol, int gl, unsigned gm) {
+  constexpr int CPL = (n + G - 1) / G;
+  const int q = c.q, qm = c.qmax;
+  const double h = c.h;
+  o.cnt.nst = c.cnt.nst + 1;
+#pragma unroll
+  for (int i = 0; i < kZn + 2; ++i) o.tau[i] = c.tau[i];
+#pragma unroll
+  for (int i = kZn + 1; i >= 2; --i)
+    if (i <= q) o.tau[i] = o.tau[i - 1];
+  if (q == 1 && o.cnt.nst > 1) o.tau[2] = o.tau[1];
+  o.tau[1] = h;
+  const bool save = (c.qwait - 1 == 1 && q != qm);
+  o.saved_tq5 = save ? c.tq[5] : c.saved_tq5;
+  int qwait = c.qwait - 1;
+  // completed Nordsieck columns
+  double z[CPL][kZn];
+#pragma unroll
+  for (int j = 0; j < kZn; ++j) {
+    const double lj = c.l[j];
+#pragma unroll
+    for (int cc = 0; cc < CPL; ++cc) {
+      const int i = gl + G * cc;
+      z[cc][j] = (i < n && j <= q) ? s.zn(j, i) + lj * ac[cc] : 0.0;
+    }
+  }
+  // next order and step size
+  const int L = q + 1;
+  int qprime = q;
+  double eta = 1.0, hprime = h;
+  bool keep_acor = save;
+  if (c.etamax == 1.0) {
+    qwait = qwait > 2 ? qwait : 2;
+  } else {
+    double base = kBIAS2 * dsm, ex = 1.0 / L;
+    const bool order = qwait == 0;
+    const bool down = order && q > 1, up = order && q != qm && o.saved_tq5 != 0.0;
+    if (order) {
+      // lane 1 of the group evaluates the power for order q - 1, lane 2 for
+      // order q + 1, the others for order q
+      double dn = 0.0, dp = 0.0;
+      const double ratio = h / o.tau[2];
+      double rp = 1.0;
+      for (int k = 0; k < L; ++k) rp *= ratio;
+      const double cquot = up ? (c.tq[5] / o.saved_tq5) * rp : 0.0;
+#pragma unroll
+      for (int cc = 0; cc < CPL; ++cc) {
+        const int i = gl + G * cc;
+        if (i < n) {
+          const double w = s.ewt(i);
+          double zq = z[cc][1];
+#pragma unroll
+          for (int j = 2; j < kZn; ++j)
+            if (j == q) zq = z[cc][j];
+          const double t = zq * w;
+          dn += t * t;
+          const double u = (ac[cc] - cquot * s.zn(qm, i)) * w;
+          dp += u * u;
+        }
+      }
+      dn = gsum<G>(dn, gm);
+      dp = gsum<G>(dp, gm);
+      const double ddn = sqrt(dn / n) * c.tq[1], dup = sqrt(dp / n) * c.tq[3];
+      if (gl == 1 && down) {
+        base = kBIAS1 * ddn;
+        ex = 1.0 / q;
+      } else if (gl == 2 && up) {
+        base = kBIAS3 * dup;
+        ex = 1.0 / (L + 1);
+      }
+    }
+    const double et = 1.0 / (pow(base, ex) + kADDON);
+    const double etaq = __shfl_sync(gm, et, 0, G);
+    if (!order) {
+      eta = etaq;
+    } else {
+      const double e1 = __shfl_sync(gm, et, 1, G), e2 = __shfl_sync(gm, et, 2, G);
+      const double etaqm1 = down ? e1 : 0.0, etaqp1 = up ? e2 : 0.0;
+      qwait = 2;
+      const double etam = fmax(etaqm1, fmax(etaq, etaqp1));
+      if (etam < kTHRESH) {
+        eta = 1.0;
+      } else if (etam == etaq) {
+        eta = etaq;
+      } else if (etam == etaqm1) {
+        eta = etaqm1;
+        qprime = q - 1;
+      } else {
+        eta = etaqp1;
+        qprime = q + 1;
+        keep_acor = true;
+      }
+    }
+    if (eta < kTHRESH) {
+      eta = 1.0;
+    } else {
+      eta = fmin(eta, c.etamax);
+      hprime = h * eta;
+    }
+  }
+  o.etamax = (o.cnt.nst <= kSMALL_NST) ? kETAMX2 : kETAMX3;
+  o.nstloc = c.nstloc + 1;
+  // error weights of the next step, from the completed state
+#pragma unroll
+  for (int cc = 0; cc < CPL; ++cc) {
+    const int i = gl + G * cc;
+    if (i < n) {
+      g.ewt(i) = 1.0 / (rtol * fabs(z[cc][0]) + __ldg(atolv + i));
+      if (keep_acor) g.zn(qm, i) = ac[cc];
+    }
+  }
+  o.saved_t = c.tn;
+  o.qprime = qprime;
+  o.hprime = hprime;
+  o.eta = eta;
+  o.q = q;
+  o.L = L;
+  o.h = h;
+  o.hscale = c.hscale;
+  if (hprime != h) {
+    if (qprime != q) {
+      // order change: the columns the new order needs
+      double lj[kZn];
+#pragma unroll
+      for (int j = 0; j < kZn; ++j) lj[j] = 0.0;
+      lj[2] = 1.0;
+      if (qprime > q) {
+        double alpha1 = 1.0, prod = 1.0, xiold = 1.0, alpha0 = -1.0, hsum = c.hscale;
+#pragma unroll
+        for (int j = 1; j < kZn - 1; ++j) {
+          if (j < q) {
+            hsum += o.tau[j + 1];
+            const double xi = hsum / c.hscale;
+            prod *= xi;
+            alpha0 -= 1.0 / (j + 1);
+            alpha1 += 1.0 / xi;
+#pragma unroll
+            for (int i = j + 2; i >= 2; --i)
+              if (i < kZn) lj[i] = lj[i] * xiold + lj[i - 1];
+            xiold = xi;
+          }
+        }
+        const double A1 = (-alpha0 - alpha1) / prod;
+#pragma unroll
+        for (int cc = 0; cc < CPL; ++cc) {
+          const double zz = A1 * ac[cc];
+#pragma unroll
+          for (int j = 2; j < kZn; ++j) {
+            if (j <= q) z[cc][j] += lj[j] * zz;
+            else if (j == q + 1) z[cc][j] = zz;
+          }
+        }
+      } else {
+        double hsum = 0.0;
+#pragma unroll
+        for (int j = 1; j < kZn - 2; ++j) {
+          if (j <= q - 2) {
+            hsum += o.tau[j];
+            const double xi = hsum / c.hscale;
+#pragma unroll
+            for (int i = j + 2; i >= 2; --i)
+              if (i < kZn) lj[i] = lj[i] * xi + lj[i - 1];
+          }
+        }
+#pragma unroll
+        for (int cc = 0; cc < CPL; ++cc) {
+          double zq = z[cc][1];
+#pragma unroll
+          for (int j = 2; j < kZn; ++j)
+            if (j == q) zq = z[cc][j];
+#pragma unroll
+          for (int j = 2; j < kZn; ++j)
+            if (j < q) z[cc][j] -= lj[j] * zq;
+        }
+      }
+      o.q = qprime;
+      o.L = qprime + 1;
+      qwait = o.L;
+    }
+    double factor = eta;
+#pragma unroll
+    for (int j = 1; j < kZn; ++j) {
+      if (j <= o.q) {
+#pragma unroll
+        for (int cc = 0; cc < CPL; ++cc) z[cc][j] *= factor;
+        factor *= eta;
+      }
+    }
+    o.h = c.hscale * eta;
+    o.hscale = o.h;
+  }
+  o.qwait = qwait;
+  // prediction zn := zn * Pascal, columns stored once
+  o.tn = c.tn + o.h;
+  const int qn = o.q;
+#pragma unroll
+  for (int cc = 0; cc < CPL; ++cc) {
+    const int i = gl + G * cc;
+#pragma unroll
+    for (int k = 1; k < kZn; ++k)
+#pragma unroll
+      for (int j = kZn - 1; j >= 1; --j)
+        if (j >= k && j <= qn) z[cc][j - 1] += z[cc][j];
+    if (i < n) {
+#pragma unroll
+      for (int j = 0; j < kZn; ++j)
+        if (j <= qn) g.zn(j, i) = z[cc][j];
+      g.yev(i) = z[cc][0];
+    }
+  }
+  // coefficients of the step and the matrix it needs
+  o.gammap = c.gammap;
+  o.tq[1] = c.tq[1];
+  o.tq[3] = c.tq[3];
+#pragma unroll
+  for (int j = 0; j < kZn; ++j) o.l[j] = 0.0;
+  o.nstlj = c.nstlj;
+  o.cnt.nje = c.cnt.nje;
+  r_set_bdf(o);
+  o.ncf = o.nef = 0;
+  o.nflag = kFirstCall;
+  o.convfail = kNoFailures;
+  o.jcur = 0;
+  o.jbad = 0;
+  o.attempt = 0;
+  o.callSetup = (o.cnt.nst >= c.nstlp + kMSBP) || (fabs(o.gamrat - 1.0) > kDGMAX_LSETUP);
+  o.setup_conv = c.setup_conv;
+  return r_ask_attempt(o);
+}
+
 // Advance the cell from resume point `lab` until it needs a right-hand side
-// at v.yev (returns kNeedRhs with c.label set to the label that consumes it),
-// a setup (kNeedSetup, or kNeedSetupJac with a Jacobian refresh), or is
-// finished (kDone, *status set).
-template <int n, int G, typename LUT>
+// at v.yev (returns kNeedRhs, or kNeedSetup / kNeedSetupJac when its Newton
+// matrix is rebuilt before that f is consumed, with c.label set to the label
+// that consumes it) or is finished (kDone, *status set).  The Newton
+// iteration itself is the step kernel's: a cell leaves here before it.
+template <int n, int G>
 __device__ __forceinline__ int r_advance(RCell& c, const RVec<n>& v, int lab, const double* atolv, double rtol,
-                                         const double* J, const LUT* A, int gl, unsigned gm, int* status,
-                                         double stall_ratio = 0.0, double keep_ratio = 0.0) {
+                                         int gl, unsigned gm, int* status) {
   for (int guard = 0; guard < 256; ++guard) {
     switch (lab) {
       case kLAfterF0: {
@@ -683,90 +975,18 @@ __device__ __forceinline__ int r_advance(RCell& c, const RVec<n>& v, int lab, co
         break;
       }
       case kLNlsAttempt: {
-        each<n, G>(gl, [&](int i) {
-          v.acor(i) = 0.0;
-          v.yev(i) = v.zn(0, i);
-        });
-        c.label = kLAfterNStart;
-        return kNeedRhs;
+        each<n, G>(gl, [&](int i) { v.yev(i) = v.zn(0, i); });
+        return r_ask_attempt(c);
       }
-      case kLAfterNStart: {
-        each<n, G>(gl, [&](int i) { v.ftemp(i) = v.fv(i); });
-        if (c.callSetup) {
-          c.setup_conv = c.jbad ? kFailBadJ : c.convfail;
-          c.label = kLAfterSetup;
-          // CVODE's jbad rule: recompute J on the first step, every msbj
-          // steps, or after a convergence failure (with a stale J, or with
-          // gamma little changed)
-          const double dgamma = fabs(c.gamma / c.gammap - 1.0);
-          const bool jbad = (c.cnt.nst == 0) || (c.cnt.nst >= c.nstlj + kMSBJ) ||
-                            (c.setup_conv == kFailBadJ && dgamma < kDGMAX_JBAD) || (c.setup_conv == kFailOther);
-          c.jcur = jbad ? 1 : 0;
-          if (jbad) {
-            c.cnt.nje++;
-            c.nstlj = c.cnt.nst;
-            return kNeedSetupJac;
-          }
-          return kNeedSetup;
-        }
-        c.mnewt = 0;
-        c.delp = 0.0;
-        lab = kLNewtonIter;
-        break;
-      }
-      case kLAfterSetup: {
+      case kLAfterSetup:  // only a failed setup comes here
         c.callSetup = 0;
-        c.refine_ratio = kRefineUnknown;
-        if (c.setup_ier) {
-          lab = kLNlsFail2;
-          break;
-        }
-        c.mnewt = 0;
-        c.delp = 0.0;
-        lab = kLNewtonIter;
+        lab = kLNlsFail2;
         break;
-      }
-      case kLNewtonIter: {
-        c.cnt.nni++;
-        double del, anrm;
-        bool stall = false;
-        // the FP64 refinement runs on the first correction with a new matrix,
-        // and again on every later one unless that first measurement showed
-        // the FP32 solve alone accurate to keep_ratio
-        const bool refine = !(keep_ratio > 0.0 && c.refine_ratio <= keep_ratio);
-        float ratio = c.refine_ratio;
-        g_newton<n, G, LUT>(v, J, A, c.rl1, c.gamma, c.gamma_lu, c.gamrat, gl, gm, &del, &anrm, stall_ratio,
-                            &stall, refine, &ratio);
-        c.refine_ratio = ratio;
-        if (stall) {
-          // the FP32 inverse does not resolve this iteration matrix: the cell
-          // is left untouched for the pass with the FP64 LU
-          *status = kStatusRefineStall;
-          return kDone;
-        }
-        if (c.mnewt > 0) c.crate = fmax(kCRDOWN * c.crate, del / c.delp);
-        const double dcon = del * fmin(1.0, c.crate) / c.tq[4];
-        if (dcon <= 1.0) {
-          c.acnrm = (c.mnewt == 0) ? del : anrm;
-          c.jcur = 0;
-          lab = kLNlsSuccess;
-          break;
-        }
-        if ((c.mnewt >= 1 && del > kRDIV * c.delp) || !(del == del) || c.mnewt + 1 >= kMAXCOR) {
-          lab = kLNlsRecover;
-          break;
-        }
-        c.delp = del;
-        c.mnewt++;
-        each<n, G>(gl, [&](int i) { v.yev(i) = v.zn(0, i) + v.acor(i); });
-        c.label = kLAfterNIter;
-        return kNeedRhs;
-      }
-      case kLAfterNIter: {
-        each<n, G>(gl, [&](int i) { v.ftemp(i) = v.fv(i); });
-        lab = kLNewtonIter;
-        break;
-      }
+      case kLStall:
+        // the FP32 inverse does not resolve this iteration matrix: the cell
+        // is left untouched for the pass with the FP64 LU
+        *status = kStatusRefineStall;
+        return kDone;
       case kLNlsRecover: {
         if (!c.jcur && c.attempt < 3) {
           c.callSetup = 1;
@@ -914,7 +1134,6 @@ __device__ __forceinline__ void r_begin(RCell& c, const RVec<n>& v, const double
 #pragma unroll 2
   for (int i = 0; i < n; ++i) {
     for (int j = 1; j < kZn; ++j) v.zn(j, i) = 0.0;
-    v.acor(i) = 0.0;
     v.yev(i) = v.zn(0, i);
   }
   r_set_ewt<n, 1>(v, atolv, rtol, 0);

@@ -142,7 +142,7 @@ cudaError_t tpc_launch(int N, int lut_bytes, const ReactParams& P, const TpcPara
 
 // ------------------------------------------------------ round-based path
 constexpr int kRoundsRhsBlock = 64;  // threads per CTA of the rhs kernel
-enum { kRoundsStart = 0, kRoundsRhs, kRoundsCtrl, kRoundsJac, kRoundsGj };
+enum { kRoundsStart = 0, kRoundsRhs, kRoundsStep, kRoundsJac, kRoundsGj, kRoundsCtrl };
 
 // Per-warp shared scratch of the setup kernels.  Jacobian kernel: C, g/RT,
 // h/RT, third-body row [Npad] and the Jacobian [n][n] (double).
@@ -154,6 +154,16 @@ struct RoundsSetupLayout {
   long long gbytes_per_warp;
 };
 
+// Lists a round's kernels append to: cells that need a right-hand side next
+// round (entries of cells whose Newton matrix is rebuilt before that f is
+// consumed carry kSetupFlag), those cells again, the subset of them whose
+// Jacobian is recomputed, and the cells the control kernel takes this round.
+enum { kRlRhs = 0, kRlSetup, kRlJac, kRlCtrl, kRoundLists };
+constexpr int kSetupFlag = 1 << 30;
+// slot lists of a chunk: the first three of the above twice (read and written
+// in turn) and the control kernel's
+constexpr int kRoundSlotLists = 2 * kRlCtrl + 1;
+
 struct RoundsParams {
   ReactParams P;
   rounds::RState S;
@@ -162,19 +172,15 @@ struct RoundsParams {
   long long nchunk;  // cells in the chunk
   const int* list_in;
   const int* cnt_in;
-  int* list_out;     // cells that need a right-hand side next round
-  int* cnt_out;
-  int* list_setup;   // cells that need a Newton-matrix setup this round
-  int* cnt_setup;
-  int* list_jac;     // the subset of list_setup whose Jacobian is recomputed
-  int* cnt_jac;
+  int* list[kRoundLists];  // lists the kernel appends to (the kRl* indices)
+  int* cnt_next;           // their counters [kRoundLists]; cleared by the right-hand-side kernel
   unsigned char* wscratch;  // [setup warps][SL.gbytes_per_warp]
   int const_mech;           // 1: the packed table is in the constant bank
   int gen_mech;             // 1: the mechanism has a generated right-hand side
 };
 
 struct RoundsGrids {
-  int start, rhs, ctrl, jac, gj;
+  int start, rhs, step, ctrl, jac, gj;
 };
 
 // Handle accessors (defined with the handle in b200chem.cu).
@@ -192,7 +198,7 @@ RoundsSetupLayout rounds_setup_layout(int N, int R, int lut_bytes);
 long long rounds_state_bytes_per_cell(int N, int lut_bytes);
 rounds::RState rounds_carve(void* base, long long cap, int N, int lut_bytes);
 cudaError_t rounds_grids_for(int N, int lut_bytes, const RoundsSetupLayout& SL, int sm_count, RoundsGrids* G);
-cudaError_t rounds_launch(int N, int lut_bytes, int what, const RoundsParams& R, const RoundsGrids& G, int after_rhs,
+cudaError_t rounds_launch(int N, int lut_bytes, int what, const RoundsParams& R, const RoundsGrids& G, int setup_pass,
                           cudaStream_t st);
 
 // ------------------------------------------- packed constant-memory table

@@ -4,13 +4,15 @@
 // A react call is processed in chunks of cells (as many as the state buffer
 // holds).  For one chunk:
 //   start                     load every cell, mask / validity checks, list A
-//   repeat until A is empty:
+//   repeat until A is empty (S, SJ: the cells of A whose Newton matrix is
+//   rebuilt, and those of them whose Jacobian is recomputed):
 //     rhs   (A)               f(y) for every cell of A (thread per cell)
-//     ctrl  (A -> B, S)       resume each cell with its f: next f -> B,
-//                             Newton-matrix setup -> S, finished -> outputs
-//     setup (S)               Jacobian + inverse (warp per cell)
-//     ctrl  (S -> B)          resume the set-up cells
-//     swap A, B
+//     step  (A without S)     Newton correction and step; next f -> B (S', SJ'
+//                             as the prediction needs), anything rarer -> W
+//     jac   (SJ), gj (S)      Jacobian, inverse (warp per cell)
+//     step  (S)               the same for the set-up cells
+//     ctrl  (W)               the rare paths; finished cells -> outputs
+//     swap A, B and the setup lists
 // Lists are appended with warp-aggregated atomics, so a warp's slots stay in
 // order and the interleaved state accesses stay coalesced as cells drop out.
 #include <algorithm>
@@ -46,7 +48,9 @@ __device__ __forceinline__ CellLoc locate(const ReactParams& P, long long cell) 
   return L;
 }
 
-// Append `val` to list/cnt for the lanes with pred (all 32 lanes call it).
+// Append `val` of the lanes with pred to one list of counter cnt, or of the
+// lanes whose bit k of `which` is set to list k (all 32 lanes call it): one
+// atomic per warp and list.
 __device__ __forceinline__ void warp_append(bool pred, int val, int* list, int* cnt) {
   const unsigned m = __ballot_sync(kFull, pred);
   if (m == 0) return;
@@ -56,6 +60,33 @@ __device__ __forceinline__ void warp_append(bool pred, int val, int* list, int* 
   if (lane == leader) base = atomicAdd(cnt, __popc(m));
   base = __shfl_sync(kFull, base, leader);
   if (pred) list[base + __popc(m & ((1u << lane) - 1u))] = val;
+}
+
+// The lists' atomics are issued together by lanes 0..kRoundLists - 1, so a
+// warp waits for one of them and not for their sum.
+__device__ __forceinline__ void warp_append_lists(int which, int slot, int rhs_val, const RoundsParams& R) {
+  const int lane = threadIdx.x & 31;
+  unsigned m[kRoundLists], mine = 0;
+#pragma unroll
+  for (int k = 0; k < kRoundLists; ++k) {
+    m[k] = __ballot_sync(kFull, (which >> k) & 1);
+    if (lane == k) mine = m[k];
+  }
+  int base = 0;
+  if (mine) base = atomicAdd(R.cnt_next + lane, __popc(mine));
+#pragma unroll
+  for (int k = 0; k < kRoundLists; ++k) {
+    const int b = __shfl_sync(kFull, base, k);
+    if ((which >> k) & 1) R.list[k][b + __popc(m[k] & ((1u << lane) - 1u))] = (k == kRlRhs) ? rhs_val : slot;
+  }
+}
+
+// Lists a cell with this need goes to.
+__device__ __forceinline__ int lists_of(int need) {
+  return need == kNeedRhs ? 1 << kRlRhs
+         : need == kNeedSetup ? (1 << kRlRhs) | (1 << kRlSetup)
+         : need == kNeedSetupJac ? (1 << kRlRhs) | (1 << kRlSetup) | (1 << kRlJac)
+                                 : 0;
 }
 
 // Warp-aggregated statistics of the lanes with `done` (all 32 lanes call it).
@@ -381,7 +412,7 @@ __global__ void __launch_bounds__(128) rk_start(RoundsParams R) {
       }
       if (!go && P.status) P.status[cell] = code;
     }
-    warp_append(go, (int)slot, R.list_out, R.cnt_out);
+    warp_append(go, (int)slot, R.list[kRlRhs], R.cnt_next + kRlRhs);
     warp_stats(P.stats, done, true, masked, CellCounters{0, 0, 0, 0, 0, 0, 0});
   }
 }
@@ -400,11 +431,13 @@ __global__ void __launch_bounds__(kRoundsRhsBlock, B200_RHS_MIN_CTAS) rk_rhs(Rou
   if (threadIdx.x == 0) s_mech = R.P.mech;
   __syncthreads();
   const int cnt = *R.cnt_in;
+  // counters of the lists this round's later kernels append to
+  if (blockIdx.x == 0 && threadIdx.x < kRoundLists) R.cnt_next[threadIdx.x] = 0;
   double* sC = reinterpret_cast<double*>(dsm) + threadIdx.x;
   double* sG = sC + NS * blockDim.x;
   double* sW = sG + NS * blockDim.x;
   for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < cnt; idx += gridDim.x * blockDim.x) {
-    const int slot = R.list_in[idx];
+    const int slot = R.list_in[idx] & ~kSetupFlag;
     const RVec<n> v{reinterpret_cast<double*>(rec_of(R.S, slot) + R.S.L.off_vec)};
     if (R.gen_mech) {
       // generated code for this mechanism: every coefficient an immediate
@@ -419,24 +452,10 @@ __global__ void __launch_bounds__(kRoundsRhsBlock, B200_RHS_MIN_CTAS) rk_rhs(Rou
   }
 }
 
-// Minimum resident CTAs per SM requested for the control kernel (its
-// register budget: 3 -> 168 registers per thread).
-#ifndef B200_CTRL_MIN_CTAS
-#define B200_CTRL_MIN_CTAS 3
-#endif
-
-// Lanes per cell of the control kernel.
-#ifndef B200_CTRL_LANES
-#define B200_CTRL_LANES 8
-#endif
-constexpr int ctrl_group(int n) { return n <= 32 ? B200_CTRL_LANES : 16; }
-
-// L2 prefetch of the control kernel: 0 none; 1 the vectors and matrices of
-// each cell as it starts (they stream in while the step-control scalars are
-// processed); 2 also the scalars and vectors of the cell the group takes
-// next.
-#ifndef B200_CTRL_PREFETCH
-#define B200_CTRL_PREFETCH 1
+// Minimum resident CTAs (of 128 threads) per SM requested for the step
+// kernel: bounds its registers per thread.
+#ifndef B200_STEP_MIN_CTAS
+#define B200_STEP_MIN_CTAS 4
 #endif
 
 // Bulk prefetch of [p, p + bytes) into L2 (p and bytes multiples of 16; a
@@ -445,36 +464,178 @@ __device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
-// One cell of the control kernel, G lanes per cell: resume the CVODE state
-// machine (after_rhs: consuming the f just evaluated, counted in nfe;
-// otherwise coming back from a setup), write the outputs of a finished cell,
-// and append the cell to the list of its next need.  Every lane of the warp
-// calls it (the appends are warp-collective); `live` marks the groups with a
-// cell.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+}
+
+// Shared memory of one cell of the step kernel: the scalars and the vectors
+// it reads, as they lie in the record, n doubles of scratch, and 16 bytes
+// that spread the cells of a warp over the banks.
+template <int n>
+constexpr int step_read_bytes() { return (int)sizeof(RCell) + 8 * kVecsRead * n; }
+template <int n>
+constexpr int step_cell_bytes() { return step_read_bytes<n>() + 8 * ((n + 1) / 2 * 2) + 16; }
+template <int n>
+constexpr int step_smem() { return 128 / ctrl_group(n) * step_cell_bytes<n>(); }
+
+// One cell of the step kernel, G lanes per cell: the Newton correction with
+// the f just evaluated, then the next Newton iterate or, after a converged
+// iteration that passes the error test, the next prediction.  Anything else
+// (the start of a cell, failures, its last step) goes to the control kernel,
+// with the label it resumes at.  Every lane of the warp calls it (the appends
+// are warp-collective); `live` marks the groups with a cell; sm: the cell's
+// shared memory.
 template <int NS, int G, typename LUT>
-__device__ __forceinline__ void ctrl_cell(const RoundsParams& R, bool live, int slot, bool after_rhs, int gl,
-                                          unsigned gm, int idx_next) {
+__device__ __forceinline__ void step_cell(const RoundsParams& R, bool live, int slot, unsigned char* sm, int gl,
+                                          unsigned gm) {
+  constexpr int n = NS + 1;
+  constexpr int CPL = (n + G - 1) / G;
+  const ReactParams& P = R.P;
+  int which = 0, rhs_val = slot;
+  if (live) {
+    unsigned char* rec = rec_of(R.S, slot);
+    if (gl == 0) l2_prefetch(rec + R.S.L.off_j, (uint32_t)(R.S.L.stride - R.S.L.off_j));
+    for (int b = gl * 16; b < step_read_bytes<n>(); b += G * 16) cp_async16(sm + b, rec + b);
+    cp_async_wait();
+    __syncwarp(gm);
+    RCell& c = *reinterpret_cast<RCell*>(sm);
+    const RVec<n> s{reinterpret_cast<double*>(sm + sizeof(RCell))};
+    const RVec<n> g{reinterpret_cast<double*>(rec + sizeof(RCell))};
+    const int label = c.label;
+    which = 1 << kRlCtrl;
+    if (label == kLAfterNStart || label == kLAfterNIter || (label == kLAfterSetup && c.setup_ier == 0)) {
+      const bool iter = label == kLAfterNIter;
+      const int mnewt = iter ? c.mnewt : 0;
+      double ac[CPL];
+#pragma unroll
+      for (int cc = 0; cc < CPL; ++cc) {
+        const int i = gl + G * cc;
+        ac[cc] = (iter && i < n) ? s.acor(i) : 0.0;
+      }
+      double del, anrm;
+      bool stall = false;
+      float ratio = (label == kLAfterSetup) ? kRefineUnknown : c.refine_ratio;
+      // the FP64 refinement runs on the first correction with a new matrix,
+      // and again on every later one unless that first measurement showed
+      // the FP32 solve alone accurate to refine_keep
+      const bool refine = !(P.refine_keep > 0.0 && ratio <= P.refine_keep);
+      g_newton<n, G, LUT>(s, reinterpret_cast<const double*>(rec + R.S.L.off_j),
+                          reinterpret_cast<const LUT*>(rec + R.S.L.off_a),
+                          reinterpret_cast<double*>(sm + step_read_bytes<n>()), c.rl1, c.gamma, c.gamma_lu, c.gamrat,
+                          gl, gm, ac, &del, &anrm, sizeof(LUT) == 4 ? P.refine_stall : 0.0, &stall, refine, &ratio);
+      const double crate = (mnewt > 0) ? fmax(kCRDOWN * c.crate, del / c.delp) : c.crate;
+      const double dcon = del * fmin(1.0, crate) / c.tq[4];
+      const double acnrm = (mnewt == 0) ? del : anrm;
+      const double dsm = acnrm * c.tq[2];
+      const bool conv = dcon <= 1.0;
+      const bool step = !stall && conv && dsm <= 1.0 && !(c.tn - c.dt >= 0.0) && c.nstloc + 1 < c.max_steps;
+      const bool again = !stall && !conv &&
+                         !((mnewt >= 1 && del > kRDIV * c.delp) || !(del == del) || mnewt + 1 >= kMAXCOR);
+      RCell o;
+      if (step) {
+        const int need = g_finish_step<n, G>(c, o, s, g, ac, dsm, P.atol, P.rtol, gl, gm);
+        which = lists_of(need);
+        if (need != kNeedRhs) rhs_val |= kSetupFlag;
+      } else {
+#pragma unroll
+        for (int cc = 0; cc < CPL; ++cc) {
+          const int i = gl + G * cc;
+          if (i < n) {
+            g.acor(i) = ac[cc];
+            if (again) g.yev(i) = s.zn(0, i) + ac[cc];
+          }
+        }
+        if (again) which = 1 << kRlRhs;
+      }
+      __syncwarp(gm);  // every lane is done reading c
+      if (gl == 0) {
+        c.cnt.nfe++;
+        c.cnt.nni++;
+        c.crate = crate;
+        c.refine_ratio = ratio;
+        if (step) {
+#define B200_ST(f) c.f = o.f;
+          B200_ST(h) B200_ST(hprime) B200_ST(hscale) B200_ST(eta) B200_ST(etamax) B200_ST(tn) B200_ST(gamma)
+          B200_ST(gamrat) B200_ST(rl1) B200_ST(saved_tq5) B200_ST(saved_t) B200_ST(q) B200_ST(qprime) B200_ST(L)
+          B200_ST(qwait) B200_ST(nstlj) B200_ST(jcur) B200_ST(ncf) B200_ST(nef) B200_ST(nflag) B200_ST(convfail)
+          B200_ST(callSetup) B200_ST(jbad) B200_ST(attempt) B200_ST(nstloc) B200_ST(setup_conv) B200_ST(label)
+          B200_ST(cnt.nst) B200_ST(cnt.nje)
+#undef B200_ST
+#pragma unroll
+          for (int i = 1; i < kZn + 2; ++i) c.tau[i] = o.tau[i];
+#pragma unroll
+          for (int i = 1; i < 6; ++i) c.tq[i] = o.tq[i];
+#pragma unroll
+          for (int i = 0; i < kZn; ++i) c.l[i] = o.l[i];
+        } else if (again) {
+          c.delp = del;
+          c.mnewt = mnewt + 1;
+          c.label = kLAfterNIter;
+        } else {
+          c.acnrm = acnrm;
+          c.mnewt = mnewt;
+          if (conv) c.jcur = 0;
+          c.label = stall ? kLStall : conv ? kLNlsSuccess : kLNlsRecover;
+        }
+      }
+      __syncwarp(gm);
+      for (int b = gl * 16; b < (int)sizeof(RCell); b += G * 16)
+        *reinterpret_cast<uint4*>(rec + b) = *reinterpret_cast<const uint4*>(sm + b);
+    }
+  }
+  __syncwarp();  // the shared copies are free again
+  warp_append_lists(gl == 0 ? which : 0, slot, rhs_val, R);
+}
+
+// Newton correction and step of the cells of list_in, G lanes per cell.
+// setup_pass: the cells whose Newton matrix this round's setup kernels
+// rebuilt; otherwise the others (those entries, flagged, are passed over).
+template <int NS, typename LUT>
+__global__ void __launch_bounds__(128, B200_STEP_MIN_CTAS) rk_step(RoundsParams R, int setup_pass) {
+  constexpr int n = NS + 1;
+  constexpr int G = ctrl_group(n);
+  constexpr int GPW = 32 / G;  // cells per warp
+  extern __shared__ __align__(16) unsigned char dsm[];
+  const int cnt = *R.cnt_in;
+  const int lane = threadIdx.x & 31, gl = lane % G, gi = lane / G;
+  const unsigned gm = (G == 32) ? kFull : (((1u << G) - 1u) << (gi * G));
+  unsigned char* sm = dsm + (threadIdx.x / G) * step_cell_bytes<n>();
+  const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nw = (gridDim.x * blockDim.x) >> 5;
+  for (int base = wid * GPW; base < cnt; base += nw * GPW) {
+    const int idx = base + gi;
+    const int entry = idx < cnt ? R.list_in[idx] : kSetupFlag;
+    step_cell<NS, G, LUT>(R, !(entry & kSetupFlag), entry & ~kSetupFlag, sm, gl, gm);
+  }
+}
+
+// Minimum resident CTAs (of 128 threads) per SM requested for the control
+// kernel: bounds its registers per thread.
+#ifndef B200_CTRL_MIN_CTAS
+#define B200_CTRL_MIN_CTAS 3
+#endif
+
+// One cell of the control kernel, G lanes per cell: resume the CVODE state
+// machine, write the outputs of a finished cell, and append the cell to the
+// lists of its next need.  Every lane of the warp calls it (the appends are
+// warp-collective); `live` marks the groups with a cell.
+template <int NS, int G>
+__device__ __forceinline__ void ctrl_cell(const RoundsParams& R, bool live, int slot, int gl, unsigned gm) {
   constexpr int n = NS + 1;
   const ReactParams& P = R.P;
   int need = kDone, status = 0;
   RCell c;
   if (live) {
     unsigned char* rec = rec_of(R.S, slot);
-    if (B200_CTRL_PREFETCH >= 1 && gl == 0)
-      l2_prefetch(rec + R.S.L.off_vec, (uint32_t)(R.S.L.off_j - R.S.L.off_vec));
-    if (B200_CTRL_PREFETCH >= 2 && gl == 0 && idx_next >= 0)
-      l2_prefetch(rec_of(R.S, R.list_in[idx_next]), (uint32_t)R.S.L.off_j);
     load_cell(c, rec);
-    // the Jacobian and the inverse only when this pass starts with a Newton
-    // iteration (a pass that ends in a setup would fetch them for nothing)
-    if (B200_CTRL_PREFETCH >= 1 && gl == 0 &&
-        (c.label == kLAfterNIter || c.label == kLAfterSetup || (c.label == kLAfterNStart && !c.callSetup)))
-      l2_prefetch(rec + R.S.L.off_j, (uint32_t)(R.S.L.stride - R.S.L.off_j));
-    if (after_rhs) c.cnt.nfe++;
+    // a cell the step kernel passed on as it was consumes its f here
+    if (c.label <= kLAfterSetup) c.cnt.nfe++;
     const RVec<n> v{reinterpret_cast<double*>(rec + R.S.L.off_vec)};
-    need = r_advance<n, G, LUT>(c, v, c.label, P.atol, P.rtol, reinterpret_cast<const double*>(rec + R.S.L.off_j),
-                                reinterpret_cast<const LUT*>(rec + R.S.L.off_a), gl, gm, &status,
-                                sizeof(LUT) == 4 ? P.refine_stall : 0.0, sizeof(LUT) == 4 ? P.refine_keep : 0.0);
+    need = r_advance<n, G>(c, v, c.label, P.atol, P.rtol, gl, gm, &status);
     __syncwarp(gm);
     if (gl == 0) store_cell(c, rec);
     if (need == kDone) {
@@ -510,17 +671,13 @@ __device__ __forceinline__ void ctrl_cell(const RoundsParams& R, bool live, int 
     }
   }
   const bool lead = live && gl == 0;
-  warp_append(lead && need == kNeedRhs, slot, R.list_out, R.cnt_out);
-  warp_append(lead && (need == kNeedSetup || need == kNeedSetupJac), slot, R.list_setup, R.cnt_setup);
-  warp_append(lead && need == kNeedSetupJac, slot, R.list_jac, R.cnt_jac);
+  warp_append_lists(lead ? lists_of(need) : 0, slot, need == kNeedRhs ? slot : (slot | kSetupFlag), R);
   warp_stats(P.stats, lead && need == kDone && status != kStatusRefineStall, status != 0, false, c.cnt);
 }
 
-// Resume the cells of list_in, G lanes per cell.  after_rhs: each consumes
-// the f just evaluated (counted in nfe); otherwise they come back from a
-// setup.
-template <int NS, typename LUT>
-__global__ void __launch_bounds__(128, B200_CTRL_MIN_CTAS) rk_ctrl(RoundsParams R, int after_rhs) {
+// The cells of list_in through the state machine, G lanes per cell.
+template <int NS>
+__global__ void __launch_bounds__(128, B200_CTRL_MIN_CTAS) rk_ctrl(RoundsParams R) {
   constexpr int n = NS + 1;
   constexpr int G = ctrl_group(n);
   constexpr int GPW = 32 / G;  // cells per warp
@@ -532,8 +689,24 @@ __global__ void __launch_bounds__(128, B200_CTRL_MIN_CTAS) rk_ctrl(RoundsParams 
   for (int base = wid * GPW; base < cnt; base += nw * GPW) {
     const int idx = base + gi;
     const bool live = idx < cnt;
-    const int nxt = idx + nw * GPW;
-    ctrl_cell<NS, G, LUT>(R, live, live ? R.list_in[idx] : 0, after_rhs != 0, gl, gm, nxt < cnt ? nxt : -1);
+    ctrl_cell<NS, G>(R, live, live ? R.list_in[idx] : 0, gl, gm);
+  }
+}
+
+// Row i of the inverse into the record, 16 bytes a store: entry j is
+// src[pinv[j]] (the pivot permutation of the columns; pinv = nullptr: none).
+template <int n, typename LUT>
+__device__ __forceinline__ void store_inverse_row(const LUT* src, const int* pinv, LUT* Ar, int i) {
+  constexpr int G = ctrl_group(n), V = vec_of<LUT>();
+#pragma unroll
+  for (int jb = 0; jb < (n + V - 1) / V; ++jb) {
+    __align__(16) LUT t[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const int j = jb * V + e;
+      t[e] = j < n ? src[pinv ? pinv[j] : j] : (LUT)0;
+    }
+    *reinterpret_cast<uint4*>(Ar + mat_vec<n, G, V>(i / G, i % G, jb)) = *reinterpret_cast<const uint4*>(t);
   }
 }
 
@@ -543,11 +716,12 @@ __global__ void __launch_bounds__(128, B200_CTRL_MIN_CTAS) rk_ctrl(RoundsParams 
 // exchanged: step k takes as pivot the unused row p_k with the largest
 // |a[., k]|, and at the end the inverse is (A^-1)[k][j] = X[p_k][q_j] with
 // q_j the step at which row j was the pivot; that permutation is applied
-// while the result is written column-major to Ar.  Xs, prow, pinv: per-warp
+// while the result is written to Ar (mat_idx order).  Xs, prow, pinv: per-warp
 // shared scratch.  Returns 0, or k+1 when no usable pivot is left at step k.
 template <int n, typename LUT>
-__device__ __forceinline__ int reg_gj_inverse(const double* J, int ldj, const double* dsc, double gamma, LUT* Xs,
-                                              int ldl, int* prow, int* pinv, LUT* Ar, int lda, int lane) {
+__device__ __forceinline__ int reg_gj_inverse(const double* J, const double* dsc, double gamma, LUT* Xs, int ldl,
+                                              int* prow, int* pinv, LUT* Ar, int lane) {
+  constexpr int G = ctrl_group(n);
   static_assert(n <= 32, "one row per lane");
   constexpr bool kScaled = sizeof(LUT) == 4;
   const bool row = lane < n;
@@ -555,10 +729,16 @@ __device__ __forceinline__ int reg_gj_inverse(const double* J, int ldj, const do
   const double rdi = 1.0 / di;
   LUT a[n];
 #pragma unroll
-  for (int j = 0; j < n; ++j) {
-    const double rdj = __shfl_sync(kFull, rdi, j);
-    const double mij = ((lane == j) ? 1.0 : 0.0) - gamma * (row ? J[j * ldj + lane] : 0.0);
-    a[j] = row ? (LUT)(kScaled ? mij * di * rdj : mij) : (LUT)0;
+  for (int jb = 0; jb < n / kVJ; ++jb) {
+    double2 jv = make_double2(0.0, 0.0);
+    if (row) jv = *reinterpret_cast<const double2*>(J + mat_vec<n, G, kVJ>(lane / G, lane % G, jb));
+#pragma unroll
+    for (int e = 0; e < kVJ; ++e) {
+      const int j = jb * kVJ + e;
+      const double rdj = __shfl_sync(kFull, rdi, j);
+      const double mij = ((lane == j) ? 1.0 : 0.0) - gamma * (e ? jv.y : jv.x);
+      a[j] = row ? (LUT)(kScaled ? mij * di * rdj : mij) : (LUT)0;
+    }
   }
   // Pivot search by one warp reduction: key = the bits of |a[k]| (FP32; the
   // high word for FP64) with the low 5 bits replaced by (31 - lane), so the
@@ -619,12 +799,7 @@ __device__ __forceinline__ int reg_gj_inverse(const double* J, int ldj, const do
     prow[mystep] = lane;
   }
   __syncwarp();
-  if (lane < n) {
-    const int pk = prow[lane];
-    for (int j = 0; j < n; ++j) Ar[j * lda + lane] = Xs[pk * ldl + pinv[j]];
-  } else if (lane < lda) {
-    for (int j = 0; j < n; ++j) Ar[j * lda + lane] = (LUT)0;  // column padding
-  }
+  if (lane < n) store_inverse_row<n, LUT>(Xs + prow[lane] * ldl, pinv, Ar, lane);
   __syncwarp();
   return 0;
 }
@@ -634,8 +809,9 @@ __device__ __forceinline__ int reg_gj_inverse(const double* J, int ldj, const do
 // lane; the pivot row's owner writes it to shared memory and every lane
 // updates both of its rows from 16-byte reads of it.
 template <int n, typename LUT>
-__device__ __forceinline__ int reg_gj_inverse2(const double* J, int ldj, const double* dsc, double gamma, LUT* Xs,
-                                               int ldl, int* prow, int* pinv, LUT* Ar, int lda, int lane) {
+__device__ __forceinline__ int reg_gj_inverse2(const double* J, const double* dsc, double gamma, LUT* Xs, int ldl,
+                                               int* prow, int* pinv, LUT* Ar, int lane) {
+  constexpr int G = ctrl_group(n);
   static_assert(n > 32 && n <= 64 && sizeof(LUT) == 4, "two FP32 rows per lane");
   const int r1 = lane + 32;
   const bool row1 = r1 < n;
@@ -643,12 +819,19 @@ __device__ __forceinline__ int reg_gj_inverse2(const double* J, int ldj, const d
   const double rd0 = 1.0 / d0, rd1 = 1.0 / d1;
   LUT a0[n], a1[n];
 #pragma unroll
-  for (int j = 0; j < n; ++j) {
-    const double rdj = (j < 32) ? __shfl_sync(kFull, rd0, j) : __shfl_sync(kFull, rd1, j - 32);
-    const double m0 = ((lane == j) ? 1.0 : 0.0) - gamma * J[j * ldj + lane];
-    const double m1 = row1 ? ((r1 == j) ? 1.0 : 0.0) - gamma * J[j * ldj + r1] : 0.0;
-    a0[j] = (LUT)(m0 * d0 * rdj);
-    a1[j] = row1 ? (LUT)(m1 * d1 * rdj) : (LUT)0;
+  for (int jb = 0; jb < n / kVJ; ++jb) {
+    const double2 j0 = *reinterpret_cast<const double2*>(J + mat_vec<n, G, kVJ>(lane / G, lane % G, jb));
+    double2 j1 = make_double2(0.0, 0.0);
+    if (row1) j1 = *reinterpret_cast<const double2*>(J + mat_vec<n, G, kVJ>(r1 / G, r1 % G, jb));
+#pragma unroll
+    for (int e = 0; e < kVJ; ++e) {
+      const int j = jb * kVJ + e;
+      const double rdj = (j < 32) ? __shfl_sync(kFull, rd0, j) : __shfl_sync(kFull, rd1, j - 32);
+      const double m0 = ((lane == j) ? 1.0 : 0.0) - gamma * (e ? j0.y : j0.x);
+      const double m1 = row1 ? ((r1 == j) ? 1.0 : 0.0) - gamma * (e ? j1.y : j1.x) : 0.0;
+      a0[j] = (LUT)(m0 * d0 * rdj);
+      a1[j] = row1 ? (LUT)(m1 * d1 * rdj) : (LUT)0;
+    }
   }
   constexpr int kChunks = (n + 3) / 4;
   constexpr int kBuf = 64;
@@ -732,12 +915,7 @@ __device__ __forceinline__ int reg_gj_inverse2(const double* J, int ldj, const d
   __syncwarp();
   for (int h = 0; h < 2; ++h) {
     const int i = lane + 32 * h;
-    if (i < n) {
-      const int pk = prow[i];
-      for (int j = 0; j < n; ++j) Ar[j * lda + i] = Xs[pk * ldl + pinv[j]];
-    } else if (i < lda) {
-      for (int j = 0; j < n; ++j) Ar[j * lda + i] = (LUT)0;  // column padding
-    }
+    if (i < n) store_inverse_row<n, LUT>(Xs + prow[i] * ldl, pinv, Ar, i);
   }
   __syncwarp();
   return 0;
@@ -750,13 +928,15 @@ __device__ __forceinline__ int reg_gj_inverse2(const double* J, int ldj, const d
 // third-body terms (the default efficiency 1 of every species as a row
 // vector u added to all columns at the end, the non-default ones per
 // species).  Then lane l finishes column l (mass units) and its temperature
-// row entry, and writes the column into the cell record (column-major, ldj).
+// row entry in shared memory, and the warp writes the matrix into the cell
+// record (mat_idx order, consecutive 16-byte stores).
 // s: C, g/RT, h/RT [Npad]; Js: [n][n] column-major; us: [Npad] (shared).
-template <int CPL>
+template <int n, int CPL>
 __device__ __forceinline__ void warp_jac(const DevMech& m, const GrpScratch& s, double* Js, double* us,
-                                         const Vec<CPL>& y, const Vec<CPL>& fy, double* J, int ldj, int lane) {
+                                         const Vec<CPL>& y, const Vec<CPL>& fy, double* J, int lane) {
   const Grp<32> g(lane);
-  const int N = m.N, R = m.R, n = N + 1;
+  constexpr int N = n - 1;
+  const int R = m.R;
   const double T = grp_get_T<32, CPL>(g, y, N);
   const double lnT = log(T), invT = 1.0 / T;
   double cpk[CPL], hk[CPL], dcpk[CPL];
@@ -850,22 +1030,33 @@ __device__ __forceinline__ void warp_jac(const DevMech& m, const GrpScratch& s, 
     const int l = lane + 32 * c;
     if (l > N) continue;
     const double inv_wl = (l < N) ? __ldg(m.inv_mw + l) : 1.0;
-    const double* src = Js + l * n;
-    double* dst = J + l * ldj;
+    double* col = Js + l * n;
     double sum = 0.0;
     for (int k = 0; k < N; ++k) {
-      const double v = (src[k] + ((l < N) ? us[k] : 0.0)) * __ldg(m.mw + k) * inv_wl;
-      dst[k] = v;
+      const double v = (col[k] + ((l < N) ? us[k] : 0.0)) * __ldg(m.mw + k) * inv_wl;
+      col[k] = v;
       sum += s.hRT[k] * v;
     }
-    dst[N] = -(sum + ((l < N) ? Tdot * cpk[c] : cpdot + Tdot * drcp)) / rcp;
+    col[N] = -(sum + ((l < N) ? Tdot * cpk[c] : cpdot + Tdot * drcp)) / rcp;
+  }
+  __syncwarp();
+  constexpr int G = ctrl_group(n), JB = n / kVJ;
+  static_assert(n % kVJ == 0, "no column padding in J");
+#pragma unroll
+  for (int cc = 0; cc < (n + G - 1) / G; ++cc) {
+    const int rows = (n - cc * G < G) ? n - cc * G : G;
+    double2* dst = reinterpret_cast<double2*>(J + mat_vec<n, G, kVJ>(cc, 0, 0));
+    for (int t = lane; t < rows * JB; t += 32) {
+      const int jb = t / rows, i = cc * G + t % rows;
+      dst[t] = make_double2(Js[(jb * kVJ) * n + i], Js[(jb * kVJ + 1) * n + i]);
+    }
   }
   __syncwarp();
 }
 
 // Jacobian refresh for the cells of the setup list whose matrix CVODE's
-// jbad rule marks stale: the analytic FP64 Jacobian (column-major) into the
-// cell record, one warp per cell.
+// jbad rule marks stale: the analytic FP64 Jacobian into the cell record, one
+// warp per cell.
 // Minimum resident CTAs per SM requested for the Jacobian kernel (bounds
 // its registers per thread; n > 32 keeps 2: its shared memory allows no
 // more).
@@ -897,17 +1088,17 @@ __global__ void __launch_bounds__(128, CPL == 1 ? B200_JAC_MIN_CTAS : 2) rk_jac(
   for (long long idx = gw; idx < cnt; idx += nwarps) {
     const int slot = R.list_in[idx];
     unsigned char* rec = rec_of(R.S, slot);
-    // the control kernel chose these cells by CVODE's jbad rule and already
-    // counted the refresh
+    // the cells were chosen by CVODE's jbad rule at their prediction, which
+    // already counted the refresh
     const RVec<n> v{reinterpret_cast<double*>(rec + RL.off_vec)};
     Vec<CPL> y, fy;
 #pragma unroll
     for (int cc = 0; cc < CPL; ++cc) {
       const int i = lane + 32 * cc;
       y.v[cc] = (i < n) ? v.yev(i) : 0.0;
-      fy.v[cc] = (i < n) ? v.ftemp(i) : 0.0;
+      fy.v[cc] = (i < n) ? v.fv(i) : 0.0;
     }
-    warp_jac<CPL>(s_mech, ms, Js, us, y, fy, reinterpret_cast<double*>(rec + RL.off_j), RL.ldj, lane);
+    warp_jac<n, CPL>(s_mech, ms, Js, us, y, fy, reinterpret_cast<double*>(rec + RL.off_j), lane);
     __syncwarp();
   }
 }
@@ -920,7 +1111,7 @@ __global__ void __launch_bounds__(128, CPL == 1 ? B200_JAC_MIN_CTAS : 2) rk_jac(
 
 // Newton-matrix inverse of the cells of the setup list, one warp per cell:
 // Gauss-Jordan inverse of D (I - gamma J) D^-1 with D = diag(ewt) (FP32) or
-// of I - gamma J (FP64), written column-major into the cell record.
+// of I - gamma J (FP64), written into the cell record.
 template <int NS, typename LUT, int CPL>
 __global__ void __launch_bounds__(128, CPL == 1 ? B200_GJ_MIN_CTAS : 2) rk_gj(RoundsParams R) {
   constexpr int n = NS + 1;
@@ -957,21 +1148,21 @@ __global__ void __launch_bounds__(128, CPL == 1 ? B200_GJ_MIN_CTAS : 2) rk_gj(Ro
     __syncwarp();
     int ier;
     if constexpr (CPL == 1) {
-      ier = reg_gj_inverse<(CPL == 1 ? n : 1), LUT>(J, RL.ldj, Dsc, gamma, A, SL.ldl, ipiv, ipiv2, Ar, RL.lda,
-                                                    lane);
+      ier = reg_gj_inverse<(CPL == 1 ? n : 2), LUT>(J, Dsc, gamma, A, SL.ldl, ipiv, ipiv2, Ar, lane);
     } else if constexpr (CPL == 2 && sizeof(LUT) == 4) {
-      ier = reg_gj_inverse2<(CPL == 2 ? n : 33), LUT>(J, RL.ldj, Dsc, gamma, A, SL.ldl, ipiv, ipiv2, Ar, RL.lda,
-                                                      lane);
+      ier = reg_gj_inverse2<(CPL == 2 ? n : 34), LUT>(J, Dsc, gamma, A, SL.ldl, ipiv, ipiv2, Ar, lane);
     } else {
-      ier = grp_gj_inverse<32, LUT>(J, RL.ldj, A, SL.ldl, ipiv, fcol, Dsc, n, gamma, lane);
+      static_assert(sizeof(LUT) == 8, "the unscaled matrix");
+      constexpr int G = ctrl_group(n);
+      for (int e = lane; e < n * n; e += 32) {
+        const int i = e / n, j = e % n;
+        A[i * SL.ldl + j] = ((i == j) ? 1.0 : 0.0) - gamma * J[mat_idx<n, G, kVJ>(i, j)];
+      }
+      __syncwarp();
+      ier = grp_gj_eliminate<32, LUT>(A, SL.ldl, ipiv, fcol, n, lane);
       __syncwarp();
       if (ier == 0)
-        for (int j = 0; j < n; ++j)
-#pragma unroll
-          for (int cc = 0; cc < CPL; ++cc) {
-            const int i = lane + 32 * cc;
-            if (i < n) Ar[j * RL.lda + i] = A[i * SL.ldl + j];
-          }
+        for (int i = lane; i < n; i += 32) store_inverse_row<n, LUT>(A + i * SL.ldl, nullptr, Ar, i);
     }
     __syncwarp();
     if (lane == 0) {
@@ -1002,6 +1193,8 @@ cudaError_t rounds_setup_attrs(const RoundsSetupLayout& SL) {
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(rk_jac<NS, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * SL.jac_smem_per_warp);
   if (e != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(rk_step<NS, LUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, step_smem<n>());
+  if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(rk_gj<NS, LUT, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               4 * SL.gj_smem_per_warp);
 }
@@ -1018,7 +1211,11 @@ cudaError_t rounds_grids(const RoundsSetupLayout& SL, int sm_count, RoundsGrids*
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rk_rhs<NS>, kRoundsRhsBlock, 0)) != cudaSuccess)
     return e;
   G->rhs = std::max(1, b) * sm_count;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rk_ctrl<NS, LUT>, 128, 0)) != cudaSuccess) return e;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rk_step<NS, LUT>, 128, step_smem<n>())) !=
+      cudaSuccess)
+    return e;
+  G->step = std::max(1, b) * sm_count;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rk_ctrl<NS>, 128, 0)) != cudaSuccess) return e;
   G->ctrl = std::max(1, b) * sm_count;
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rk_jac<NS, CPL>, 128, 4 * SL.jac_smem_per_warp)) !=
       cudaSuccess)
@@ -1033,7 +1230,7 @@ cudaError_t rounds_grids(const RoundsSetupLayout& SL, int sm_count, RoundsGrids*
 }
 
 template <int NS, typename LUT>
-cudaError_t rounds_launch_t(int what, const RoundsParams& R, const RoundsGrids& G, int after_rhs, cudaStream_t st) {
+cudaError_t rounds_launch_t(int what, const RoundsParams& R, const RoundsGrids& G, int setup_pass, cudaStream_t st) {
   constexpr int n = NS + 1;
   constexpr int CPL = (n + 31) / 32;
   switch (what) {
@@ -1044,8 +1241,11 @@ cudaError_t rounds_launch_t(int what, const RoundsParams& R, const RoundsGrids& 
       // the generated right-hand side keeps everything in registers
       rk_rhs<NS><<<G.rhs, kRoundsRhsBlock, R.gen_mech ? 0 : rhs_smem<NS>(kRoundsRhsBlock), st>>>(R);
       break;
+    case kRoundsStep:
+      rk_step<NS, LUT><<<G.step, 128, step_smem<n>(), st>>>(R, setup_pass);
+      break;
     case kRoundsCtrl:
-      rk_ctrl<NS, LUT><<<G.ctrl, 128, 0, st>>>(R, after_rhs);
+      rk_ctrl<NS><<<G.ctrl, 128, 0, st>>>(R);
       break;
     case kRoundsJac:
       rk_jac<NS, CPL><<<G.jac, 128, 4 * R.SL.jac_smem_per_warp, st>>>(R);
@@ -1077,7 +1277,7 @@ RoundsSetupLayout rounds_setup_layout(int N, int R, int lut_bytes) {
 }
 
 long long rounds_state_bytes_per_cell(int N, int lut_bytes) {
-  return rounds_record_layout(N + 1, lut_bytes).stride + 4LL * 4;  // record + four slot lists
+  return rounds_record_layout(N + 1, lut_bytes).stride + 4LL * kRoundSlotLists;  // record + slot lists
 }
 
 RState rounds_carve(void* base, long long cap, int N, int lut_bytes) {
@@ -1097,17 +1297,17 @@ cudaError_t rounds_grids_for(int N, int lut_bytes, const RoundsSetupLayout& SL, 
   return cudaErrorInvalidValue;
 }
 
-cudaError_t rounds_launch(int N, int lut_bytes, int what, const RoundsParams& R, const RoundsGrids& G, int after_rhs,
+cudaError_t rounds_launch(int N, int lut_bytes, int what, const RoundsParams& R, const RoundsGrids& G, int setup_pass,
                           cudaStream_t st) {
   if (N == 9)
-    return lut_bytes == 4 ? rounds_launch_t<9, float>(what, R, G, after_rhs, st)
-                          : rounds_launch_t<9, double>(what, R, G, after_rhs, st);
+    return lut_bytes == 4 ? rounds_launch_t<9, float>(what, R, G, setup_pass, st)
+                          : rounds_launch_t<9, double>(what, R, G, setup_pass, st);
   if (N == 21)
-    return lut_bytes == 4 ? rounds_launch_t<21, float>(what, R, G, after_rhs, st)
-                          : rounds_launch_t<21, double>(what, R, G, after_rhs, st);
+    return lut_bytes == 4 ? rounds_launch_t<21, float>(what, R, G, setup_pass, st)
+                          : rounds_launch_t<21, double>(what, R, G, setup_pass, st);
   if (N == 53)
-    return lut_bytes == 4 ? rounds_launch_t<53, float>(what, R, G, after_rhs, st)
-                          : rounds_launch_t<53, double>(what, R, G, after_rhs, st);
+    return lut_bytes == 4 ? rounds_launch_t<53, float>(what, R, G, setup_pass, st)
+                          : rounds_launch_t<53, double>(what, R, G, setup_pass, st);
   return cudaErrorInvalidValue;
 }
 
