@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "jac_table.h"
 #include "react_group.cuh"
 
 using namespace b200;
@@ -247,6 +248,7 @@ struct b200chem_reactor {
   long long launches = 0;  // kernels launched by this handle (instrumentation)
   unsigned char* h_cmech = nullptr;  // pinned packed constant-memory table (null: too large)
   int cmech_bytes = 0;
+  bool jac_table = false;  // the mechanism fits the round integrator's Jacobian table
   int gen_mech = 0;  // 1: a generated right-hand side matches the mechanism
   unsigned long long digest = 0;  // FNV-1a digest of the mechanism description
   b200chem_tuning tune{};           // launch shape of the round-based integrator
@@ -532,10 +534,11 @@ int launch_rounds(b200chem_reactor* h, const ReactParams& P, cudaStream_t st, in
   if (!rounds_supported(h->N))
     return set_err(B200CHEM_EINVAL, "round-based integrator not compiled for N=%d", h->N);
   const int lut = force_lut ? force_lut : (h->opts.lu_fp64 ? 8 : 4);
-  const RoundsSetupLayout SL = rounds_setup_layout(h->N, h->R, lut);
-  if (4 * std::max(SL.jac_smem_per_warp, SL.gj_smem_per_warp) > h->smem_optin - 2048)
+  if (!h->jac_table) return set_err(B200CHEM_ETOOBIG, "mechanism too large for the round-based integrator");
+  const RoundsSetupLayout SL = rounds_setup_layout(h->N, lut, h->mech.jt_nd);
+  if (std::max(SL.jac_smem, 4 * SL.gj_smem_per_warp) > h->smem_optin - 2048)
     return set_err(B200CHEM_ETOOBIG, "setup kernels need %d B of shared memory per CTA",
-                   4 * std::max(SL.jac_smem_per_warp, SL.gj_smem_per_warp));
+                   std::max(SL.jac_smem, 4 * SL.gj_smem_per_warp));
   if (h->rgrid_lut != lut) {
     CK(rounds_grids_for(h->N, lut, SL, h->sm_count, &h->rgrid));
     h->rgrid_lut = lut;
@@ -560,8 +563,7 @@ int launch_rounds(b200chem_reactor* h, const ReactParams& P, cudaStream_t st, in
   const size_t state_bytes = (size_t)per_cell * cap + 16 * 256;
   int err = ensure_buffer(&h->d_rounds, &h->rounds_bytes, state_bytes, st, "round-integrator state");
   if (err) return err;
-  err = ensure_buffer(&h->d_rwarp, &h->rwarp_bytes, (size_t)h->rgrid.jac * 4 * SL.gbytes_per_warp, st,
-                      "setup scratch");
+  err = ensure_buffer(&h->d_rwarp, &h->rwarp_bytes, (size_t)h->rgrid.jac * SL.gbytes_per_cta, st, "setup scratch");
   if (err) return err;
   if (!h->d_rcnt) {
     CK(cudaMalloc(&h->d_rcnt, 2 * kRoundLists * sizeof(int)));
@@ -670,7 +672,7 @@ int do_react(b200chem_reactor* h, const std::vector<DevBox>& boxes, long long to
   if (total > 0) {
     // auto: the round-based integrator where its species count is compiled,
     // else the group integrator (any species count)
-    const int k = (h->opts.kernel == 0) ? (rounds_supported(h->N) ? 3 : 2) : h->opts.kernel;
+    const int k = (h->opts.kernel == 0) ? (rounds_supported(h->N) && h->jac_table ? 3 : 2) : h->opts.kernel;
     const int ppm = h->opts.refine_stall_ppm;
     const int keep = h->opts.refine_keep_ppm;
     if (k == 3 && !h->opts.lu_fp64 && keep > 0) P.refine_keep = keep * 1e-6;
@@ -968,7 +970,14 @@ b200chem_handle b200chem_create(const b200chem_mech_desc* md, const b200chem_opt
       memcpy(cblob.data() + hd.off_effm1, effm1.data(), sizeof(double) * effm1.size());
     }
   }
+  // the round integrator's Jacobian table; a mechanism it cannot hold runs on
+  // the group integrator
+  JacTable jt;
+  h->jac_table = build_jac_table(N, R, rtype.data(), sp.data(), nu.data(), effptr.data(), effsp.data(), effm1.data(),
+                                 (N + 1) | 1, kJtCoefBits, &jt);
   std::vector<unsigned char> buf;
+  size_t o_jtd = push(buf, jt.dptr), o_jto = push(buf, jt.off), o_jtt = push(buf, jt.tgt), o_jtm = push(buf, jt.term),
+         o_jtc = push(buf, jt.coef);
   size_t o_mw = push(buf, mw), o_imw = push(buf, imw), o_nasa = push(buf, nasa), o_rtype = push(buf, rtype),
          o_rflags = push(buf, rflags), o_arr = push(buf, arr), o_arrlo = push(buf, arrlo),
          o_arrrev = push(buf, arrrev), o_troe = push(buf, troe), o_sp = push(buf, sp), o_nu = push(buf, nu),
@@ -1016,6 +1025,13 @@ b200chem_handle b200chem_create(const b200chem_mech_desc* md, const b200chem_opt
   m.inc_ptr = reinterpret_cast<const int*>(base + o_incptr);
   m.inc_rxn = reinterpret_cast<const int*>(base + o_incrxn);
   m.inc_nu = reinterpret_cast<const double*>(base + o_incnu);
+  m.jt_slices = jt.slices;
+  m.jt_nd = jt.nd;
+  m.jt_dptr = reinterpret_cast<const int*>(base + o_jtd);
+  m.jt_off = reinterpret_cast<const int*>(base + o_jto);
+  m.jt_tgt = reinterpret_cast<const int*>(base + o_jtt);
+  m.jt_term = reinterpret_cast<const unsigned*>(base + o_jtm);
+  m.jt_coef = reinterpret_cast<const double*>(base + o_jtc);
   if (!cblob.empty()) {
     if ((e = cudaMallocHost(&h->h_cmech, cblob.size())) != cudaSuccess) return fail(e, "cudaMallocHost(table)");
     memcpy(h->h_cmech, cblob.data(), cblob.size());
@@ -1513,7 +1529,7 @@ int b200chem_autotune(b200chem_handle h, const double* rhoY, const double* extF_
   if (!h || ncells <= 0 || !rhoY || !extF_rhoY || !T || !rhoH || !extF_rhoH)
     return set_err(B200CHEM_EINVAL, "bad arguments");
   if (!(dt_react > 0.0)) return set_err(B200CHEM_EINVAL, "dt_react must be positive");
-  const int kern = (h->opts.kernel == 0) ? (rounds_supported(h->N) ? 3 : 2) : h->opts.kernel;
+  const int kern = (h->opts.kernel == 0) ? (rounds_supported(h->N) && h->jac_table ? 3 : 2) : h->opts.kernel;
   if (kern != 3) return set_err(B200CHEM_EINVAL, "the autotuner tunes the round-based integrator (kernel 0 or 3)");
   if (max_trials <= 0) max_trials = 48;
   const cudaStream_t st = static_cast<cudaStream_t>(stream);

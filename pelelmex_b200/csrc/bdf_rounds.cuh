@@ -1133,8 +1133,7 @@ __device__ __forceinline__ void r_begin(RCell& c, const RVec<n>& v, const double
   for (int i = 0; i < kZn; ++i) c.l[i] = 0.0;
 #pragma unroll 2
   for (int i = 0; i < n; ++i) {
-    for (int j = 1; j < kZn; ++j) v.zn(j, i) = 0.0;
-    v.yev(i) = v.zn(0, i);
+    v.yev(i) = v.zn(0, i);  // the higher columns are written before they are read
   }
   r_set_ewt<n, 1>(v, atolv, rtol, 0);
   c.label = kLAfterF0;

@@ -144,14 +144,16 @@ cudaError_t tpc_launch(int N, int lut_bytes, const ReactParams& P, const TpcPara
 constexpr int kRoundsRhsBlock = 64;  // threads per CTA of the rhs kernel
 enum { kRoundsStart = 0, kRoundsRhs, kRoundsStep, kRoundsJac, kRoundsGj, kRoundsCtrl };
 
-// Per-warp shared scratch of the setup kernels.  Jacobian kernel: C, g/RT,
-// h/RT, third-body row [Npad] and the Jacobian [n][n] (double).
-// Inverse kernel: Dsc [Npad] (double), matrix [n][ldl] and pivot column
-// [Npad] (LUT), two index arrays [Npad] (int).
+// Scratch of the setup kernels.  Jacobian kernel, per team of warps: C, g/RT,
+// h/RT, hm [Npad], the Jacobian, the third-body row and the temperature row,
+// and the reactions' derivatives [jac_nd] (here or in device memory).
+// Inverse kernel, per warp: Dsc [Npad] (double), matrix [n][ldl] and pivot
+// column [Npad] (LUT), two index arrays [Npad] (int), or the lane groups' form.
 struct RoundsSetupLayout {
-  int Npad, Rpad, ldl;
-  int jac_smem_per_warp, gj_smem_per_warp;
-  long long gbytes_per_warp;
+  int Npad, ldl;
+  int jac_nd, jac_d_global, jac_smem_per_team, jac_smem;
+  int gj_smem_per_warp;
+  long long gbytes_per_cta;  // device memory per CTA of the Jacobian kernel
 };
 
 // Lists a round's kernels append to: cells that need a right-hand side next
@@ -174,7 +176,7 @@ struct RoundsParams {
   const int* cnt_in;
   int* list[kRoundLists];  // lists the kernel appends to (the kRl* indices)
   int* cnt_next;           // their counters [kRoundLists]; cleared by the right-hand-side kernel
-  unsigned char* wscratch;  // [setup warps][SL.gbytes_per_warp]
+  unsigned char* wscratch;  // [CTAs of the Jacobian kernel][SL.gbytes_per_cta]
   int const_mech;           // 1: the packed table is in the constant bank
   int gen_mech;             // 1: the mechanism has a generated right-hand side
 };
@@ -194,7 +196,7 @@ unsigned long long handle_digest(b200chem_handle h);  // FNV-1a digest of the me
 int handle_sm_count(b200chem_handle h);
 
 bool rounds_supported(int N);
-RoundsSetupLayout rounds_setup_layout(int N, int R, int lut_bytes);
+RoundsSetupLayout rounds_setup_layout(int N, int lut_bytes, int jac_nd);
 long long rounds_state_bytes_per_cell(int N, int lut_bytes);
 rounds::RState rounds_carve(void* base, long long cap, int N, int lut_bytes);
 cudaError_t rounds_grids_for(int N, int lut_bytes, const RoundsSetupLayout& SL, int sm_count, RoundsGrids* G);

@@ -39,7 +39,16 @@ struct DevMech {
   const int* inc_ptr;    // [N+1] species -> (reaction, net nu) incidence
   const int* inc_rxn;    // [nnz]
   const double* inc_nu;  // [nnz]
+  // Jacobian table (JacTable in jac_table.h): entries in slices of 32, each a
+  // sum of coefficient * derivative terms
+  int jt_slices, jt_nd;
+  const int* jt_dptr;        // [R] first derivative of a reaction
+  const int* jt_off;         // [slices + 1] first term row of a slice
+  const int* jt_tgt;         // [slices][32] where the entry's sum goes (-1: nowhere)
+  const unsigned* jt_term;   // [term rows][32] derivative index << kJtCoefBits | coefficient
+  const double* jt_coef;
 };
+constexpr int kJtCoefBits = 12, kJtCoefs = 1 << kJtCoefBits;
 
 // Species-indexed views used by the per-reaction evaluation (unit stride).
 struct SpView {

@@ -693,6 +693,12 @@ __global__ void __launch_bounds__(128, B200_CTRL_MIN_CTAS) rk_ctrl(RoundsParams 
   }
 }
 
+// Shared memory of one cell of the lane-group inversion: 1 / dsc [n], the
+// matrix [n][n | 1] (FP32) and two index arrays [n].
+__host__ __device__ constexpr int gj_cell_bytes(int n) {
+  return 8 * n + 4 * ((n * (n | 1) + 3) / 4 * 4) + (8 * n + 15) / 16 * 16;
+}
+
 // Row i of the inverse into the record, 16 bytes a store: entry j is
 // src[pinv[j]] (the pivot permutation of the columns; pinv = nullptr: none).
 template <int n, typename LUT>
@@ -749,20 +755,23 @@ __device__ __forceinline__ int reg_gj_inverse(const double* J, const double* dsc
   // by one FMA per column: a_ij -= g_i * a_pj with g_i = a_ik / a_pk off the
   // pivot row and g_p = 1 - 1 / a_pk on it (which scales the pivot row by
   // 1 / a_pk); column k is set last (1 / a_pk on the pivot row, -g_i off it).
+  // The columns rotate by one register per step, so that column k is always
+  // a[0] and the loop needs no unrolling (unrolled, the 54-step form is 150 KB
+  // of code and waits for instructions: 766,122 inverses 38 ms, now 26).
   constexpr int kVec = 16 / (int)sizeof(LUT);      // LUTs per 16-byte chunk
   constexpr int kChunks = (n + kVec - 1) / kVec;
   constexpr int kBuf = 32;                         // LUTs per row buffer (>= kChunks * kVec)
   static_assert(kChunks * kVec <= kBuf, "row buffer");
   unsigned used = 0;
   int mystep = -1;
-#pragma unroll
+#pragma unroll 1
   for (int k = 0; k < n; ++k) {
     LUT* buf = Xs + (k & 1) * kBuf;
     unsigned key = 0u;
     if (row && !((used >> lane) & 1u)) {
       unsigned bits;
-      if constexpr (sizeof(LUT) == 4) bits = __float_as_uint(fabsf((float)a[k]));
-      else bits = (unsigned)__double2hiint(fabs((double)a[k]));
+      if constexpr (sizeof(LUT) == 4) bits = __float_as_uint(fabsf((float)a[0]));
+      else bits = (unsigned)__double2hiint(fabs((double)a[0]));
       key = (bits & ~31u) | (unsigned)(31 - lane);
     }
     const unsigned kmax = __reduce_max_sync(kFull, key);
@@ -783,14 +792,13 @@ __device__ __forceinline__ int reg_gj_inverse(const double* J, const double* dsc
     LUT pr[kChunks * kVec];
 #pragma unroll
     for (int c = 0; c < kChunks; ++c) *reinterpret_cast<uint4*>(pr + c * kVec) = *reinterpret_cast<const uint4*>(buf + c * kVec);
-    const LUT pv = pr[k];
+    const LUT pv = pr[0];
     if (!(fabs(pv) > (LUT)0) || isnan(pv)) return k + 1;  // zero or NaN pivot (warp-uniform)
     const LUT inv = (LUT)1 / pv;
-    const LUT gi = (lane == p) ? (LUT)1 - inv : a[k] * inv;
+    const LUT gi = (lane == p) ? (LUT)1 - inv : a[0] * inv;
 #pragma unroll
-    for (int j = 0; j < n; ++j)
-      if (j != k) a[j] = fma(-gi, pr[j], a[j]);
-    a[k] = (lane == p) ? inv : -gi;
+    for (int j = 1; j < n; ++j) a[j - 1] = fma(-gi, pr[j], a[j]);
+    a[n - 1] = (lane == p) ? inv : -gi;
   }
   if (row) {
 #pragma unroll
@@ -802,6 +810,131 @@ __device__ __forceinline__ int reg_gj_inverse(const double* J, const double* dsc
   if (lane < n) store_inverse_row<n, LUT>(Xs + prow[lane] * ldl, pinv, Ar, lane);
   __syncwarp();
   return 0;
+}
+
+// The same inverse for n <= 32 in FP32 by a group of G lanes per cell, lane g
+// holding rows g, g + G, ... in registers: a pivot step costs its search, its
+// exchange and its reciprocal once for the 32 / G cells of a warp, and a row
+// chunk read from shared memory feeds every row of the lane.  All lanes of the
+// warp call it; a group without a cell (live false) works on zeros.  Xs: two
+// alternating pivot-row buffers, then the n x ldl result; rds: 1 / dsc [n].
+// Bound by the latency of a pivot step (16 warps per SM, three quarters of the
+// stalls wait for the previous one): 17.4 M inverses of 22 x 22 take 58 ms, 73
+// with one warp and 32 unrolled steps per cell.
+// Returns 0, or k+1 when no usable pivot is left at step k.
+template <int n, int G>
+__device__ __forceinline__ int grp_reg_gj_inverse(const double* J, bool live, const double (&di)[(n + G - 1) / G],
+                                                  double* rds, double gamma, float* Xs, int* prow, int* pinv,
+                                                  float* Ar, int gl) {
+  static_assert(n <= 32, "the pivot key holds five bits of the row");
+  constexpr int CPL = (n + G - 1) / G;
+  constexpr int ldl = n | 1;
+  constexpr int kChunks = (n + 3) / 4, kBuf = 4 * kChunks;
+#pragma unroll
+  for (int cc = 0; cc < CPL; ++cc) {
+    const int i = gl + G * cc;
+    if (i < n) rds[i] = 1.0 / di[cc];
+  }
+  __syncwarp();
+  float a[CPL][n];
+#pragma unroll
+  for (int cc = 0; cc < CPL; ++cc) {
+    const int i = gl + G * cc;
+#pragma unroll
+    for (int jb = 0; jb < n / kVJ; ++jb) {
+      double2 jv = make_double2(0.0, 0.0);
+      if (live && i < n) jv = *reinterpret_cast<const double2*>(J + mat_vec<n, G, kVJ>(cc, gl, jb));
+#pragma unroll
+      for (int e = 0; e < kVJ; ++e) {
+        const int j = jb * kVJ + e;
+        const double mij = ((i == j) ? 1.0 : 0.0) - gamma * (e ? jv.y : jv.x);
+        a[cc][j] = (i < n) ? (float)(mij * di[cc] * rds[j]) : 0.0f;
+      }
+    }
+  }
+  unsigned used = 0;  // bit cc: this lane's row cc was a pivot
+  int step[CPL], ier = 0;
+#pragma unroll
+  for (int cc = 0; cc < CPL; ++cc) step[cc] = 0;
+#pragma unroll 1
+  for (int k = 0; k < n; ++k) {
+    float* buf = Xs + (k & 1) * kBuf;
+    unsigned key = 0u;
+#pragma unroll
+    for (int cc = 0; cc < CPL; ++cc) {
+      const int i = gl + G * cc;
+      if (i < n && !((used >> cc) & 1u)) {
+        const unsigned kk = (__float_as_uint(fabsf(a[cc][0])) & ~31u) | (unsigned)(31 - i);
+        key = key > kk ? key : kk;
+      }
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+      const unsigned t = __shfl_xor_sync(kFull, key, o, G);
+      key = key > t ? key : t;
+    }
+    if (ier == 0 && (key >> 5) == 0u) ier = k + 1;  // no nonzero candidate: singular (group-uniform)
+    const int p = 31 - (int)(key & 31u);
+#pragma unroll
+    for (int cc = 0; cc < CPL; ++cc) {
+      if (p == gl + G * cc) {
+        used |= 1u << cc;
+        step[cc] = k;
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) {
+          float4 t;
+          t.x = a[cc][4 * c];
+          t.y = (4 * c + 1 < n) ? a[cc][4 * c + 1 < n ? 4 * c + 1 : 0] : 0.f;
+          t.z = (4 * c + 2 < n) ? a[cc][4 * c + 2 < n ? 4 * c + 2 : 0] : 0.f;
+          t.w = (4 * c + 3 < n) ? a[cc][4 * c + 3 < n ? 4 * c + 3 : 0] : 0.f;
+          reinterpret_cast<float4*>(buf)[c] = t;
+        }
+      }
+    }
+    __syncwarp();
+    const float pv = buf[0];
+    if (ier == 0 && (!(fabsf(pv) > 0.f) || isnan(pv))) ier = k + 1;  // zero or NaN pivot (group-uniform)
+    const float inv = 1.f / pv;
+    float gf[CPL];
+#pragma unroll
+    for (int cc = 0; cc < CPL; ++cc) gf[cc] = (p == gl + G * cc) ? 1.f - inv : a[cc][0] * inv;
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c) {
+      const float4 q = reinterpret_cast<const float4*>(buf)[c];
+      const float qv[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int j = 4 * c + e;
+        if (j < n && j > 0) {
+#pragma unroll
+          for (int cc = 0; cc < CPL; ++cc) a[cc][j - 1] = fmaf(-gf[cc], qv[e], a[cc][j]);
+        }
+      }
+    }
+#pragma unroll
+    for (int cc = 0; cc < CPL; ++cc) a[cc][n - 1] = (p == gl + G * cc) ? inv : -gf[cc];
+  }
+  __syncwarp();  // the pivot-row buffers lie in Xs
+#pragma unroll
+  for (int cc = 0; cc < CPL; ++cc) {
+    const int i = gl + G * cc;
+    if (i < n) {
+#pragma unroll
+      for (int j = 0; j < n; ++j) Xs[i * ldl + j] = a[cc][j];
+      pinv[i] = step[cc];
+      prow[step[cc]] = i;
+    }
+  }
+  __syncwarp();
+  if (live && ier == 0) {
+#pragma unroll
+    for (int cc = 0; cc < CPL; ++cc) {
+      const int i = gl + G * cc;
+      if (i < n) store_inverse_row<n, float>(Xs + prow[i] * ldl, pinv, Ar, i);
+    }
+  }
+  __syncwarp();
+  return ier;
 }
 
 // The same inverse for 32 < n <= 64 in FP32: lane l holds rows l and l + 32
@@ -837,13 +970,13 @@ __device__ __forceinline__ int reg_gj_inverse2(const double* J, const double* ds
   constexpr int kBuf = 64;
   unsigned used0 = 0, used1 = 0;
   int step0 = -1, step1 = -1;
-#pragma unroll
+#pragma unroll 1
   for (int k = 0; k < n; ++k) {
     LUT* buf = Xs + (k & 1) * kBuf;
     unsigned key = 0u;
-    if (!((used0 >> lane) & 1u)) key = (__float_as_uint(fabsf(a0[k])) & ~63u) | (unsigned)(63 - lane);
+    if (!((used0 >> lane) & 1u)) key = (__float_as_uint(fabsf(a0[0])) & ~63u) | (unsigned)(63 - lane);
     if (row1 && !((used1 >> lane) & 1u)) {
-      const unsigned k1 = (__float_as_uint(fabsf(a1[k])) & ~63u) | (unsigned)(63 - r1);
+      const unsigned k1 = (__float_as_uint(fabsf(a1[0])) & ~63u) | (unsigned)(63 - r1);
       key = key > k1 ? key : k1;
     }
     const unsigned kmax = __reduce_max_sync(kFull, key);
@@ -878,11 +1011,11 @@ __device__ __forceinline__ int reg_gj_inverse2(const double* J, const double* ds
       }
     }
     __syncwarp();
-    const LUT pv = buf[k];
+    const LUT pv = buf[0];
     if (!(fabsf(pv) > 0.f) || isnan(pv)) return k + 1;  // zero or NaN pivot (warp-uniform)
     const LUT inv = 1.f / pv;
-    const LUT g0 = (p == lane) ? 1.f - inv : a0[k] * inv;
-    const LUT g1 = (p == r1) ? 1.f - inv : a1[k] * inv;
+    const LUT g0 = (p == lane) ? 1.f - inv : a0[0] * inv;
+    const LUT g1 = (p == r1) ? 1.f - inv : a1[0] * inv;
 #pragma unroll
     for (int c = 0; c < kChunks; ++c) {
       const float4 q = reinterpret_cast<const float4*>(buf)[c];
@@ -890,14 +1023,14 @@ __device__ __forceinline__ int reg_gj_inverse2(const double* J, const double* ds
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int j = 4 * c + e;
-        if (j < n && j != k) {
-          a0[j] = fmaf(-g0, qv[e], a0[j]);
-          a1[j] = fmaf(-g1, qv[e], a1[j]);
+        if (j < n && j > 0) {
+          a0[j - 1] = fmaf(-g0, qv[e], a0[j]);
+          a1[j - 1] = fmaf(-g1, qv[e], a1[j]);
         }
       }
     }
-    a0[k] = (p == lane) ? inv : -g0;
-    a1[k] = (p == r1) ? inv : -g1;
+    a0[n - 1] = (p == lane) ? inv : -g0;
+    a1[n - 1] = (p == r1) ? inv : -g1;
   }
   __syncwarp();  // the row buffers live in Xs
 #pragma unroll
@@ -921,36 +1054,68 @@ __device__ __forceinline__ int reg_gj_inverse2(const double* J, const double* ds
   return 0;
 }
 
-// Analytic Jacobian of one cell by one warp, lane per reaction: each lane
-// evaluates its reactions (rates and their derivatives) and adds their
-// contributions to a shared-memory Jacobian with atomics -- the mass-action
-// columns of the reaction's own species, the temperature column, and the
-// third-body terms (the default efficiency 1 of every species as a row
-// vector u added to all columns at the end, the non-default ones per
-// species).  Then lane l finishes column l (mass units) and its temperature
-// row entry in shared memory, and the warp writes the matrix into the cell
+// Warps that work on one cell in the Jacobian kernel: one where a warp covers
+// the reactions in two or three strides, a CTA of four for the large
+// mechanism, whose Jacobian and rates (38 KB of shared memory) would leave
+// five warps on an SM and whose few refreshes per round are a matter of
+// latency.
+constexpr int jac_warps(int n) { return n <= 32 ? 1 : 4; }
+// Leading dimension of the shared Jacobian: odd, so that the lanes of a row
+// hit different banks.
+constexpr int jac_ld(int n) { return n | 1; }
+
+// Analytic Jacobian of one cell by a team of W warps.  1. lane per reaction:
+// the derivatives of its rate by the concentration of each of its slots, by T,
+// and by the third-body concentration (D).  2. lane per entry of the Jacobian:
+// the sum of nu D over the reactions that reach it, from the mechanism's
+// table (jt_*: entries in slices of 32 of about equal length, so that a term
+// is one coalesced load and no two lanes write the same entry; the shared
+// atomics this replaces were retry loops: 286,308 Jacobians of 53 species took
+// 28 ms and take 15; with 21 species both take 15 ns a cell, the reactions).  The default third-body efficiency 1 of every
+// species is a row vector u added to all columns, the non-default ones are
+// terms.  3. the temperature row; 4. mass units, and the matrix into the cell
 // record (mat_idx order, consecutive 16-byte stores).
-// s: C, g/RT, h/RT [Npad]; Js: [n][n] column-major; us: [Npad] (shared).
-template <int n, int CPL>
-__device__ __forceinline__ void warp_jac(const DevMech& m, const GrpScratch& s, double* Js, double* us,
-                                         const Vec<CPL>& y, const Vec<CPL>& fy, double* J, int lane) {
+// s: C, g/RT, h/RT, hm [Npad]; Js: [n][ld] column-major, then u [N] and the
+// temperature row [n]; entries outside the table stay zero.
+template <int n, int CPL, int W>
+__device__ __forceinline__ void team_jac(const DevMech& m, const GrpScratch& s, double* hm, double* Js, double* D,
+                                         const Vec<CPL>& y, const Vec<CPL>& fy, double* J, int tid) {
+  constexpr int N = n - 1, ld = jac_ld(n), TS = 32 * W;
+  const int lane = tid & 31;
   const Grp<32> g(lane);
-  constexpr int N = n - 1;
   const int R = m.R;
+  double* u = Js + n * ld;
+  double* tr = u + N;
+  auto sync = [] {
+    if constexpr (W == 1) __syncwarp();
+    else __syncthreads();
+  };
   const double T = grp_get_T<32, CPL>(g, y, N);
   const double lnT = log(T), invT = 1.0 / T;
   double cpk[CPL], hk[CPL], dcpk[CPL];
-  grp_species<32, CPL>(m, s, g, y, T, lnT, cpk, hk, dcpk);
-  double csum = 0.0;
+  grp_species<32, CPL>(m, s, g, y, T, lnT, cpk, hk, dcpk);  // every warp writes the same values
+  double csum = 0.0, rcp = 0.0, drcp = 0.0, cpdot = 0.0, Tdot = 0.0;
 #pragma unroll
-  for (int c = 0; c < CPL; ++c)
-    if (lane + 32 * c < N) csum += y.v[c] * __ldg(m.inv_mw + lane + 32 * c);
+  for (int c = 0; c < CPL; ++c) {
+    const int k = lane + 32 * c;
+    if (k < N) {
+      csum += y.v[c] * __ldg(m.inv_mw + k);
+      rcp += y.v[c] * cpk[c];
+      drcp += y.v[c] * dcpk[c];
+      cpdot += cpk[c] * fy.v[c];
+      hm[k] = hk[c] * __ldg(m.mw + k);
+    } else if (k == N) {
+      Tdot = fy.v[c];
+    }
+  }
   const double Ctot = g.sum(csum);
+  rcp = g.sum(rcp);
+  drcp = g.sum(drcp);
+  cpdot = g.sum(cpdot);
+  Tdot = g.sum(Tdot);
   const double lnPRT = log(kPatm / (kRu * T));
-  for (int e = lane; e < n * n; e += 32) Js[e] = 0.0;
-  for (int k = lane; k < n; k += 32) us[k] = 0.0;
-  __syncwarp();
-  for (int j = lane; j < R; j += 32) {
+  sync();
+  for (int j = tid; j < R; j += TS) {
     const RxnEval e = eval_reaction<true>(m, SpView{s.C, s.gRT, s.hRT}, j, T, lnT, invT, Ctot, lnPRT);
     const int type = __ldg(m.rtype + j);
     const double mult = (type == 1) ? e.M : 1.0;
@@ -958,134 +1123,118 @@ __device__ __forceinline__ void warp_jac(const DevMech& m, const GrpScratch& s, 
     if (type == 1) ceff = e.kf * e.pf - e.kr * e.pr;
     else if (type >= 2) ceff = e.dkf_dM * (e.pf - (e.kf > 0.0 ? e.kr / e.kf : 0.0) * e.pr);
     const double kfm = mult * e.kf, krm = mult * e.kr;
-    const double dqdT = mult * (e.kf * e.dlnkf_dT * e.pf - e.dkr_dT * e.pr);
-    int sp[8], nu[8];
+    double c[8];
+    int nu[8];
 #pragma unroll
     for (int sl = 0; sl < 8; ++sl) {
-      sp[sl] = __ldg(m.sp + sl * R + j);
-      nu[sl] = __ldg(m.nu + sl * R + j);
+      const int k = __ldg(m.sp + sl * R + j), v = __ldg(m.nu + sl * R + j);
+      nu[sl] = k >= 0 ? (v < 0 ? -v : v) : 0;
+      c[sl] = k >= 0 ? s.C[k] : 1.0;
     }
-    // mass-action columns: reactant slots (forward), product slots (reverse)
+    double* d = D + __ldg(m.jt_dptr + j);
+    // derivative by each slot's concentration: reactants forward, products reverse
 #pragma unroll
     for (int a = 0; a < 8; ++a) {
-      if (sp[a] < 0) continue;
-      const int va = (a < 4) ? -nu[a] : nu[a];
-      double p = va * ipow(s.C[sp[a]], va - 1);
-      const int b0 = (a < 4) ? 0 : 4;
+      if (nu[a] == 0) continue;
+      double p = nu[a] * ipow(c[a], nu[a] - 1);
 #pragma unroll
-      for (int s2 = 0; s2 < 4; ++s2) {
-        const int o = b0 + s2;
-        if (o != a && sp[o] >= 0) p *= ipow(s.C[sp[o]], (a < 4) ? -nu[o] : nu[o]);
-      }
-      const double d = (a < 4) ? kfm * p : -krm * p;
-      double* col = Js + sp[a] * n;
-#pragma unroll
-      for (int r = 0; r < 8; ++r)
-        if (sp[r] >= 0) atomicAdd(col + sp[r], (double)nu[r] * d);
+      for (int o = (a < 4 ? 0 : 4); o < (a < 4 ? 4 : 8); ++o)
+        if (o != a) p *= ipow(c[o], nu[o]);
+      *d++ = (a < 4) ? kfm * p : -krm * p;
     }
-    // temperature column and third-body terms
-    double* colT = Js + N * n;
-#pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      if (sp[r] < 0) continue;
-      atomicAdd(colT + sp[r], (double)nu[r] * dqdT);
-      if (type != 0) atomicAdd(us + sp[r], (double)nu[r] * ceff);
-    }
-    if (type != 0) {
-      const int q0 = __ldg(m.eff_ptr + j), q1 = __ldg(m.eff_ptr + j + 1);
-      for (int q = q0; q < q1; ++q) {
-        double* col = Js + __ldg(m.eff_sp + q) * n;
-        const double d = __ldg(m.eff_m1 + q) * ceff;
-#pragma unroll
-        for (int r = 0; r < 8; ++r)
-          if (sp[r] >= 0) atomicAdd(col + sp[r], (double)nu[r] * d);
-      }
-    }
+    *d++ = mult * (e.kf * e.dlnkf_dT * e.pf - e.dkr_dT * e.pr);
+    if (type != 0) *d = ceff;
   }
-  // every lane is done with h/RT (read by the reaction derivatives) before it
-  // is overwritten with the mass-specific enthalpy
-  __syncwarp();
-  // temperature-row ingredients
-  double rcp = 0.0, drcp = 0.0, cpdot = 0.0, Tdot = 0.0;
-#pragma unroll
-  for (int c = 0; c < CPL; ++c) {
-    const int k = lane + 32 * c;
-    if (k < N) {
-      rcp += y.v[c] * cpk[c];
-      drcp += y.v[c] * dcpk[c];
-      cpdot += cpk[c] * fy.v[c];
-      s.hRT[k] = hk[c];  // mass-specific h for the temperature row
-    } else if (k == N) {
-      Tdot = fy.v[c];
+  sync();
+  for (int sl = tid >> 5; sl < m.jt_slices; sl += W) {
+    const int t0 = __ldg(m.jt_off + sl), t1 = __ldg(m.jt_off + sl + 1);
+    double v = 0.0;
+#pragma unroll 4
+    for (int t = t0; t < t1; ++t) {
+      const unsigned term = __ldg(m.jt_term + t * 32 + lane);
+      v += __ldg(m.jt_coef + (term & (kJtCoefs - 1))) * D[term >> kJtCoefBits];
     }
+    const int tgt = __ldg(m.jt_tgt + sl * 32 + lane);
+    if (tgt >= 0) Js[tgt] = v;
   }
-  rcp = g.sum(rcp);
-  drcp = g.sum(drcp);
-  cpdot = g.sum(cpdot);
-  Tdot = g.sum(Tdot);
-  __syncwarp();
-  // lane l finishes column l: mass units, default third-body row, T row
-#pragma unroll
-  for (int c = 0; c < CPL; ++c) {
-    const int l = lane + 32 * c;
-    if (l > N) continue;
-    const double inv_wl = (l < N) ? __ldg(m.inv_mw + l) : 1.0;
-    double* col = Js + l * n;
+  sync();
+  for (int l = tid; l < n; l += TS) {
+    const double* col = Js + l * ld;
     double sum = 0.0;
-    for (int k = 0; k < N; ++k) {
-      const double v = (col[k] + ((l < N) ? us[k] : 0.0)) * __ldg(m.mw + k) * inv_wl;
-      col[k] = v;
-      sum += s.hRT[k] * v;
+    double extra = 0.0;
+    if (l < N) {
+      for (int k = 0; k < N; ++k) sum += hm[k] * (col[k] + u[k]);
+      sum *= __ldg(m.inv_mw + l);
+    } else {
+      for (int k = 0; k < N; ++k) sum += hm[k] * col[k];
+      extra = cpdot + Tdot * drcp;
     }
-    col[N] = -(sum + ((l < N) ? Tdot * cpk[c] : cpdot + Tdot * drcp)) / rcp;
+    // Tdot * cp of the column's species: the lane that holds species l has it
+    tr[l] = -(sum + extra) / rcp;
   }
-  __syncwarp();
+  sync();
+  if (tid < 32) {
+#pragma unroll
+    for (int c = 0; c < CPL; ++c) {
+      const int l = lane + 32 * c;
+      if (l < N) tr[l] -= Tdot * cpk[c] / rcp;
+    }
+  }
+  sync();
   constexpr int G = ctrl_group(n), JB = n / kVJ;
   static_assert(n % kVJ == 0, "no column padding in J");
 #pragma unroll
   for (int cc = 0; cc < (n + G - 1) / G; ++cc) {
     const int rows = (n - cc * G < G) ? n - cc * G : G;
     double2* dst = reinterpret_cast<double2*>(J + mat_vec<n, G, kVJ>(cc, 0, 0));
-    for (int t = lane; t < rows * JB; t += 32) {
+    for (int t = tid; t < rows * JB; t += TS) {
       const int jb = t / rows, i = cc * G + t % rows;
-      dst[t] = make_double2(Js[(jb * kVJ) * n + i], Js[(jb * kVJ + 1) * n + i]);
+      double v[kVJ];
+#pragma unroll
+      for (int e = 0; e < kVJ; ++e) {
+        const int j = jb * kVJ + e;
+        if (i == N) v[e] = tr[j];
+        else if (j < N) v[e] = (Js[j * ld + i] + u[i]) * __ldg(m.mw + i) * __ldg(m.inv_mw + j);
+        else v[e] = Js[j * ld + i] * __ldg(m.mw + i);
+      }
+      dst[t] = make_double2(v[0], v[1]);
     }
   }
-  __syncwarp();
+  sync();
 }
 
 // Jacobian refresh for the cells of the setup list whose matrix CVODE's
-// jbad rule marks stale: the analytic FP64 Jacobian into the cell record, one
-// warp per cell.
-// Minimum resident CTAs per SM requested for the Jacobian kernel (bounds
-// its registers per thread; n > 32 keeps 2: its shared memory allows no
-// more).
+// jbad rule marks stale: the analytic FP64 Jacobian into the cell record.
+// Minimum resident CTAs (of 128 threads) per SM requested for the Jacobian
+// kernel (bounds its registers per thread).
 #ifndef B200_JAC_MIN_CTAS
-#define B200_JAC_MIN_CTAS 8
+#define B200_JAC_MIN_CTAS 5
 #endif
 
-template <int NS, int CPL>
-__global__ void __launch_bounds__(128, CPL == 1 ? B200_JAC_MIN_CTAS : 2) rk_jac(RoundsParams R) {
-  constexpr int n = NS + 1;
+template <int NS>
+__global__ void __launch_bounds__(128, B200_JAC_MIN_CTAS) rk_jac(RoundsParams R) {
+  constexpr int n = NS + 1, CPL = (n + 31) / 32, W = jac_warps(n), ld = jac_ld(n);
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ DevMech s_mech;
   if (threadIdx.x == 0) s_mech = R.P.mech;
   __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int cnt = *R.cnt_in;
+  if ((long long)blockIdx.x * (4 / W) >= cnt) return;
   const RoundsSetupLayout& SL = R.SL;
-  double* d = reinterpret_cast<double*>(dsm + (size_t)w * SL.jac_smem_per_warp);
+  const int team = threadIdx.x / (32 * W), tid = threadIdx.x % (32 * W), lane = tid & 31;
+  const int gt = blockIdx.x * (4 / W) + team, nteams = gridDim.x * (4 / W);
+  double* d = reinterpret_cast<double*>(dsm + (size_t)team * SL.jac_smem_per_team);
   GrpScratch ms;
   ms.C = d;
   ms.gRT = d + SL.Npad;
   ms.hRT = d + 2 * SL.Npad;
-  double* us = d + 3 * SL.Npad;
-  double* Js = d + 4 * SL.Npad;
   ms.q = ms.r1 = ms.r2 = ms.r3 = ms.r4 = nullptr;
-  const long long gw = (long long)blockIdx.x * (blockDim.x >> 5) + w;
-  const int cnt = *R.cnt_in;
+  double* hm = d + 3 * SL.Npad;
+  double* Js = d + 4 * SL.Npad;
+  double* D = SL.jac_d_global ? reinterpret_cast<double*>(R.wscratch) + (size_t)gt * SL.jac_nd : Js + n * ld + NS + n;
+  for (int e = tid; e < n * ld + NS; e += 32 * W) Js[e] = 0.0;
   const RLayout RL = R.S.L;
-  const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long idx = gw; idx < cnt; idx += nwarps) {
+  for (int idx = gt; idx < cnt; idx += nteams) {
     const int slot = R.list_in[idx];
     unsigned char* rec = rec_of(R.S, slot);
     // the cells were chosen by CVODE's jbad rule at their prediction, which
@@ -1098,83 +1247,118 @@ __global__ void __launch_bounds__(128, CPL == 1 ? B200_JAC_MIN_CTAS : 2) rk_jac(
       y.v[cc] = (i < n) ? v.yev(i) : 0.0;
       fy.v[cc] = (i < n) ? v.fv(i) : 0.0;
     }
-    warp_jac<n, CPL>(s_mech, ms, Js, us, y, fy, reinterpret_cast<double*>(rec + RL.off_j), lane);
-    __syncwarp();
+    team_jac<n, CPL, W>(s_mech, ms, hm, Js, D, y, fy, reinterpret_cast<double*>(rec + RL.off_j), tid);
   }
 }
 
-// Minimum resident CTAs per SM requested for the inversion kernel (bounds
-// its registers per thread).
+// Minimum resident CTAs (of 128 threads) per SM requested for the inversion
+// kernel (bounds its registers per thread): 4 for the lane groups (three rows
+// of 22 FP32 entries per lane), 6 for one row per lane, 2 for two rows.
 #ifndef B200_GJ_MIN_CTAS
-#define B200_GJ_MIN_CTAS 6
+#define B200_GJ_MIN_CTAS 4
 #endif
+template <int n, typename LUT>
+constexpr bool gj_by_groups() { return n <= 32 && sizeof(LUT) == 4; }
+template <int n, typename LUT>
+constexpr int gj_min_ctas() { return gj_by_groups<n, LUT>() ? B200_GJ_MIN_CTAS : n <= 32 ? 6 : 2; }
 
-// Newton-matrix inverse of the cells of the setup list, one warp per cell:
-// Gauss-Jordan inverse of D (I - gamma J) D^-1 with D = diag(ewt) (FP32) or
-// of I - gamma J (FP64), written into the cell record.
-template <int NS, typename LUT, int CPL>
-__global__ void __launch_bounds__(128, CPL == 1 ? B200_GJ_MIN_CTAS : 2) rk_gj(RoundsParams R) {
+// Bookkeeping of a setup in the cell's scalars.
+__device__ __forceinline__ void gj_done(RCell* cp, double gamma, int ier) {
+  cp->cnt.nlu++;
+  cp->gamma_lu = gamma;
+  cp->gamrat = 1.0;
+  cp->gammap = gamma;
+  cp->crate = 1.0;
+  cp->nstlp = cp->cnt.nst;
+  cp->setup_ier = ier;
+}
+
+// Newton-matrix inverse of the cells of the setup list: Gauss-Jordan inverse
+// of D (I - gamma J) D^-1 with D = diag(ewt) (FP32) or of I - gamma J (FP64),
+// written into the cell record.  One warp per cell, or (n <= 32 in FP32) the
+// lane groups of the step kernel, whose rows are the ones it reads and writes.
+template <int NS, typename LUT>
+__global__ void __launch_bounds__(128, gj_min_ctas<NS + 1, LUT>()) rk_gj(RoundsParams R) {
   constexpr int n = NS + 1;
+  constexpr int WCPL = (n + 31) / 32;  // rows per lane of the warp forms
   extern __shared__ __align__(16) unsigned char dsm[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const RoundsSetupLayout& SL = R.SL;
-  unsigned char* sb = dsm + (size_t)w * SL.gj_smem_per_warp;
-  double* Dsc = reinterpret_cast<double*>(sb);
-  LUT* A = reinterpret_cast<LUT*>(Dsc + SL.Npad);
-  LUT* fcol = A + (size_t)n * SL.ldl;
-  int* ipiv = reinterpret_cast<int*>(fcol + SL.Npad);
-  int* ipiv2 = ipiv + SL.Npad;
   const int cnt = *R.cnt_in;
   const RLayout RL = R.S.L;
-  const long long gw = (long long)blockIdx.x * (blockDim.x >> 5) + w;
-  const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long idx = gw; idx < cnt; idx += nwarps) {
-    const int slot = R.list_in[idx];
-    unsigned char* rec = rec_of(R.S, slot);
-    RCell* cp = reinterpret_cast<RCell*>(rec);
-    const RVec<n> v{reinterpret_cast<double*>(rec + RL.off_vec)};
-    const double* J = reinterpret_cast<const double*>(rec + RL.off_j);
-    LUT* Ar = reinterpret_cast<LUT*>(rec + RL.off_a);
-    const double gamma = cp->gamma;
+  const int gw = blockIdx.x * (blockDim.x >> 5) + w;
+  const int nwarps = gridDim.x * (blockDim.x >> 5);
+  if constexpr (gj_by_groups<n, LUT>()) {
+    constexpr int G = ctrl_group(n), GPW = 32 / G, CPL = (n + G - 1) / G;
+    const int gl = lane % G, gi = lane / G;
+    double* rds = reinterpret_cast<double*>(dsm + (size_t)(threadIdx.x / G) * gj_cell_bytes(n));
+    float* Xs = reinterpret_cast<float*>(rds + n);
+    int* prow = reinterpret_cast<int*>(Xs + (n * (n | 1) + 3) / 4 * 4);
+    int* pinv = prow + n;
+    for (int base = gw * GPW; base < cnt; base += nwarps * GPW) {
+      const bool live = base + gi < cnt;
+      unsigned char* rec = rec_of(R.S, live ? R.list_in[base + gi] : 0);
+      RCell* cp = reinterpret_cast<RCell*>(rec);
+      const RVec<n> v{reinterpret_cast<double*>(rec + RL.off_vec)};
+      const double gamma = live ? cp->gamma : 0.0;
+      double di[CPL];
 #pragma unroll
-    for (int cc = 0; cc < CPL; ++cc) {
-      const int i = lane + 32 * cc;
-      if (i < n) {
-        const double ds = (sizeof(LUT) == 4) ? v.ewt(i) : 1.0;
-        Dsc[i] = ds;
-        v.dsc(i) = ds;
+      for (int cc = 0; cc < CPL; ++cc) {
+        const int i = gl + G * cc;
+        di[cc] = (live && i < n) ? v.ewt(i) : 1.0;
+        if (live && i < n) v.dsc(i) = di[cc];
       }
+      const int ier = grp_reg_gj_inverse<n, G>(reinterpret_cast<const double*>(rec + RL.off_j), live, di, rds, gamma,
+                                               Xs, prow, pinv, reinterpret_cast<float*>(rec + RL.off_a), gl);
+      if (live && gl == 0) gj_done(cp, gamma, ier);
     }
-    __syncwarp();
-    int ier;
-    if constexpr (CPL == 1) {
-      ier = reg_gj_inverse<(CPL == 1 ? n : 2), LUT>(J, Dsc, gamma, A, SL.ldl, ipiv, ipiv2, Ar, lane);
-    } else if constexpr (CPL == 2 && sizeof(LUT) == 4) {
-      ier = reg_gj_inverse2<(CPL == 2 ? n : 34), LUT>(J, Dsc, gamma, A, SL.ldl, ipiv, ipiv2, Ar, lane);
-    } else {
-      static_assert(sizeof(LUT) == 8, "the unscaled matrix");
-      constexpr int G = ctrl_group(n);
-      for (int e = lane; e < n * n; e += 32) {
-        const int i = e / n, j = e % n;
-        A[i * SL.ldl + j] = ((i == j) ? 1.0 : 0.0) - gamma * J[mat_idx<n, G, kVJ>(i, j)];
+  } else {
+    unsigned char* sb = dsm + (size_t)w * SL.gj_smem_per_warp;
+    double* Dsc = reinterpret_cast<double*>(sb);
+    LUT* A = reinterpret_cast<LUT*>(Dsc + SL.Npad);
+    LUT* fcol = A + (size_t)n * SL.ldl;
+    int* ipiv = reinterpret_cast<int*>(fcol + SL.Npad);
+    int* ipiv2 = ipiv + SL.Npad;
+    for (int idx = gw; idx < cnt; idx += nwarps) {
+      const int slot = R.list_in[idx];
+      unsigned char* rec = rec_of(R.S, slot);
+      RCell* cp = reinterpret_cast<RCell*>(rec);
+      const RVec<n> v{reinterpret_cast<double*>(rec + RL.off_vec)};
+      const double* J = reinterpret_cast<const double*>(rec + RL.off_j);
+      LUT* Ar = reinterpret_cast<LUT*>(rec + RL.off_a);
+      const double gamma = cp->gamma;
+#pragma unroll
+      for (int cc = 0; cc < WCPL; ++cc) {
+        const int i = lane + 32 * cc;
+        if (i < n) {
+          const double ds = (sizeof(LUT) == 4) ? v.ewt(i) : 1.0;
+          Dsc[i] = ds;
+          v.dsc(i) = ds;
+        }
       }
       __syncwarp();
-      ier = grp_gj_eliminate<32, LUT>(A, SL.ldl, ipiv, fcol, n, lane);
+      int ier;
+      if constexpr (WCPL == 1) {
+        ier = reg_gj_inverse<n, LUT>(J, Dsc, gamma, A, SL.ldl, ipiv, ipiv2, Ar, lane);
+      } else if constexpr (WCPL == 2 && sizeof(LUT) == 4) {
+        ier = reg_gj_inverse2<n, LUT>(J, Dsc, gamma, A, SL.ldl, ipiv, ipiv2, Ar, lane);
+      } else {
+        static_assert(sizeof(LUT) == 8, "the unscaled matrix");
+        constexpr int G = ctrl_group(n);
+        for (int e = lane; e < n * n; e += 32) {
+          const int i = e / n, j = e % n;
+          A[i * SL.ldl + j] = ((i == j) ? 1.0 : 0.0) - gamma * J[mat_idx<n, G, kVJ>(i, j)];
+        }
+        __syncwarp();
+        ier = grp_gj_eliminate<32, LUT>(A, SL.ldl, ipiv, fcol, n, lane);
+        __syncwarp();
+        if (ier == 0)
+          for (int i = lane; i < n; i += 32) store_inverse_row<n, LUT>(A + i * SL.ldl, nullptr, Ar, i);
+      }
       __syncwarp();
-      if (ier == 0)
-        for (int i = lane; i < n; i += 32) store_inverse_row<n, LUT>(A + i * SL.ldl, nullptr, Ar, i);
+      if (lane == 0) gj_done(cp, gamma, ier);
+      __syncwarp();
     }
-    __syncwarp();
-    if (lane == 0) {
-      cp->cnt.nlu++;
-      cp->gamma_lu = gamma;
-      cp->gamrat = 1.0;
-      cp->gammap = gamma;
-      cp->crate = 1.0;
-      cp->nstlp = cp->cnt.nst;
-      cp->setup_ier = ier;
-    }
-    __syncwarp();
   }
 }
 
@@ -1187,22 +1371,20 @@ int rhs_smem(int block) { return 3 * NS * block * (int)sizeof(double); }
 template <int NS, typename LUT>
 cudaError_t rounds_setup_attrs(const RoundsSetupLayout& SL) {
   constexpr int n = NS + 1;
-  constexpr int CPL = (n + 31) / 32;
   cudaError_t e = cudaFuncSetAttribute(rk_rhs<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        rhs_smem<NS>(kRoundsRhsBlock));
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(rk_jac<NS, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * SL.jac_smem_per_warp);
+  e = cudaFuncSetAttribute(rk_jac<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SL.jac_smem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(rk_step<NS, LUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, step_smem<n>());
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(rk_gj<NS, LUT, CPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(rk_gj<NS, LUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               4 * SL.gj_smem_per_warp);
 }
 
 template <int NS, typename LUT>
 cudaError_t rounds_grids(const RoundsSetupLayout& SL, int sm_count, RoundsGrids* G) {
   constexpr int n = NS + 1;
-  constexpr int CPL = (n + 31) / 32;
   cudaError_t e = rounds_setup_attrs<NS, LUT>(SL);
   if (e != cudaSuccess) return e;
   int b = 0;
@@ -1217,11 +1399,11 @@ cudaError_t rounds_grids(const RoundsSetupLayout& SL, int sm_count, RoundsGrids*
   G->step = std::max(1, b) * sm_count;
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rk_ctrl<NS>, 128, 0)) != cudaSuccess) return e;
   G->ctrl = std::max(1, b) * sm_count;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rk_jac<NS, CPL>, 128, 4 * SL.jac_smem_per_warp)) !=
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rk_jac<NS>, 128, SL.jac_smem)) !=
       cudaSuccess)
     return e;
   G->jac = std::max(1, b) * sm_count;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rk_gj<NS, LUT, CPL>, 128, 4 * SL.gj_smem_per_warp)) !=
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rk_gj<NS, LUT>, 128, 4 * SL.gj_smem_per_warp)) !=
       cudaSuccess)
     return e;
   G->gj = std::max(1, b) * sm_count;
@@ -1232,7 +1414,6 @@ cudaError_t rounds_grids(const RoundsSetupLayout& SL, int sm_count, RoundsGrids*
 template <int NS, typename LUT>
 cudaError_t rounds_launch_t(int what, const RoundsParams& R, const RoundsGrids& G, int setup_pass, cudaStream_t st) {
   constexpr int n = NS + 1;
-  constexpr int CPL = (n + 31) / 32;
   switch (what) {
     case kRoundsStart:
       rk_start<NS><<<G.start, 128, 0, st>>>(R);
@@ -1248,10 +1429,10 @@ cudaError_t rounds_launch_t(int what, const RoundsParams& R, const RoundsGrids& 
       rk_ctrl<NS><<<G.ctrl, 128, 0, st>>>(R);
       break;
     case kRoundsJac:
-      rk_jac<NS, CPL><<<G.jac, 128, 4 * R.SL.jac_smem_per_warp, st>>>(R);
+      rk_jac<NS><<<G.jac, 128, R.SL.jac_smem, st>>>(R);
       break;
     case kRoundsGj:
-      rk_gj<NS, LUT, CPL><<<G.gj, 128, 4 * R.SL.gj_smem_per_warp, st>>>(R);
+      rk_gj<NS, LUT><<<G.gj, 128, 4 * R.SL.gj_smem_per_warp, st>>>(R);
       break;
     default:
       return cudaErrorInvalidValue;
@@ -1263,16 +1444,23 @@ cudaError_t rounds_launch_t(int what, const RoundsParams& R, const RoundsGrids& 
 
 bool rounds_supported(int N) { return N == 9 || N == 21 || N == 53; }
 
-RoundsSetupLayout rounds_setup_layout(int N, int R, int lut_bytes) {
+RoundsSetupLayout rounds_setup_layout(int N, int lut_bytes, int jac_nd) {
   RoundsSetupLayout L;
   const int n = N + 1;
   L.Npad = ((n + 31) / 32) * 32;
-  L.Rpad = std::max(32, ((R + 31) / 32) * 32);
   L.ldl = n | 1;
-  L.jac_smem_per_warp = (int)(8LL * (4 * L.Npad + (long long)n * n));
-  const long long b = 8LL * L.Npad + (long long)lut_bytes * ((long long)n * L.ldl + L.Npad) + 4LL * 2 * L.Npad;
+  // scratch of a Jacobian team; the reactions' derivatives move to device
+  // memory where they would leave fewer than two CTAs on an SM
+  const int teams = 4 / jac_warps(n);
+  const long long fixed = 8LL * (4 * L.Npad + n * jac_ld(n) + N + n), dbytes = 8LL * jac_nd;
+  L.jac_nd = jac_nd;
+  L.jac_d_global = teams * (fixed + dbytes) > 100 * 1024;
+  L.jac_smem_per_team = (int)((fixed + (L.jac_d_global ? 0 : dbytes) + 15) & ~15LL);
+  L.jac_smem = teams * L.jac_smem_per_team;
+  L.gbytes_per_cta = L.jac_d_global ? teams * dbytes : 0;
+  long long b = 8LL * L.Npad + (long long)lut_bytes * ((long long)n * L.ldl + L.Npad) + 4LL * 2 * L.Npad;
+  if (n <= 32 && lut_bytes == 4) b = 32LL / ctrl_group(n) * gj_cell_bytes(n);
   L.gj_smem_per_warp = (int)((b + 15) & ~15LL);
-  L.gbytes_per_warp = (8LL * 4LL * L.Rpad + 255) & ~255LL;
   return L;
 }
 
