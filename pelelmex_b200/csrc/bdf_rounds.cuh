@@ -463,6 +463,14 @@ constexpr int kStatusRefineStall = -100;
 // refine_ratio of a cell whose current matrix has not been measured yet
 constexpr float kRefineUnknown = 3.0e38f;
 
+// Column vectors of a matrix-vector product that are unrolled together: all of
+// a small matrix (4 at a time costs 6 % of the step kernel at n = 22), 4 of a
+// large one, whose loads spill otherwise (7 % at n = 54).
+template <int n>
+constexpr int mat_unroll(int jb) {
+  return n <= 32 ? jb : 4;
+}
+
 // x := D^-1 A D x for the group's cell: A is the scaled inverse (mat_idx
 // order), D = dsc; LUT = double: A is the plain inverse.  Lane gl holds
 // components gl + G cc of x and dsc; the multipliers go through xs (n entries
@@ -485,7 +493,7 @@ __device__ __forceinline__ void g_apply_inverse(const LUT* __restrict__ A, const
   LUT acc[CPL];
 #pragma unroll
   for (int cc = 0; cc < CPL; ++cc) acc[cc] = (LUT)0;
-#pragma unroll
+#pragma unroll(mat_unroll<n>(JB))
   for (int jb = 0; jb < JB; ++jb) {
     const Vec16 bv = *reinterpret_cast<const Vec16*>(xs + jb * V);
     const LUT* b = reinterpret_cast<const LUT*>(&bv);
@@ -541,7 +549,7 @@ __device__ __forceinline__ void g_newton(const RVec<n>& v, const double* __restr
       double r[CPL];
 #pragma unroll
       for (int cc = 0; cc < CPL; ++cc) r[cc] = 0.0;
-#pragma unroll
+#pragma unroll(mat_unroll<n>(JB))
       for (int jb = 0; jb < JB; ++jb) {
         const double2 xv = *reinterpret_cast<const double2*>(xs + jb * kVJ);
 #pragma unroll

@@ -453,10 +453,15 @@ __global__ void __launch_bounds__(kRoundsRhsBlock, B200_RHS_MIN_CTAS) rk_rhs(Rou
 }
 
 // Minimum resident CTAs (of 128 threads) per SM requested for the step
-// kernel: bounds its registers per thread.
-#ifndef B200_STEP_MIN_CTAS
-#define B200_STEP_MIN_CTAS 4
-#endif
+// kernel: bounds its registers per thread.  The kernel is bound by the cells'
+// records (8 KB at 22 components) from HBM, and more cells in flight do not
+// help it: the matrices prefetched for them drop out of L2 before they are read
+// (9500 cells hold 78 MB), and loads that the registers of 2 CTAs keep in flight
+// hide the latency as well.  128^3 CH4, per react: 168 ms at 2 CTAs, 186 at 3,
+// 201 at 4, 250 at 5.  A small record (2.3 KB at 10 components) leaves the
+// arithmetic, for which more warps are better (32^3 H2: 2.1 ms at 4, 2.2 at 3,
+// 2.6 at 2).
+constexpr int step_min_ctas(int n) { return n <= 16 ? 4 : 2; }
 
 // Bulk prefetch of [p, p + bytes) into L2 (p and bytes multiples of 16; a
 // hint: no completion to wait for).
@@ -498,6 +503,7 @@ __device__ __forceinline__ void step_cell(const RoundsParams& R, bool live, int 
   int which = 0, rhs_val = slot;
   if (live) {
     unsigned char* rec = rec_of(R.S, slot);
+    // the matrices stream into L2 while the scalars and vectors are copied
     if (gl == 0) l2_prefetch(rec + R.S.L.off_j, (uint32_t)(R.S.L.stride - R.S.L.off_j));
     for (int b = gl * 16; b < step_read_bytes<n>(); b += G * 16) cp_async16(sm + b, rec + b);
     cp_async_wait();
@@ -595,7 +601,7 @@ __device__ __forceinline__ void step_cell(const RoundsParams& R, bool live, int 
 // setup_pass: the cells whose Newton matrix this round's setup kernels
 // rebuilt; otherwise the others (those entries, flagged, are passed over).
 template <int NS, typename LUT>
-__global__ void __launch_bounds__(128, B200_STEP_MIN_CTAS) rk_step(RoundsParams R, int setup_pass) {
+__global__ void __launch_bounds__(128, step_min_ctas(NS + 1)) rk_step(RoundsParams R, int setup_pass) {
   constexpr int n = NS + 1;
   constexpr int G = ctrl_group(n);
   constexpr int GPW = 32 / G;  // cells per warp
