@@ -20,6 +20,7 @@
 //
 // Every wait on the mbarrier is bounded; on timeout the kernel raises a flag
 // in err (read by the host) and stops issuing work.
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -422,6 +423,111 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_bf16_tc(GemmArgs g) {
   if (warp == 0) tmem_dealloc(tmem, ncols);
 }
 
+// ------------------------------------------------------------ split-K GEMM
+// Few output tiles over a long K (the weight gradients: 256 x 256 over the
+// batch): one tile per CTA leaves all but two SMs idle and a serial chain of
+// chunks, 330 us for K = 16384.  Here a cluster of kSplit CTAs shares one
+// 128 x NT tile, each with its own range of K and a ring of staged chunks,
+// and adds the partial sums through distributed shared memory in rank order
+// (the same bits every time); NT is at most 64, so the 256 x 256 case runs on
+// 64 SMs.  FP32 output without activation.
+constexpr int kSplit = 8;
+constexpr int kSplitStages = 4;
+constexpr int kSplitKC = 64;
+
+// N tile: the largest multiple of 16 up to 64 that divides N.
+inline int split_nt(int N) {
+  for (int nt = 64; nt > 16; nt -= 16)
+    if (N % nt == 0) return nt;
+  return 16;
+}
+inline int split_smem(int NT) { return kSplitStages * (kTileM + NT) * kSplitKC * 2; }
+
+__global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kThreads) gemm_bf16_splitk(GemmArgs g, int NT) {
+  extern __shared__ __align__(1024) unsigned char smem[];
+  __shared__ __align__(8) uint64_t bar[kSplitStages];
+  __shared__ uint32_t tmem_base_s;
+  namespace cg = cooperative_groups;
+  const cg::cluster_group cluster = cg::this_cluster();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = (int)cluster.block_rank(), tile = blockIdx.x / kSplit;
+  const int ntiles = g.N / NT, mt = tile / ntiles, n0 = (tile % ntiles) * NT;
+  const int chunks = g.K / kSplitKC, per = (chunks + kSplit - 1) / kSplit;
+  const int c0 = rank * per, cnt = max(0, min(chunks, c0 + per) - c0);
+  const int stage_bytes = (kTileM + NT) * kSplitKC * 2;
+  const uint32_t ncols = NT <= 32 ? 32 : 64;
+  if (warp == 0) tmem_alloc(&tmem_base_s, ncols);
+  if (tid == 0) {
+    for (int s = 0; s < kSplitStages; ++s) mbar_init(&bar[s], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_base_s;
+  const uint32_t idesc = umma_idesc_bf16(kTileM, NT);
+  auto stage = [&](int i) {  // chunk i of this CTA into its ring slot; always one copy group
+    if (i < cnt) {
+      unsigned char* As = smem + (i % kSplitStages) * stage_bytes;
+      const int k0 = (c0 + i) * kSplitKC;
+      stage_tile(As, g.A + (long long)mt * kTileM * g.lda, g.lda, kTileM, kTileM, k0, kSplitKC);
+      stage_tile(As + kTileM * kSplitKC * 2, g.B + (long long)n0 * g.ldb, g.ldb, NT, NT, k0, kSplitKC);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int i = 0; i < kSplitStages - 1; ++i) stage(i);
+  bool fail = false;
+  for (int i = 0; i < cnt; ++i) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kSplitStages - 2) : "memory");
+    fence_async_smem();
+    if (__syncthreads_or(fail)) break;
+    if (tid == 0) {
+      tc_fence_after();
+      const uint32_t a0 = smem_u32(smem + (i % kSplitStages) * stage_bytes), b0 = a0 + kTileM * kSplitKC * 2;
+      for (int ks = 0; ks < kSplitKC / 16; ++ks)
+        umma_bf16(tmem, umma_desc(a0 + ks * 256u, 128u, kSplitKC / 8 * 128u),
+                  umma_desc(b0 + ks * 256u, 128u, kSplitKC / 8 * 128u), idesc, (i > 0 || ks > 0) ? 1u : 0u);
+      umma_commit(&bar[i % kSplitStages]);
+    }
+    // the slot of chunk i + 3 is free once the MMAs of chunk i - 1 are done
+    if (i > 0) fail = !mbar_wait_bounded(&bar[(i - 1) % kSplitStages], ((i - 1) / kSplitStages) & 1);
+    stage(i + kSplitStages - 1);
+  }
+  if (cnt > 0 && !fail) fail = !mbar_wait_bounded(&bar[(cnt - 1) % kSplitStages], ((cnt - 1) / kSplitStages) & 1);
+  stage_wait();
+  if (__syncthreads_or(fail) && tid == 0 && g.err) atomicExch(g.err, 1);
+  tc_fence_after();
+  // partial tile to shared memory (the stages are free), rows padded
+  const int ld = NT + 4;
+  float* part = reinterpret_cast<float*>(smem);
+  for (int q0 = 0; q0 < NT; q0 += 32) {
+    float v[32];
+    tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)q0, v);
+    float* row = part + (warp * 32 + lane) * ld + q0;
+#pragma unroll
+    for (int i = 0; i < 32; i += 4)
+      if (q0 + i < NT)
+        *reinterpret_cast<float4*>(row + i) = cnt > 0 ? make_float4(v[i], v[i + 1], v[i + 2], v[i + 3])
+                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  tc_fence_before();
+  cluster.sync();
+  tc_fence_after();
+  // this CTA adds rows 16 rank .. 16 rank + 15 of all partial tiles
+  constexpr int kRows = kTileM / kSplit;
+  for (int e = tid; e < kRows * NT; e += kThreads) {
+    const int r = rank * kRows + e / NT, c = e % NT;
+    float s = 0.f;
+#pragma unroll
+    for (int p = 0; p < kSplit; ++p) s += cluster.map_shared_rank(part, p)[r * ld + c];
+    const int col = n0 + c;
+    if (col < g.n_valid)
+      static_cast<float*>(g.C)[((long long)mt * kTileM + r) * g.ldc + col] = s + (g.bias ? g.bias[col] : 0.f);
+  }
+  cluster.sync();  // no CTA leaves while another reads its shared memory
+  if (warp == 0) tmem_dealloc(tmem, ncols);
+}
+
 // ------------------------------------------------ warp-specialised GEMM
 // For B resident in shared memory (K <= 256, N <= 256): the weights of one
 // layer times 128-row tiles of activations, pipelined across tiles.
@@ -786,6 +892,17 @@ extern "C" int b200chem_mlp_gemm_bf16(const void* A, long long lda, const void* 
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }
   if (arep != 1) return -1;  // two-term A operands need the warp-specialised kernel
+  // Split K where the tiles would leave most SMs idle: 16 chunks of K and more
+  // (each of the cluster's CTAs gets at least two) with fewer 128 x 256 tiles
+  // than half the SMs.
+  if (epi == kEpiF32 && !resident && K % kSplitKC == 0 && K >= 2 * kSplit * kSplitKC &&
+      2 * (M / kTileM) * ((N + 255) / 256) < sms) {
+    const int nt = split_nt(N), ssm = split_smem(nt);
+    if (cudaFuncSetAttribute(gemm_bf16_splitk, cudaFuncAttributeMaxDynamicSharedMemorySize, ssm) != cudaSuccess)
+      return -2;
+    gemm_bf16_splitk<<<(M / kTileM) * (N / nt) * kSplit, kThreads, ssm, st>>>(g, nt);
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  }
   const int NT = N <= 256 ? N : 256;
   const int KC = resident ? K : 64;
   const int smem = kTileM * KC * 2 + NT * KC * 2;
