@@ -70,7 +70,7 @@ def build(force: bool = False, verbose: bool = False, ptxas_v: bool = False, job
 
     def compile_one(src: Path):
         obj = objdir / (src.stem + ".o")
-        cmd = [nvcc(), *ARCH, *NVCC_FLAGS, "-c", "-o", str(obj), str(src), "-I", str(INCLUDE), "-I",
+        cmd = [nvcc(), *ARCH, *NVCC_FLAGS, "-c", "-o", str(obj), str(src), "-I", str(INCLUDE), "-I", str(CSRC), "-I",
                str(gen.parent)]
         if ptxas_v:
             cmd += ["-Xptxas", "-v"]

@@ -190,12 +190,15 @@ __global__ void thermo_hr_kernel(DevMech m, const double* __restrict__ T, const 
   for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < ncells;
        c += (long long)gridDim.x * blockDim.x) {
     const double t = T[c];
-    const double lnT = log(t);
     double hr = 0.0;
+#pragma unroll 3
     for (int k = 0; k < m.N; ++k) {
-      double cpR, hRT, sR, dcpR;
-      nasa7(m, k, t, lnT, cpR, hRT, sR, dcpR);
-      const double hk = hRT * kRu * t * __ldg(m.inv_mw + k) * 0.0001;  // erg/g -> J/kg
+      // h_k = Ru T / W_k (h/RT), the NASA-7 polynomial without its divisions
+      const double* a = m.nasa + (t < __ldg(m.nasa + k) ? 1 : 8) * m.N + k;
+      const double p = __ldg(a) + t * (__ldg(a + m.N) * 0.5 +
+                                       t * (__ldg(a + 2 * m.N) * (1.0 / 3.0) +
+                                            t * (__ldg(a + 3 * m.N) * 0.25 + t * (__ldg(a + 4 * m.N) * 0.2))));
+      const double hk = (p * t + __ldg(a + 5 * m.N)) * (kRu * 0.0001) * __ldg(m.inv_mw + k);  // erg/g -> J/kg
       if (Hi) Hi[(long long)k * ncells + c] = hk;
       if (HR) hr = fma(-hk, IR[(long long)k * ncells + c], hr);
     }
@@ -217,6 +220,11 @@ struct StagedBuf {
   bool pending = false;
   cudaEvent_t ev = nullptr;
 };
+
+// Launch shapes of a round by how many cells are live: many (right-hand sides
+// by thread), few (by warp), and so few that the grids shrink to them.
+constexpr int kRoundClasses = 3;
+constexpr int kTinyCells = 1024;
 
 struct b200chem_reactor {
   int device = 0;
@@ -252,9 +260,11 @@ struct b200chem_reactor {
   int gen_mech = 0;  // 1: a generated right-hand side matches the mechanism
   unsigned long long digest = 0;  // FNV-1a digest of the mechanism description
   b200chem_tuning tune{};           // launch shape of the round-based integrator
-  cudaStream_t cap_stream = nullptr;  // private stream the round graph is captured on
-  cudaGraphExec_t rgraph = nullptr;   // executable graph of rounds_per_check rounds
-  int rgraph_rounds = 0;              // rounds in rgraph
+  cudaStream_t cap_stream = nullptr;  // private streams the round graph is captured on:
+  cudaStream_t cap_side = nullptr;    // the second one takes the setup kernels
+  cudaEvent_t cap_ev[2] = {};         // fork and join of the two
+  cudaGraphExec_t rgraph[kRoundClasses] = {};  // executable graphs of rounds_per_check rounds, by live-cell class
+  int rgraph_rounds[kRoundClasses] = {};       // rounds in each
   StagedBuf cboxes;                   // advanceChemistry box descriptors
   StagedBuf fboxes;                   // getScalarReactForce box descriptors
   int* d_retry = nullptr;             // per-cell flags of the FP64 fallback pass
@@ -467,9 +477,13 @@ struct RoundLists {
 // Newton correction and step of those that keep their Newton matrix; Jacobian
 // and inverse of the others, then their step; the control kernel for whatever
 // the step kernel passed on.  Every kernel appends to the lists of the next
-// round, whose counters the right-hand-side kernel clears.
+// round, whose counters the right-hand-side kernel clears.  side (may be st):
+// the Jacobian and the inverse need nothing of this round's other kernels and
+// share no data with them before the step of their cells, so in the captured
+// graph they run on a branch of their own: a round of few cells is a chain of
+// kernels of 5 to 20 us each, and this takes two of the six off it.
 int enqueue_round(b200chem_reactor* h, int lut, RoundsParams R, const RoundsGrids& G, const RoundLists& Ls, int cur,
-                  cudaStream_t st) {
+                  cudaStream_t st, cudaStream_t side) {
   const int* cnt = Ls.cnt[cur];
   R.cnt_next = Ls.cnt[1 - cur];
   for (int k = 0; k < kRoundLists; ++k) R.list[k] = Ls.lst[1 - cur][k];
@@ -480,25 +494,40 @@ int enqueue_round(b200chem_reactor* h, int lut, RoundsParams R, const RoundsGrid
       {kRoundsGj, B200CHEM_PROF_GJ, 0, kRlSetup, cnt, Ls.lst[cur][kRlSetup]},
       {kRoundsStep, B200CHEM_PROF_CTRL_SETUP, 1, kRlSetup, cnt, Ls.lst[cur][kRlSetup]},
       {kRoundsCtrl, B200CHEM_PROF_CTRL_RARE, 0, kRlCtrl, R.cnt_next, Ls.lst[1 - cur][kRlCtrl]}};
+  if (side != st) {
+    CK(cudaEventRecord(h->cap_ev[0], st));
+    CK(cudaStreamWaitEvent(side, h->cap_ev[0], 0));
+  }
   for (const auto& k : seq) {
     R.list_in = k.list;
     R.cnt_in = k.c + k.in;
-    const int err = launch_kernel(h, lut, k.what, k.kind, R, G, k.setup_pass, R.cnt_in, 0, st);
+    const bool setup = k.what == kRoundsJac || k.what == kRoundsGj;
+    if (side != st && k.setup_pass) {
+      CK(cudaEventRecord(h->cap_ev[1], side));
+      CK(cudaStreamWaitEvent(st, h->cap_ev[1], 0));
+    }
+    const int err = launch_kernel(h, lut, k.what, k.kind, R, G, k.setup_pass, R.cnt_in, 0, setup ? side : st);
     if (err) return err;
   }
   return 0;
 }
 
 // Captures `rounds` rounds (an even number: the two sets of lists swap roles
-// every round, so the graph starts and ends on the same one) into h->rgraph,
+// every round, so the graph starts and ends on the same one) into h->rgraph[cls],
 // updating the executable graph in place when only kernel parameters
 // changed.
 int capture_rounds(b200chem_reactor* h, int lut, const RoundsParams& R, const RoundsGrids& G, int rounds,
-                   const RoundLists& Ls) {
+                   const RoundLists& Ls, int cls) {
+  // few cells: the setup kernels on a branch (many: 10 % slower, the kernels
+  // that overlap contend for the L2)
+  cudaGraphExec_t& exec = h->rgraph[cls];
   if (!h->cap_stream) CK(cudaStreamCreateWithFlags(&h->cap_stream, cudaStreamNonBlocking));
+  if (!h->cap_side) CK(cudaStreamCreateWithFlags(&h->cap_side, cudaStreamNonBlocking));
+  for (cudaEvent_t& e : h->cap_ev)
+    if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   CK(cudaStreamBeginCapture(h->cap_stream, cudaStreamCaptureModeThreadLocal));
   int err = 0;
-  for (int r = 0; r < rounds && !err; ++r) err = enqueue_round(h, lut, R, G, Ls, r & 1, h->cap_stream);
+  for (int r = 0; r < rounds && !err; ++r) err = enqueue_round(h, lut, R, G, Ls, r & 1, h->cap_stream, cls > 0 ? h->cap_side : h->cap_stream);
   cudaGraph_t g = nullptr;
   const cudaError_t ce = cudaStreamEndCapture(h->cap_stream, &g);
   if (err || ce != cudaSuccess) {
@@ -506,25 +535,25 @@ int capture_rounds(b200chem_reactor* h, int lut, const RoundsParams& R, const Ro
     cudaGetLastError();
     return err ? err : set_err(B200CHEM_ECUDA, "graph capture of the rounds failed: %s", cudaGetErrorString(ce));
   }
-  if (h->rgraph && h->rgraph_rounds == rounds) {
+  if (exec && h->rgraph_rounds[cls] == rounds) {
     cudaGraphExecUpdateResultInfo info;
-    if (cudaGraphExecUpdate(h->rgraph, g, &info) != cudaSuccess) {
+    if (cudaGraphExecUpdate(exec, g, &info) != cudaSuccess) {
       cudaGetLastError();
-      cudaGraphExecDestroy(h->rgraph);
-      h->rgraph = nullptr;
+      cudaGraphExecDestroy(exec);
+      exec = nullptr;
     }
-  } else if (h->rgraph) {
-    cudaGraphExecDestroy(h->rgraph);
-    h->rgraph = nullptr;
+  } else if (exec) {
+    cudaGraphExecDestroy(exec);
+    exec = nullptr;
   }
   cudaError_t ie = cudaSuccess;
-  if (!h->rgraph) ie = cudaGraphInstantiate(&h->rgraph, g, 0);
+  if (!exec) ie = cudaGraphInstantiate(&exec, g, 0);
   cudaGraphDestroy(g);
   if (ie != cudaSuccess) {
-    h->rgraph = nullptr;
+    exec = nullptr;
     return set_err(B200CHEM_ECUDA, "cannot instantiate the round graph: %s", cudaGetErrorString(ie));
   }
-  h->rgraph_rounds = rounds;
+  h->rgraph_rounds[cls] = rounds;
   return 0;
 }
 
@@ -540,12 +569,12 @@ int launch_rounds(b200chem_reactor* h, const ReactParams& P, cudaStream_t st, in
     return set_err(B200CHEM_ETOOBIG, "setup kernels need %d B of shared memory per CTA",
                    std::max(SL.jac_smem, 4 * SL.gj_smem_per_warp));
   if (h->rgrid_lut != lut) {
-    CK(rounds_grids_for(h->N, lut, SL, h->sm_count, &h->rgrid));
+    CK(rounds_grids_for(h->N, h->R, h->gen_mech, lut, SL, h->sm_count, &h->rgrid));
     h->rgrid_lut = lut;
   }
   const b200chem_tuning& T = h->tune;
   RoundsGrids G = h->rgrid;
-  G.rhs = tuned_grid(h->rgrid.rhs, h->sm_count, T.rhs_ctas_per_sm);
+  G.rhs.thread = tuned_grid(h->rgrid.rhs.thread, h->sm_count, T.rhs_ctas_per_sm);
   G.step = tuned_grid(h->rgrid.step, h->sm_count, T.ctrl_ctas_per_sm);
   G.ctrl = tuned_grid(h->rgrid.ctrl, h->sm_count, T.ctrl_ctas_per_sm);
   G.jac = tuned_grid(h->rgrid.jac, h->sm_count, T.jac_ctas_per_sm);
@@ -602,17 +631,33 @@ int launch_rounds(b200chem_reactor* h, const ReactParams& P, cudaStream_t st, in
     err = launch_kernel(h, lut, kRoundsStart, B200CHEM_PROF_START, R, G, 0, nullptr, R.nchunk, st);
     if (err) return err;
     h->launches++;
-    if (graph) {
-      err = capture_rounds(h, lut, R, G, per_check, Ls);
-      if (err) return err;
-    }
+    // the launch shape follows the live cells, which only become fewer
+    bool captured[kRoundClasses] = {};
+    long long live = R.nchunk;
     for (long long round = 0;; round += per_check) {
       if (round >= max_rounds) return set_err(B200CHEM_EINTEGRATE, "round-based integrator did not finish");
+      const int cls = live <= kTinyCells ? 2 : live <= G.rhs.warp_cells ? 1 : 0;
+      RoundsGrids Gc = G;
+      Gc.rhs_by_warp = R.gen_mech && live <= G.rhs.warp_cells;
+      if (cls == 2) {
+        const int per_cta = 128 / rounds::ctrl_group(h->n);
+        const int need = (kTinyCells + per_cta - 1) / per_cta;
+        Gc.step = std::min(G.step, need);
+        Gc.ctrl = std::min(G.ctrl, need);
+        Gc.gj = std::min(G.gj, h->n <= 32 && lut == 4 ? need : kTinyCells / 4);
+        Gc.rhs.warp = std::min(G.rhs.warp, kTinyCells / 4);
+        Gc.rhs.thread = std::min(G.rhs.thread, kTinyCells / kRoundsRhsBlock);
+      }
       if (graph) {
-        CK(cudaGraphLaunch(h->rgraph, st));
+        if (!captured[cls]) {
+          err = capture_rounds(h, lut, R, Gc, per_check, Ls, cls);
+          if (err) return err;
+          captured[cls] = true;
+        }
+        CK(cudaGraphLaunch(h->rgraph[cls], st));
       } else {
         for (int r = 0; r < per_check; ++r) {
-          err = enqueue_round(h, lut, R, G, Ls, r & 1, st);
+          err = enqueue_round(h, lut, R, Gc, Ls, r & 1, st, st);
           if (err) return err;
         }
       }
@@ -620,7 +665,8 @@ int launch_rounds(b200chem_reactor* h, const ReactParams& P, cudaStream_t st, in
       // per_check is even: the live cells are back in the first list
       CK(cudaMemcpyAsync(h->h_rcnt, Ls.cnt[0] + kRlRhs, sizeof(int), cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));
-      if (*h->h_rcnt == 0) break;
+      live = *h->h_rcnt;
+      if (live == 0) break;
     }
   }
   return 0;
@@ -1608,7 +1654,7 @@ int b200chem_autotune(b200chem_handle h, const double* rhoY, const double* extF_
     return set_err(B200CHEM_EINTEGRATE, "react of the autotuner sample failed under the starting launch shape");
   }
   const int sm = h->sm_count;
-  const int max_per_sm[4] = {std::max(1, h->rgrid.rhs / sm), std::max(1, h->rgrid.ctrl / sm),
+  const int max_per_sm[4] = {std::max(1, h->rgrid.rhs.thread / sm), std::max(1, h->rgrid.step / sm),
                              std::max(1, h->rgrid.jac / sm), std::max(1, h->rgrid.gj / sm)};
   for (int pass = 0; pass < 2 && !err && trials < max_trials; ++pass) {
     for (int field = 0; field < 7 && !err && trials < max_trials; ++field) {
@@ -1673,7 +1719,8 @@ int b200chem_destroy(b200chem_handle h) {
   if (h->d_rcnt) cudaFree(h->d_rcnt);
   if (h->h_rcnt) cudaFreeHost(h->h_rcnt);
   if (h->h_cmech) cudaFreeHost(h->h_cmech);
-  if (h->rgraph) cudaGraphExecDestroy(h->rgraph);
+  for (cudaGraphExec_t g : h->rgraph)
+    if (g) cudaGraphExecDestroy(g);
   staged_free(h->cboxes);
   staged_free(h->fboxes);
   if (h->d_zero_mask) cudaFree(h->d_zero_mask);
@@ -1681,6 +1728,9 @@ int b200chem_destroy(b200chem_handle h) {
   for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
   if (h->h_pcnt) cudaFreeHost(h->h_pcnt);
   if (h->cap_stream) cudaStreamDestroy(h->cap_stream);
+  if (h->cap_side) cudaStreamDestroy(h->cap_side);
+  for (cudaEvent_t e : h->cap_ev)
+    if (e) cudaEventDestroy(e);
   delete h;
   return 0;
 }
@@ -1727,6 +1777,10 @@ static int inst_launch(b200chem_handle h, const double* rhoY, const double* rhoH
                        int64_t ncells, void* stream) {
   if (!h || !rhoY || !rhoH || !T || ncells < 0) return set_err(B200CHEM_EINVAL, "bad arguments");
   if (ncells == 0) return 0;
+  if (h->gen_mech) {  // the generated right-hand side; other mechanisms a warp per cell from the tables
+    CK(inst_launch_gen(h->mech, rhoY, rhoH, T, rhoYdot, ncells, h->sm_count, static_cast<cudaStream_t>(stream)));
+    return 0;
+  }
   InstParams P;
   P.mech = h->mech;
   P.rhoY = rhoY;

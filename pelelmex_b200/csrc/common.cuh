@@ -145,7 +145,7 @@ constexpr int kRoundsRhsBlock = 64;  // threads per CTA of the rhs kernel
 enum { kRoundsStart = 0, kRoundsRhs, kRoundsStep, kRoundsJac, kRoundsGj, kRoundsCtrl };
 
 // Scratch of the setup kernels.  Jacobian kernel, per team of warps: C, g/RT,
-// h/RT, hm [Npad], the Jacobian, the third-body row and the temperature row,
+// h/RT, hm [Npad], the Jacobian, the third-body, rate and temperature rows,
 // and the reactions' derivatives [jac_nd] (here or in device memory).
 // Inverse kernel, per warp: Dsc [Npad] (double), matrix [n][ldl] and pivot
 // column [Npad] (LUT), two index arrays [Npad] (int), or the lane groups' form.
@@ -181,8 +181,15 @@ struct RoundsParams {
   int gen_mech;             // 1: the mechanism has a generated right-hand side
 };
 
+// CTAs of the right-hand-side kernels that fit the GPU (one thread per cell;
+// one warp per cell, for at most warp_cells live cells and generated code only).
+struct RhsGrid {
+  int thread, warp, warp_cells;
+};
 struct RoundsGrids {
-  int start, rhs, step, ctrl, jac, gj;
+  int start, step, ctrl, jac, gj;
+  RhsGrid rhs;
+  int rhs_by_warp;  // which of the two a launch takes
 };
 
 // Handle accessors (defined with the handle in b200chem.cu).
@@ -196,10 +203,23 @@ unsigned long long handle_digest(b200chem_handle h);  // FNV-1a digest of the me
 int handle_sm_count(b200chem_handle h);
 
 bool rounds_supported(int N);
+// Right-hand-side kernels (react_rhs.cu): CTAs that fit the GPU, and a launch.
+cudaError_t rhs_grid(int N, int R, int gen, int sm_count, RhsGrid* G);
+cudaError_t rhs_launch(int N, const RoundsParams& R, int grid, int by_warp, cudaStream_t st);
+// The generated code's thread form (react_gen.cu); grid: CTAs that fit the GPU.
+cudaError_t gen_rhs_grid(int N, int sm_count, int* grid);
+cudaError_t gen_rhs_launch(int N, const RoundsParams& R, int grid, cudaStream_t st);
+cudaError_t gen_rates_launch(int N, const DevMech& m, const double* rhoY, const double* T, double* dot,
+                             long long ncells, int grid, cudaStream_t st);
+// T from (h, Y) and mass production rates (null: T only) with the generated
+// right-hand side of the mechanism, one thread per cell, MKS.
+cudaError_t inst_launch_gen(const DevMech& m, const double* rhoY, const double* rhoH, double* T, double* dot,
+                            long long ncells, int sm_count, cudaStream_t st);
 RoundsSetupLayout rounds_setup_layout(int N, int lut_bytes, int jac_nd);
 long long rounds_state_bytes_per_cell(int N, int lut_bytes);
 rounds::RState rounds_carve(void* base, long long cap, int N, int lut_bytes);
-cudaError_t rounds_grids_for(int N, int lut_bytes, const RoundsSetupLayout& SL, int sm_count, RoundsGrids* G);
+cudaError_t rounds_grids_for(int N, int R, int gen, int lut_bytes, const RoundsSetupLayout& SL, int sm_count,
+                             RoundsGrids* G);
 cudaError_t rounds_launch(int N, int lut_bytes, int what, const RoundsParams& R, const RoundsGrids& G, int setup_pass,
                           cudaStream_t st);
 

@@ -2,12 +2,14 @@
 // of the reaction rates add to which entry of d(wdot)/d(C, T).
 //
 // Derivatives of reaction j, from dptr[j]: one per species slot (by that
-// slot's concentration, reactants 0..3 then products 4..7), one by T, and for
-// third-body and falloff reactions one by the third-body concentration.
+// slot's concentration, reactants 0..3 then products 4..7), one by T, the rate
+// itself, and for third-body and falloff reactions the derivative by the
+// third-body concentration.
 // Entry (k, l): sum over the reactions of nu_k times the derivative by slot l
 // or T, plus nu_k (eff_l - 1) times the third-body one where the efficiency of
 // l differs from 1.  The default efficiency's part, nu_k times the third-body
-// derivative for every l, is kept once per k (the row u).
+// derivative for every l, is kept once per k (the row u); the production rates
+// themselves, nu_k times the rates, follow it (the row w).
 #pragma once
 #include <algorithm>
 #include <cstdint>
@@ -26,7 +28,7 @@ struct JacTable {
 
 // sp, nu: [8][R] species (-1 empty) and signed stoichiometry; eff_m1:
 // efficiency - 1.  ld: column stride of the kernel's Jacobian; the row u lies
-// at (N + 1) ld.  False when the table's index fields cannot hold the
+// at (N + 1) ld, the row w behind it.  False when the table's index fields cannot hold the
 // mechanism (coef_bits of 32 for the coefficient).
 inline bool build_jac_table(int N, int R, const int* rtype, const int* sp, const int* nu, const int* eff_ptr,
                             const int* eff_sp, const double* eff_m1, int ld, int coef_bits, JacTable* T) {
@@ -52,14 +54,15 @@ inline bool build_jac_table(int N, int R, const int* rtype, const int* sp, const
       if (r.second == 0.0) continue;
       for (int c = 0; c < ncol; ++c) sums[cols[c] * ld + r.first].push_back({T->nd + c, r.second});
       sums[N * ld + r.first].push_back({T->nd + ncol, r.second});
+      sums[u0 + N + r.first].push_back({T->nd + ncol + 1, r.second});
       if (rtype[j] != 0) {
-        const int d = T->nd + ncol + 1;
+        const int d = T->nd + ncol + 2;
         sums[u0 + r.first].push_back({d, r.second});
         for (int q = eff_ptr[j]; q < eff_ptr[j + 1]; ++q)
           if (eff_m1[q] != 0.0) sums[eff_sp[q] * ld + r.first].push_back({d, r.second * eff_m1[q]});
       }
     }
-    T->nd += ncol + 1 + (rtype[j] != 0 ? 1 : 0);
+    T->nd += ncol + 2 + (rtype[j] != 0 ? 1 : 0);
   }
   if (T->nd >= (1 << (32 - coef_bits))) return false;
   std::vector<Entry> e;

@@ -19,7 +19,6 @@
 
 #include "bdf_rounds.cuh"
 #include "common.cuh"
-#include "gen_mechs.cuh"  // mechanism-specific right-hand sides (written by the build)
 
 namespace b200 {
 using namespace rounds;
@@ -120,242 +119,7 @@ __device__ __forceinline__ void warp_stats(long long* stats, bool done, bool fai
   }
 }
 
-// ------------------------------------------------------------ mechanism
-// One reaction's rate of progress for the thread's cell; C, g/RT per thread
-// in shared memory at [k * ss].  Every thread of the warp evaluates the SAME
-// reaction j, so the table reads are broadcasts and the branches uniform.
-__device__ __forceinline__ double r_progress(const DevMech& m, int j, double T, double lnT, double invT,
-                                             double Ctot, double lnPRT, const double* sC, const double* sG,
-                                             int ss) {
-  const int R = m.R;
-  const double lnA = __ldg(m.arr + j), b = __ldg(m.arr + R + j), ea = __ldg(m.arr + 2 * R + j);
-  const double kinf = exp(lnA + b * lnT - ea * invT);
-  const int type = __ldg(m.rtype + j);
-  const int flags = __ldg(m.rflags + j);
-  double M = 0.0;
-  if (type != 0) {
-    M = Ctot;
-    const int e0 = __ldg(m.eff_ptr + j), e1 = __ldg(m.eff_ptr + j + 1);
-    for (int q = e0; q < e1; ++q) M += __ldg(m.eff_m1 + q) * sC[__ldg(m.eff_sp + q) * ss];
-  }
-  double kf = kinf;
-  if (type >= 2) {
-    const double lnA0 = __ldg(m.arr_lo + j), b0 = __ldg(m.arr_lo + R + j), ea0 = __ldg(m.arr_lo + 2 * R + j);
-    const double k0 = exp(lnA0 + b0 * lnT - ea0 * invT);
-    const double Pr = k0 * M / kinf;
-    double F = 1.0;
-    if (type == 3) {
-      const double a = __ldg(m.troe + j), i3 = __ldg(m.troe + R + j), i1 = __ldg(m.troe + 2 * R + j);
-      const double t2 = __ldg(m.troe + 3 * R + j);
-      double Fc = (1.0 - a) * exp(-T * i3) + a * exp(-T * i1);
-      if (flags & 4) Fc += exp(-t2 * invT);
-      const double logFc = log10(fmax(Fc, 1e-300));
-      const double c = -0.4 - 0.67 * logFc, nn = 0.75 - 1.27 * logFc;
-      const double u = log10(fmax(Pr, 1e-300)) + c;
-      const double f1 = u / (nn - 0.14 * u);
-      F = exp(kLn10 * (logFc / (1.0 + f1 * f1)));
-    }
-    kf = kinf * Pr / (1.0 + Pr) * F;
-  }
-  // slots 0..3 reactants (nu < 0), 4..7 products (nu > 0)
-  double pf = 1.0, pr = 1.0, sg = 0.0;
-#pragma unroll
-  for (int sl = 0; sl < 8; ++sl) {
-    const int k = __ldg(m.sp + sl * R + j);
-    if (k >= 0) {
-      const int nu = __ldg(m.nu + sl * R + j);
-      const int na = nu < 0 ? -nu : nu;
-      const double ck = sC[k * ss];
-      double p = ck;
-      for (int e = 1; e < na; ++e) p *= ck;
-      if (sl < 4) pf *= p;
-      else pr *= p;
-      sg += nu * sG[k * ss];
-    }
-  }
-  double kr = 0.0;
-  if (flags & 2) {
-    const double lr = __ldg(m.arr_rev + j), br = __ldg(m.arr_rev + R + j), er = __ldg(m.arr_rev + 2 * R + j);
-    kr = exp(lr + br * lnT - er * invT);
-  } else if (flags & 1) {
-    kr = kf * exp(sg - __ldg(m.sdnu + j) * lnPRT);
-  }
-  double q = kf * pf - kr * pr;
-  if (type == 1) q *= M;
-  return q;
-}
-
-// HP right-hand side at v.yev (forcing v.F) into v.fv, thread per cell.
-template <int NS>
-__device__ __forceinline__ void r_rhs(const DevMech& m, const RVec<NS + 1>& v, double* sC, double* sG, double* sW,
-                                      int ss) {
-  const double T = v.yev(NS);
-  const double lnT = log(T), invT = 1.0 / T;
-  double Ctot = 0.0, rcp = 0.0;
-#pragma unroll 1
-  for (int k = 0; k < NS; ++k) {
-    double cpR, hRT, sR, dcpR;
-    nasa7(m, k, T, lnT, cpR, hRT, sR, dcpR);
-    const double iw = __ldg(m.inv_mw + k);
-    const double yk = v.yev(k);
-    const double Ck = yk * iw;
-    sC[k * ss] = Ck;
-    sG[k * ss] = hRT - sR;
-    sW[k * ss] = 0.0;
-    Ctot += Ck;
-    rcp += yk * cpR * kRu * iw;
-  }
-  const double lnPRT = log(kPatm / (kRu * T));
-  const int R = m.R;
-#pragma unroll 1
-  for (int j = 0; j < R; ++j) {
-    const double q = r_progress(m, j, T, lnT, invT, Ctot, lnPRT, sC, sG, ss);
-#pragma unroll
-    for (int sl = 0; sl < 8; ++sl) {
-      const int k = __ldg(m.sp + sl * R + j);
-      if (k >= 0) {
-        sW[k * ss] += (double)__ldg(m.nu + sl * R + j) * q;
-      }
-    }
-  }
-  double hs = 0.0;
-#pragma unroll 1
-  for (int k = 0; k < NS; ++k) {
-    double cpR, hRT, sR, dcpR;
-    nasa7(m, k, T, lnT, cpR, hRT, sR, dcpR);
-    const double yd = sW[k * ss] * __ldg(m.mw + k) + v.F(k);
-    v.fv(k) = yd;
-    hs += hRT * kRu * T * __ldg(m.inv_mw + k) * yd;
-  }
-  v.fv(NS) = (v.F(NS) - hs) / rcp;
-}
-
-// ------------------------------------------------ constant-memory table
-__constant__ __align__(16) unsigned char c_mech[kConstMechBytes];
-
-__device__ __forceinline__ const CMechHeader& cm_hdr() { return *reinterpret_cast<const CMechHeader*>(c_mech); }
-__device__ __forceinline__ const double* cm_d(int off) { return reinterpret_cast<const double*>(c_mech + off); }
-
-// NASA-7 cp/R, h/RT, g/RT of species k at T from the constant table.
-__device__ __forceinline__ void cm_nasa7(const CMechHeader& H, int k, double T, double lnT, double invT,
-                                        double& cpR, double& hRT, double& gRT) {
-  const double* nasa = cm_d(H.off_nasa);
-  const int N = H.N;
-  const int base = (T < nasa[k]) ? 1 : 8;
-  const double a0 = nasa[(base + 0) * N + k], a1 = nasa[(base + 1) * N + k], a2 = nasa[(base + 2) * N + k];
-  const double a3 = nasa[(base + 3) * N + k], a4 = nasa[(base + 4) * N + k], a5 = nasa[(base + 5) * N + k];
-  const double a6 = nasa[(base + 6) * N + k];
-  cpR = a0 + T * (a1 + T * (a2 + T * (a3 + T * a4)));
-  hRT = a0 + T * (a1 / 2 + T * (a2 / 3 + T * (a3 / 4 + T * a4 / 5))) + a5 * invT;
-  const double sR = a0 * lnT + T * (a1 + T * (a2 / 2 + T * (a3 / 3 + T * a4 / 4))) + a6;
-  gRT = hRT - sR;
-}
-
-// Rate of progress of reaction j from the constant table (same formulas as
-// r_progress).
-__device__ __forceinline__ double cm_progress(const CMechHeader& H, int j, double T, double lnT, double invT,
-                                              double Ctot, double lnPRT, const double* sC, const double* sG,
-                                              int ss) {
-  const RxnC& r = reinterpret_cast<const RxnC*>(c_mech + H.off_rxn)[j];
-  const int type = r.type, flags = r.flags;
-  const double kinf = exp(r.lnA + r.b * lnT - r.ea * invT);
-  double M = 0.0;
-  if (type != 0) {
-    M = Ctot;
-    const short* esp = reinterpret_cast<const short*>(c_mech + H.off_effsp);
-    const double* em1 = cm_d(H.off_effm1);
-    for (int q = r.e0; q < r.e1; ++q) M += em1[q] * sC[esp[q] * ss];
-  }
-  double kf = kinf;
-  if (type >= 2) {
-    const double k0 = exp(r.lnA0 + r.b0 * lnT - r.ea0 * invT);
-    const double Pr = k0 * M / kinf;
-    double F = 1.0;
-    if (type == 3) {
-      double Fc = (1.0 - r.ta) * exp(-T * r.t3i) + r.ta * exp(-T * r.t1i);
-      if (flags & 4) Fc += exp(-r.t2 * invT);
-      const double logFc = log10(fmax(Fc, 1e-300));
-      const double c = -0.4 - 0.67 * logFc, nn = 0.75 - 1.27 * logFc;
-      const double u = log10(fmax(Pr, 1e-300)) + c;
-      const double f1 = u / (nn - 0.14 * u);
-      F = exp(kLn10 * (logFc / (1.0 + f1 * f1)));
-    }
-    kf = kinf * Pr / (1.0 + Pr) * F;
-  }
-  double pf = 1.0, pr = 1.0, sg = 0.0;
-#pragma unroll
-  for (int sl = 0; sl < 8; ++sl) {
-    const int k = r.sp[sl];
-    if (k >= 0) {
-      const int nu = r.nu[sl];
-      const int na = nu < 0 ? -nu : nu;
-      const double ck = sC[k * ss];
-      double p = ck;
-      for (int e = 1; e < na; ++e) p *= ck;
-      if (sl < 4) pf *= p;
-      else pr *= p;
-      sg += nu * sG[k * ss];
-    }
-  }
-  double kr = 0.0;
-  if (flags & 2) kr = exp(r.lr + r.br * lnT - r.er * invT);
-  else if (flags & 1) kr = kf * exp(sg - r.sdnu * lnPRT);
-  double q = kf * pf - kr * pr;
-  if (type == 1) q *= M;
-  return q;
-}
-
-// HP right-hand side from the constant table (thread per cell).
-template <int NS>
-__device__ __forceinline__ void cm_rhs(const RVec<NS + 1>& v, double* sC, double* sG, double* sW, int ss) {
-  const CMechHeader& H = cm_hdr();
-  const double* imw = cm_d(H.off_imw);
-  const double* mw = cm_d(H.off_mw);
-  const double T = v.yev(NS);
-  const double lnT = log(T), invT = 1.0 / T;
-  double Ctot = 0.0, rcp = 0.0;
-#pragma unroll 1
-  for (int k = 0; k < NS; ++k) {
-    double cpR, hRT, gRT;
-    cm_nasa7(H, k, T, lnT, invT, cpR, hRT, gRT);
-    const double yk = v.yev(k);
-    const double Ck = yk * imw[k];
-    sC[k * ss] = Ck;
-    sG[k * ss] = gRT;
-    sW[k * ss] = 0.0;
-    Ctot += Ck;
-    rcp += yk * cpR * kRu * imw[k];
-  }
-  const double lnPRT = log(kPatm / (kRu * T));
-  const int R = H.R;
-  const RxnC* rx = reinterpret_cast<const RxnC*>(c_mech + H.off_rxn);
-#pragma unroll 1
-  for (int j = 0; j < R; ++j) {
-    const double q = cm_progress(H, j, T, lnT, invT, Ctot, lnPRT, sC, sG, ss);
-#pragma unroll
-    for (int sl = 0; sl < 8; ++sl) {
-      const int k = rx[j].sp[sl];
-      if (k >= 0) sW[k * ss] += (double)rx[j].nu[sl] * q;
-    }
-  }
-  double hs = 0.0;
-#pragma unroll 1
-  for (int k = 0; k < NS; ++k) {
-    double cpR, hRT, gRT;
-    cm_nasa7(H, k, T, lnT, invT, cpR, hRT, gRT);
-    const double yd = sW[k * ss] * mw[k] + v.F(k);
-    v.fv(k) = yd;
-    hs += hRT * kRu * T * imw[k] * yd;
-  }
-  v.fv(NS) = (v.F(NS) - hs) / rcp;
-}
-
 }  // namespace
-
-cudaError_t rounds_upload_const(const void* blob, int bytes, cudaStream_t st) {
-  if (bytes > kConstMechBytes) return cudaErrorInvalidValue;
-  return cudaMemcpyToSymbolAsync(c_mech, blob, (size_t)bytes, 0, cudaMemcpyHostToDevice, st);
-}
 
 // ---------------------------------------------------------------- kernels
 template <int NS>
@@ -414,41 +178,6 @@ __global__ void __launch_bounds__(128) rk_start(RoundsParams R) {
     }
     warp_append(go, (int)slot, R.list[kRlRhs], R.cnt_next + kRlRhs);
     warp_stats(P.stats, done, true, masked, CellCounters{0, 0, 0, 0, 0, 0, 0});
-  }
-}
-
-// Minimum resident CTAs (of 64 threads) per SM requested for the
-// right-hand-side kernel: bounds its registers per thread.
-#ifndef B200_RHS_MIN_CTAS
-#define B200_RHS_MIN_CTAS 6
-#endif
-
-template <int NS>
-__global__ void __launch_bounds__(kRoundsRhsBlock, B200_RHS_MIN_CTAS) rk_rhs(RoundsParams R) {
-  constexpr int n = NS + 1;
-  extern __shared__ __align__(16) unsigned char dsm[];
-  __shared__ DevMech s_mech;
-  if (threadIdx.x == 0) s_mech = R.P.mech;
-  __syncthreads();
-  const int cnt = *R.cnt_in;
-  // counters of the lists this round's later kernels append to
-  if (blockIdx.x == 0 && threadIdx.x < kRoundLists) R.cnt_next[threadIdx.x] = 0;
-  double* sC = reinterpret_cast<double*>(dsm) + threadIdx.x;
-  double* sG = sC + NS * blockDim.x;
-  double* sW = sG + NS * blockDim.x;
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < cnt; idx += gridDim.x * blockDim.x) {
-    const int slot = R.list_in[idx] & ~kSetupFlag;
-    const RVec<n> v{reinterpret_cast<double*>(rec_of(R.S, slot) + R.S.L.off_vec)};
-    if (R.gen_mech) {
-      // generated code for this mechanism: every coefficient an immediate
-      if constexpr (NS == 9) gen::gen_rhs_synth_h2_9(&v.yev(0), &v.F(0), &v.fv(0));
-      else if constexpr (NS == 21) gen::gen_rhs_synth_ch4_21(&v.yev(0), &v.F(0), &v.fv(0));
-      else if constexpr (NS == 53) gen::gen_rhs_synth_c12_53(&v.yev(0), &v.F(0), &v.fv(0));
-    } else if (R.const_mech) {
-      cm_rhs<NS>(v, sC, sG, sW, blockDim.x);
-    } else {
-      r_rhs<NS>(s_mech, v, sC, sG, sW, blockDim.x);
-    }
   }
 }
 
@@ -1080,18 +809,20 @@ constexpr int jac_ld(int n) { return n | 1; }
 // 28 ms and take 15; with 21 species both take 15 ns a cell, the reactions).  The default third-body efficiency 1 of every
 // species is a row vector u added to all columns, the non-default ones are
 // terms.  3. the temperature row; 4. mass units, and the matrix into the cell
-// record (mat_idx order, consecutive 16-byte stores).
-// s: C, g/RT, h/RT, hm [Npad]; Js: [n][ld] column-major, then u [N] and the
-// temperature row [n]; entries outside the table stay zero.
+// record (mat_idx order, consecutive 16-byte stores).  The rates come along, so
+// the kernel needs no f and runs beside the right-hand sides.
+// s: C, g/RT, h/RT, hm [Npad]; Js: [n][ld] column-major, then u [N], w [N] and
+// the temperature row [n]; entries outside the table stay zero.
 template <int n, int CPL, int W>
 __device__ __forceinline__ void team_jac(const DevMech& m, const GrpScratch& s, double* hm, double* Js, double* D,
-                                         const Vec<CPL>& y, const Vec<CPL>& fy, double* J, int tid) {
+                                         const Vec<CPL>& y, const Vec<CPL>& F, double* J, int tid) {
   constexpr int N = n - 1, ld = jac_ld(n), TS = 32 * W;
   const int lane = tid & 31;
   const Grp<32> g(lane);
   const int R = m.R;
   double* u = Js + n * ld;
-  double* tr = u + N;
+  double* w = u + N;
+  double* tr = w + N;
   auto sync = [] {
     if constexpr (W == 1) __syncwarp();
     else __syncthreads();
@@ -1100,7 +831,7 @@ __device__ __forceinline__ void team_jac(const DevMech& m, const GrpScratch& s, 
   const double lnT = log(T), invT = 1.0 / T;
   double cpk[CPL], hk[CPL], dcpk[CPL];
   grp_species<32, CPL>(m, s, g, y, T, lnT, cpk, hk, dcpk);  // every warp writes the same values
-  double csum = 0.0, rcp = 0.0, drcp = 0.0, cpdot = 0.0, Tdot = 0.0;
+  double csum = 0.0, rcp = 0.0, drcp = 0.0;
 #pragma unroll
   for (int c = 0; c < CPL; ++c) {
     const int k = lane + 32 * c;
@@ -1108,17 +839,12 @@ __device__ __forceinline__ void team_jac(const DevMech& m, const GrpScratch& s, 
       csum += y.v[c] * __ldg(m.inv_mw + k);
       rcp += y.v[c] * cpk[c];
       drcp += y.v[c] * dcpk[c];
-      cpdot += cpk[c] * fy.v[c];
       hm[k] = hk[c] * __ldg(m.mw + k);
-    } else if (k == N) {
-      Tdot = fy.v[c];
     }
   }
   const double Ctot = g.sum(csum);
   rcp = g.sum(rcp);
   drcp = g.sum(drcp);
-  cpdot = g.sum(cpdot);
-  Tdot = g.sum(Tdot);
   const double lnPRT = log(kPatm / (kRu * T));
   sync();
   for (int j = tid; j < R; j += TS) {
@@ -1149,6 +875,7 @@ __device__ __forceinline__ void team_jac(const DevMech& m, const GrpScratch& s, 
       *d++ = (a < 4) ? kfm * p : -krm * p;
     }
     *d++ = mult * (e.kf * e.dlnkf_dT * e.pf - e.dkr_dT * e.pr);
+    *d++ = mult * (e.kf * e.pf - e.kr * e.pr);
     if (type != 0) *d = ceff;
   }
   sync();
@@ -1164,6 +891,21 @@ __device__ __forceinline__ void team_jac(const DevMech& m, const GrpScratch& s, 
     if (tgt >= 0) Js[tgt] = v;
   }
   sync();
+  // dT/dt and sum cp_k d(rhoY_k)/dt, by every warp
+  double hdot = 0.0, cpdot = 0.0, FH = 0.0;
+#pragma unroll
+  for (int c = 0; c < CPL; ++c) {
+    const int k = lane + 32 * c;
+    if (k < N) {
+      const double yd = w[k] * __ldg(m.mw + k) + F.v[c];
+      hdot += hk[c] * yd;
+      cpdot += cpk[c] * yd;
+    } else if (k == N) {
+      FH = F.v[c];
+    }
+  }
+  const double Tdot = (g.sum(FH) - g.sum(hdot)) / rcp;
+  cpdot = g.sum(cpdot);
   for (int l = tid; l < n; l += TS) {
     const double* col = Js + l * ld;
     double sum = 0.0;
@@ -1237,8 +979,8 @@ __global__ void __launch_bounds__(128, B200_JAC_MIN_CTAS) rk_jac(RoundsParams R)
   ms.q = ms.r1 = ms.r2 = ms.r3 = ms.r4 = nullptr;
   double* hm = d + 3 * SL.Npad;
   double* Js = d + 4 * SL.Npad;
-  double* D = SL.jac_d_global ? reinterpret_cast<double*>(R.wscratch) + (size_t)gt * SL.jac_nd : Js + n * ld + NS + n;
-  for (int e = tid; e < n * ld + NS; e += 32 * W) Js[e] = 0.0;
+  double* D = SL.jac_d_global ? reinterpret_cast<double*>(R.wscratch) + (size_t)gt * SL.jac_nd : Js + n * ld + 2 * NS + n;
+  for (int e = tid; e < n * ld + 2 * NS; e += 32 * W) Js[e] = 0.0;
   const RLayout RL = R.S.L;
   for (int idx = gt; idx < cnt; idx += nteams) {
     const int slot = R.list_in[idx];
@@ -1246,14 +988,14 @@ __global__ void __launch_bounds__(128, B200_JAC_MIN_CTAS) rk_jac(RoundsParams R)
     // the cells were chosen by CVODE's jbad rule at their prediction, which
     // already counted the refresh
     const RVec<n> v{reinterpret_cast<double*>(rec + RL.off_vec)};
-    Vec<CPL> y, fy;
+    Vec<CPL> y, F;
 #pragma unroll
     for (int cc = 0; cc < CPL; ++cc) {
       const int i = lane + 32 * cc;
       y.v[cc] = (i < n) ? v.yev(i) : 0.0;
-      fy.v[cc] = (i < n) ? v.fv(i) : 0.0;
+      F.v[cc] = (i < n) ? v.F(i) : 0.0;
     }
-    team_jac<n, CPL, W>(s_mech, ms, hm, Js, D, y, fy, reinterpret_cast<double*>(rec + RL.off_j), tid);
+    team_jac<n, CPL, W>(s_mech, ms, hm, Js, D, y, F, reinterpret_cast<double*>(rec + RL.off_j), tid);
   }
 }
 
@@ -1371,16 +1113,10 @@ __global__ void __launch_bounds__(128, gj_min_ctas<NS + 1, LUT>()) rk_gj(RoundsP
 // ------------------------------------------------------------ host side
 namespace {
 
-template <int NS>
-int rhs_smem(int block) { return 3 * NS * block * (int)sizeof(double); }
-
 template <int NS, typename LUT>
 cudaError_t rounds_setup_attrs(const RoundsSetupLayout& SL) {
   constexpr int n = NS + 1;
-  cudaError_t e = cudaFuncSetAttribute(rk_rhs<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       rhs_smem<NS>(kRoundsRhsBlock));
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(rk_jac<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SL.jac_smem);
+  cudaError_t e = cudaFuncSetAttribute(rk_jac<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SL.jac_smem);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(rk_step<NS, LUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, step_smem<n>());
   if (e != cudaSuccess) return e;
@@ -1389,16 +1125,13 @@ cudaError_t rounds_setup_attrs(const RoundsSetupLayout& SL) {
 }
 
 template <int NS, typename LUT>
-cudaError_t rounds_grids(const RoundsSetupLayout& SL, int sm_count, RoundsGrids* G) {
+cudaError_t rounds_grids(int R, int gen, const RoundsSetupLayout& SL, int sm_count, RoundsGrids* G) {
   constexpr int n = NS + 1;
   cudaError_t e = rounds_setup_attrs<NS, LUT>(SL);
   if (e != cudaSuccess) return e;
   int b = 0;
-  // grid sized for the generated right-hand side (no shared memory); the
-  // table forms run the same grid-stride loop with fewer CTAs resident
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rk_rhs<NS>, kRoundsRhsBlock, 0)) != cudaSuccess)
-    return e;
-  G->rhs = std::max(1, b) * sm_count;
+  if ((e = rhs_grid(NS, R, gen, sm_count, &G->rhs)) != cudaSuccess) return e;
+  G->rhs_by_warp = 0;
   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, rk_step<NS, LUT>, 128, step_smem<n>())) !=
       cudaSuccess)
     return e;
@@ -1425,9 +1158,7 @@ cudaError_t rounds_launch_t(int what, const RoundsParams& R, const RoundsGrids& 
       rk_start<NS><<<G.start, 128, 0, st>>>(R);
       break;
     case kRoundsRhs:
-      // the generated right-hand side keeps everything in registers
-      rk_rhs<NS><<<G.rhs, kRoundsRhsBlock, R.gen_mech ? 0 : rhs_smem<NS>(kRoundsRhsBlock), st>>>(R);
-      break;
+      return rhs_launch(NS, R, G.rhs_by_warp ? G.rhs.warp : G.rhs.thread, G.rhs_by_warp, st);
     case kRoundsStep:
       rk_step<NS, LUT><<<G.step, 128, step_smem<n>(), st>>>(R, setup_pass);
       break;
@@ -1458,7 +1189,7 @@ RoundsSetupLayout rounds_setup_layout(int N, int lut_bytes, int jac_nd) {
   // scratch of a Jacobian team; the reactions' derivatives move to device
   // memory where they would leave fewer than two CTAs on an SM
   const int teams = 4 / jac_warps(n);
-  const long long fixed = 8LL * (4 * L.Npad + n * jac_ld(n) + N + n), dbytes = 8LL * jac_nd;
+  const long long fixed = 8LL * (4 * L.Npad + n * jac_ld(n) + 2 * N + n), dbytes = 8LL * jac_nd;
   L.jac_nd = jac_nd;
   L.jac_d_global = teams * (fixed + dbytes) > 100 * 1024;
   L.jac_smem_per_team = (int)((fixed + (L.jac_d_global ? 0 : dbytes) + 15) & ~15LL);
@@ -1482,12 +1213,16 @@ RState rounds_carve(void* base, long long cap, int N, int lut_bytes) {
   return S;
 }
 
-cudaError_t rounds_grids_for(int N, int lut_bytes, const RoundsSetupLayout& SL, int sm_count, RoundsGrids* G) {
-  if (N == 9) return lut_bytes == 4 ? rounds_grids<9, float>(SL, sm_count, G) : rounds_grids<9, double>(SL, sm_count, G);
+cudaError_t rounds_grids_for(int N, int R, int gen, int lut_bytes, const RoundsSetupLayout& SL, int sm_count,
+                             RoundsGrids* G) {
+  if (N == 9)
+    return lut_bytes == 4 ? rounds_grids<9, float>(R, gen, SL, sm_count, G) : rounds_grids<9, double>(R, gen, SL, sm_count, G);
   if (N == 21)
-    return lut_bytes == 4 ? rounds_grids<21, float>(SL, sm_count, G) : rounds_grids<21, double>(SL, sm_count, G);
+    return lut_bytes == 4 ? rounds_grids<21, float>(R, gen, SL, sm_count, G)
+                          : rounds_grids<21, double>(R, gen, SL, sm_count, G);
   if (N == 53)
-    return lut_bytes == 4 ? rounds_grids<53, float>(SL, sm_count, G) : rounds_grids<53, double>(SL, sm_count, G);
+    return lut_bytes == 4 ? rounds_grids<53, float>(R, gen, SL, sm_count, G)
+                          : rounds_grids<53, double>(R, gen, SL, sm_count, G);
   return cudaErrorInvalidValue;
 }
 
@@ -1505,15 +1240,4 @@ cudaError_t rounds_launch(int N, int lut_bytes, int what, const RoundsParams& R,
   return cudaErrorInvalidValue;
 }
 
-}  // namespace b200
-
-namespace b200 {
-// Generated right-hand side matching a mechanism digest: 0 none, else the
-// species count of the generated code.
-int rounds_generated_for(unsigned long long digest) {
-  if (digest == gen::kGenDigest_synth_h2_9) return 9;
-  if (digest == gen::kGenDigest_synth_ch4_21) return 21;
-  if (digest == gen::kGenDigest_synth_c12_53) return 53;
-  return 0;
-}
 }  // namespace b200

@@ -3,14 +3,14 @@ the reference's mechanisms).
 
 For a flattened mechanism this writes a device function
 
-    void gen_rhs_<name>(const double* y, const double* F, double* out)
+    void gen_rhs_<name>(const double* y, const double* F, double* out, ...)
 
 with every rate constant, stoichiometric coefficient, efficiency and NASA-7
-coefficient as an immediate, so that concentrations, g/RT and production
-rates live in registers and no table is read.  The formulas are the ones of
-the table-driven right-hand side (Chemkin formalism: Arrhenius, third body,
-Lindemann / Troe falloff, reverse rates from Kc), evaluated in the same
-order per reaction.
+coefficient as an operand in constant memory, so that concentrations and production rates live
+in registers and no table is read.  The formulas are the ones of the
+table-driven right-hand side (Chemkin formalism: Arrhenius, third body,
+Lindemann / Troe falloff, reverse rates from Kc); Kc is formed from one
+exponential per species instead of one per reaction.
 
 The function is selected at handle creation by a 64-bit FNV-1a digest of the
 mechanism description (mechanism_digest), computed identically here and in
@@ -50,135 +50,216 @@ def _d(x: float) -> str:
     return repr(float(x))
 
 
+KRU = 8.31446261815324e7  # erg/mol/K, as in the device code
+# largest magnitude of an exponential's argument in the generated code (its
+# exponential has no overflow or underflow handling)
+EXP_LIMIT = 690.0
+
+
+def _nasa_g(nasa, T):
+    """g/RT of every species at T (numpy, NASA-7)."""
+    a = np.where((T < nasa[:, :1]), nasa[:, 1:8], nasa[:, 8:15]).T
+    h = a[0] + T * (a[1] / 2 + T * (a[2] / 3 + T * (a[3] / 4 + T * a[4] / 5))) + a[5] / T
+    return h - (a[0] * np.log(T) + T * (a[1] + T * (a[2] / 2 + T * (a[3] / 3 + T * a[4] / 4))) + a[6])
+
+
+def temperature_range(flat) -> tuple:
+    """Widest range of temperatures around 1000 K in which every exponential of
+    the generated right-hand side, and every product of species exponentials,
+    stays within EXP_LIMIT; outside it the table form is used."""
+    a = flat.arrays
+    nu, sp = a["nu"], a["sp"]
+
+    def fine(T):
+        g = _nasa_g(a["nasa"], T)
+        ok = np.abs(g).max() <= EXP_LIMIT
+        for j in range(flat.n_reactions):
+            for key in ("arr", "arr_lo", "arr_rev"):
+                ok &= abs(a[key][j][0] + a[key][j][1] * np.log(T) - a[key][j][2] / T) <= EXP_LIMIT
+            side = [sum(int(nu[j, s]) * g[sp[j, s]] for s in r if sp[j, s] >= 0) for r in (range(4), range(4, 8))]
+            ok &= max(abs(side[0]), abs(side[1]), abs(side[1] - side[0])) <= EXP_LIMIT
+        return bool(ok)
+
+    lo, hi = 1000.0, 1000.0
+    while lo > 150.0 and fine(lo - 5.0):
+        lo -= 5.0
+    while hi < 8000.0 and fine(hi + 50.0):
+        hi += 50.0
+    return lo, hi
+
+
+def _chain(factors) -> str:
+    """Left-to-right product, each multiply rounded on its own."""
+    out = factors[0]
+    for f in factors[1:]:
+        out = f"__dmul_rn({out}, {f})"
+    return out
+
+
 def generate(flat, name: str) -> str:
+    """The right-hand side of one mechanism, one thread per cell.  Every
+    operation is written with its rounding (fma, __dmul_rn, ...) and in the
+    order of the table-driven warp form (rhs_warp in react_rhs.cu), so that
+    both give the same bits.  sE, sI: exp(g/RT) and exp(-g/RT) of the species,
+    per-thread columns of shared memory (stride ss): they would take the
+    registers that the concentrations and rates need.  Exponentials are
+    evaluated four at a time, in the order the reactions need them."""
     a = flat.arrays
     N, R = flat.n_species, flat.n_reactions
     mw = a["mw"]
     nasa = a["nasa"]  # [N][15]
-    out = []
-    w = out.append
-    w(f"// mechanism {name}: {N} species, {R} reactions")
-    w(f"constexpr unsigned long long kGenDigest_{name} = {mechanism_digest(flat)}ull;")
-    w(f"__device__ __forceinline__ void gen_rhs_{name}(const double* __restrict__ y, "
-      f"const double* __restrict__ F, double* __restrict__ out) {{")
-    w(f"  const double T = y[{N}];")
-    w("  const double lnT = log(T), invT = 1.0 / T;")
-    w("  const double lnPRT = log(kPatm / (kRu * T));")
-    w("  const bool lo = T < " + _d(nasa[0, 0]) + ";")
     if not np.all(nasa[:, 0] == nasa[0, 0]):
         raise ValueError("generated right-hand side needs one common NASA-7 midpoint temperature")
-    w(f"  double C[{N}], g[{N}], wd[{N}];")
+    tlo, thi = temperature_range(flat)
+    out, consts = [], {}
+    w = out.append
+
+    def _d(v):
+        """A coefficient: an entry of the mechanism's constant-memory array, which
+        the FP64 instructions take as an operand (a literal takes two moves)."""
+        v = float(v)
+        if v in (0.0, 1.0, -1.0, 2.0, -2.0):
+            return repr(v)
+        return f"kc_{name}[{consts.setdefault(v, len(consts))}]"
+
+    head = [f"// mechanism {name}: {N} species, {R} reactions",
+            f"constexpr unsigned long long kGenDigest_{name} = {mechanism_digest(flat)}ull;",
+            f"constexpr double kGenTlo_{name} = {tlo!r}, kGenThi_{name} = {thi!r};", "#ifdef B200_GEN_FUNCTIONS"]
+    w(f"__device__ __forceinline__ void gen_rhs_{name}(const double* __restrict__ y, "
+      f"const double* __restrict__ F, double* __restrict__ out, double* __restrict__ sE, double* __restrict__ sI, "
+      f"int ss) {{")
+    w(f"  const double T = y[{N}];")
+    w("  const double lnT = log(T), invT = 1.0 / T;")
+    w("  const double u = __dmul_rn(T, kRu / kPatm), iu = 1.0 / u;")
+    w("  const double oml = 1.0 - lnT;")
+    w(f"  const bool lo = T < {float(nasa[0, 0])!r};")
+    w(f"  double C[{N}], wd[{N}];")
     w("  double Ctot = 0.0, rcp = 0.0;")
-    for k in range(N):
-        lo = nasa[k, 1:8]
-        hi = nasa[k, 8:15]
-        cs = ", ".join(f"lo ? {_d(lo[i])} : {_d(hi[i])}" for i in range(7))
-        w(f"  {{ const double c[7] = {{{cs}}};")
-        w("    const double cpR = c[0] + T * (c[1] + T * (c[2] + T * (c[3] + T * c[4])));")
-        w("    const double hRT = c[0] + T * (c[1] / 2 + T * (c[2] / 3 + T * (c[3] / 4 + T * c[4] / 5))) + c[5] * invT;")
-        w("    const double sR = c[0] * lnT + T * (c[1] + T * (c[2] / 2 + T * (c[3] / 3 + T * c[4] / 4))) + c[6];")
-        w(f"    g[{k}] = hRT - sR; C[{k}] = y[{k}] * {_d(1.0 / mw[k])}; wd[{k}] = 0.0;")
-        w(f"    Ctot += C[{k}]; rcp += y[{k}] * cpR * {_d(8.31446261815324e7 / mw[k])}; }}")
+    for k0 in range(0, N, 2):
+        ks = range(k0, min(N, k0 + 2))
+        w("  { double x[4] = {0.0, 0.0, 0.0, 0.0};")
+        for b, cond in (("lo", 1), ("hi", 8)):
+            w("    if (lo) {" if b == "lo" else "    } else {")
+            for k in ks:
+                c = nasa[k, cond:cond + 7]
+                cg = [c[0], c[1] / -2.0, c[2] / -6.0, c[3] / -12.0, c[4] / -20.0, c[5], c[6]]
+                w(f"      x[{2 * (k - k0)}] = nasa_g({', '.join(_d(v) for v in cg)}, T, invT, oml);")
+                w(f"      x[{2 * (k - k0) + 1}] = nasa_cp({', '.join(_d(v) for v in c[:5])}, T);")
+        w("    }")
+        for k in ks:
+            i = 2 * (k - k0)
+            w(f"    C[{k}] = __dmul_rn(y[{k}], {_d(1.0 / mw[k])}); wd[{k}] = 0.0; Ctot = __dadd_rn(Ctot, C[{k}]);")
+            w(f"    rcp = fma(C[{k}], x[{i + 1}], rcp); x[{i + 1}] = -x[{i}];")
+        w("    const Exp4 v = pexp4(x[0], x[1], x[2], x[3]);")
+        for k in ks:
+            i = 2 * (k - k0)
+            w(f"    sE[{k} * ss] = v.x[{i}]; sI[{k} * ss] = v.x[{i + 1}];")
+        w("  }")
     sp, nu = a["sp"], a["nu"]
     effp, effs, effv = a["eff_ptr"], a["eff_sp"], a["eff_val"]
+
+    def arrh(c):
+        t = _d(c[0])
+        if c[1] != 0.0:
+            t = f"fma({_d(c[1])}, lnT, {t})"
+        if c[2] != 0.0:
+            t = f"fma({_d(-c[2])}, invT, {t})"
+        return t
+
+    # arguments of every exponential in reaction order
+    args, where, last = [], {}, {}
     for j in range(R):
         typ, fl = int(a["rtype"][j]), int(a["rflags"][j])
-        lnA, b, ea = a["arr"][j]
-        w(f"  {{ // reaction {j}")
-        arg = _d(lnA)
-        if b != 0.0:
-            arg += f" + {_d(b)} * lnT"
-        if ea != 0.0:
-            arg += f" - {_d(ea)} * invT"
-        w(f"    double kf = gexp({arg});")
+        where[j] = len(args)
+        args.append(arrh(a["arr"][j]))
+        if typ >= 2:
+            args.append(arrh(a["arr_lo"][j]))
+        if typ == 3:
+            _, t3, t1, t2 = a["troe"][j]
+            args += [f"fexp_arg(__dmul_rn(-T, {_d(1.0 / t3)}))", f"fexp_arg(__dmul_rn(-T, {_d(1.0 / t1)}))"]
+            if fl & 4:
+                args.append(f"fexp_arg(__dmul_rn({_d(-t2)}, invT))")
+        if fl & 2:
+            where[(j, "rev")] = len(args)
+            args.append(arrh(a["arr_rev"][j]))
+        last[j] = len(args)
+    done = 0
+
+    def x(i):
+        return f"x{i // 4}.x[{i % 4}]"
+
+    for j in range(R):
+        while done < last[j]:
+            four = (args[done:done + 4] + ["0.0"] * 4)[:4]
+            w(f"  const Exp4 x{done // 4} = pexp4({', '.join(four)});")
+            done += 4
+        typ, fl = int(a["rtype"][j]), int(a["rflags"][j])
+        i = where[j]
+        w(f"    {{ // reaction {j}")
         if typ != 0:
-            terms = "Ctot"
+            m = "Ctot"
             for q in range(effp[j], effp[j + 1]):
                 e = effv[q] - 1.0
                 if e != 0.0:
-                    terms += f" + {_d(e)} * C[{int(effs[q])}]"
-            w(f"    const double M = {terms};")
-        if typ >= 2:
-            l0, b0, e0 = a["arr_lo"][j]
-            arg0 = _d(l0)
-            if b0 != 0.0:
-                arg0 += f" + {_d(b0)} * lnT"
-            if e0 != 0.0:
-                arg0 += f" - {_d(e0)} * invT"
-            w(f"    const double k0 = gexp({arg0});")
-            w("    const double Pr = k0 * M / kf;")
-            if typ == 3:
-                ta, t3, t1, t2 = a["troe"][j]
-                fc = f"(1.0 - {_d(ta)}) * gexp(-T / {_d(t3)}) + {_d(ta)} * gexp(-T / {_d(t1)})"
-                if fl & 4:
-                    fc += f" + gexp(-{_d(t2)} * invT)"
-                w(f"    const double Fc = {fc};")
-                w("    const double logFc = log10(fmax(Fc, 1e-300));")
-                w("    const double cc = -0.4 - 0.67 * logFc, nn = 0.75 - 1.27 * logFc;")
-                w("    const double u = log10(fmax(Pr, 1e-300)) + cc;")
-                w("    const double f1 = u / (nn - 0.14 * u);")
-                w(f"    const double Fb = gexp({_d(np.log(10.0))} * (logFc / (1.0 + f1 * f1)));")
-                w("    kf = kf * Pr / (1.0 + Pr) * Fb;")
-            else:
-                w("    kf = kf * Pr / (1.0 + Pr);")
-        pf, pr, sg = [], [], []
-        sd = 0
-        for s in range(8):
-            k = int(sp[j, s])
-            if k < 0:
-                continue
-            v = int(nu[j, s])
-            sgn = -1 if s < 4 else 1
-            sd += sgn * v
-            (pf if s < 4 else pr).extend([f"C[{k}]"] * v)
-            sg.append(f"{'-' if sgn < 0 else '+'} {v}.0 * g[{k}]" if v != 1 else f"{'-' if sgn < 0 else '+'} g[{k}]")
-        pfs = " * ".join(pf) if pf else "1.0"
-        prs = " * ".join(pr) if pr else "1.0"
-        if fl & 2:
-            lr, br, er = a["arr_rev"][j]
-            argr = _d(lr)
-            if br != 0.0:
-                argr += f" + {_d(br)} * lnT"
-            if er != 0.0:
-                argr += f" - {_d(er)} * invT"
-            w(f"    const double kr = gexp({argr});")
-        elif fl & 1:
-            sgs = " ".join(sg).lstrip("+ ")
-            w(f"    const double kr = kf * gexp({sgs} - {_d(float(sd))} * lnPRT);")
+                    m = f"fma({_d(e)}, C[{int(effs[q])}], {m})"
+            w(f"      const double M = {m};")
+        if typ == 2:
+            w(f"      const double kf = lindemann({x(i)}, {x(i + 1)}, M);")
+        elif typ == 3:
+            al = float(a["troe"][j][0])
+            fc = f"fma({_d(1.0 - al)}, {x(i + 2)}, __dmul_rn({_d(al)}, {x(i + 3)}))"
+            if fl & 4:
+                fc = f"__dadd_rn({fc}, {x(i + 4)})"
+            w(f"      const double kf = troe({x(i)}, {x(i + 1)}, M, {fc});")
         else:
-            w("    const double kr = 0.0;")
-        w(f"    double q = kf * ({pfs}) - kr * ({prs});")
+            w(f"      const double kf = {x(i)};")
+        sides = [[int(sp[j, s]) for s in r if sp[j, s] >= 0 for _ in range(int(nu[j, s]))]
+                 for r in (range(4), range(4, 8))]
+        prods = [_chain([f"C[{k}]" for k in sd]) if sd else "1.0" for sd in sides]
+        if fl & 2:
+            w(f"      double q = __dsub_rn(__dmul_rn(kf, {prods[0]}), __dmul_rn({x(where[(j, 'rev')])}, {prods[1]}));")
+        elif fl & 1:
+            sdn = len(sides[1]) - len(sides[0])
+            fac = [f"sE[{k} * ss]" for k in sides[1]] + [f"sI[{k} * ss]" for k in sides[0]]
+            fac += ["u"] * sdn if sdn > 0 else ["iu"] * -sdn
+            w(f"      double q = __dmul_rn(kf, fma(-{_chain(fac)}, {prods[1]}, {prods[0]}));")
+        else:
+            w(f"      double q = __dmul_rn(kf, {prods[0]});")
         if typ == 1:
-            w("    q *= M;")
-        for s in range(8):
-            k = int(sp[j, s])
-            if k < 0:
-                continue
-            v = int(nu[j, s])
-            op = "-=" if s < 4 else "+="
-            w(f"    wd[{k}] {op} {'' if v == 1 else f'{v}.0 * '}q;")
-        w("  }")
+            w("      q = __dmul_rn(q, M);")
+        net = {}
+        for sgn, sd in zip((-1, 1), sides):
+            for k in sd:
+                net[k] = net.get(k, 0) + sgn
+        for k, v in sorted(net.items()):
+            if v:
+                w(f"      wd[{k}] = fma({_d(v)}, q, wd[{k}]);")
+        w("    }")
     w("  double hs = 0.0;")
     for k in range(N):
-        lo = nasa[k, 1:8]
-        hi = nasa[k, 8:15]
-        cs = ", ".join(f"lo ? {_d(lo[i])} : {_d(hi[i])}" for i in range(6))
-        w(f"  {{ const double c[6] = {{{cs}}};")
-        w("    const double hRT = c[0] + T * (c[1] / 2 + T * (c[2] / 3 + T * (c[3] / 4 + T * c[4] / 5))) + c[5] * invT;")
-        w(f"    const double yd = wd[{k}] * {_d(mw[k])} + F[{k}];")
-        w(f"    out[{k}] = yd; hs += hRT * {_d(8.31446261815324e7 / mw[k])} * T * yd; }}")
-    w(f"  out[{N}] = (F[{N}] - hs) / rcp;")
+        w("  { double hRT;")
+        for b, cond in (("lo", 1), ("hi", 8)):
+            c = nasa[k, cond:cond + 7]
+            ch = [c[0], c[1] / 2.0, c[2] / 3.0, c[3] / 4.0, c[4] / 5.0, c[5]]
+            w(f"    {'if (lo)' if b == 'lo' else 'else'} hRT = nasa_h({', '.join(_d(v) for v in ch)}, T, invT);")
+        w(f"    const double yd = fma(wd[{k}], {_d(mw[k])}, F[{k}]);")
+        w(f"    out[{k}] = yd; hs = fma(__dmul_rn(hRT, {_d(KRU / mw[k])}), yd, hs); }}")
+    w(f"  out[{N}] = fma(-T, hs, F[{N}]) / __dmul_rn(kRu, rcp);")
     w("}")
-    return "\n".join(out) + "\n"
+    w("#endif")
+    vals = [repr(v) for v in consts]
+    head.append(f"static __constant__ double kc_{name}[{len(vals)}] = {{")
+    head += ["  " + ", ".join(vals[i:i + 6]) + "," for i in range(0, len(vals), 6)] + ["};"]
+    return "\n".join(head + out) + "\n"
 
 
 def generate_bundled() -> str:
-    """Header with the generated right-hand sides of the bundled mechanisms."""
+    """Header with the generated right-hand sides of the bundled mechanisms: their
+    digests and temperature ranges, and the functions where B200_GEN_FUNCTIONS is
+    defined."""
     from . import mechanism as mechmod
     parts = ["// gen_mechs.cuh -- generated by pelelmex_b200.mechgen; do not edit.",
-             "#pragma once", "// included after mech_dev.cuh (kPatm, kRu)", "namespace b200 {", "namespace gen {",
-             "// out-of-line FP64 exp: one copy of the code for every call site",
-             "__device__ __noinline__ double gexp(double x) { return exp(x); }"]
+             "#pragma once", "#include \"rate_math.cuh\"", "namespace b200 {", "namespace gen {"]
     for name in ("synth_h2_9", "synth_ch4_21", "synth_c12_53"):
         flat = mechmod.flatten(mechmod.builtin(name))
         parts.append(generate(flat, name))

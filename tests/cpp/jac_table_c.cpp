@@ -9,7 +9,7 @@ extern "C" int jac_table_apply(int N, int R, const int* rtype, const int* sp, co
   if (!b200::build_jac_table(N, R, rtype, sp, nu, eff_ptr, eff_sp, eff_m1, ld, 12, &T)) return 1;
   *nd = T.nd;
   if (!D) return 0;
-  memset(out, 0, sizeof(double) * ((N + 1) * ld + N));
+  memset(out, 0, sizeof(double) * ((N + 1) * ld + 2 * N));
   for (int s = 0; s < T.slices; ++s)
     for (int l = 0; l < 32; ++l) {
       double v = 0.0;

@@ -40,9 +40,9 @@ def test_entries_are_the_written_out_sums(lib, name):
     args = (N, R, _ip(rtype), _ip(sp), _ip(nu), _ip(eptr), _ip(esp), _ip(em1), ld)
     assert lib.jac_table_apply(*args, None, ctypes.byref(nd), None) == 0
     D = np.random.default_rng(3).normal(size=nd.value)
-    out = np.empty((N + 1) * ld + N)
+    out = np.empty((N + 1) * ld + 2 * N)
     assert lib.jac_table_apply(*args, _ip(D), ctypes.byref(nd), _ip(out)) == 0
-    ref, u, p = np.zeros((N + 1, N)), np.zeros(N), 0
+    ref, u, w, p = np.zeros((N + 1, N)), np.zeros(N), np.zeros(N), 0
     for j in range(R):
         slots = [s for s in range(8) if sp[s, j] >= 0]
         net = np.zeros(N)
@@ -52,7 +52,8 @@ def test_entries_are_the_written_out_sums(lib, name):
             ref[sp[s, j]] += net * D[p]
             p += 1
         ref[N] += net * D[p]
-        p += 1
+        w += net * D[p + 1]
+        p += 2
         if rtype[j]:
             u += net * D[p]
             for q in range(eptr[j], eptr[j + 1]):
@@ -61,4 +62,4 @@ def test_entries_are_the_written_out_sums(lib, name):
     assert p == nd.value
     got = out[:(N + 1) * ld].reshape(N + 1, ld)[:, :N]
     # sums of at most a few hundred terms of order one, in another order
-    assert np.abs(got - ref).max() < 1e-12 and np.abs(out[(N + 1) * ld:] - u).max() < 1e-12
+    assert np.abs(got - ref).max() < 1e-12 and np.abs(out[(N + 1) * ld:] - np.concatenate([u, w])).max() < 1e-12
