@@ -443,15 +443,15 @@ cudaEvent_t prof_event(b200chem_reactor* h) {
 // bracketed by two events and the count of the list it processes is copied
 // to the host first (stream-ordered, so it is the count the kernel sees).
 int launch_kernel(b200chem_reactor* h, int lut, int what, int prof_kind, const RoundsParams& R, const RoundsGrids& G,
-                  int setup_pass, const int* cnt, long long host_cells, cudaStream_t st) {
+                  int pass, const int* cnt, long long host_cells, cudaStream_t st) {
   if (!h->prof_on || h->prof_overflow) {
-    CK(rounds_launch(h->N, lut, what, R, G, setup_pass, st));
+    CK(rounds_launch(h->N, lut, what, R, G, pass, st));
     return 0;
   }
   b200chem_reactor::ProfRec rec{prof_kind, -1, host_cells, prof_event(h), prof_event(h)};
   if (!rec.e0 || !rec.e1 || (cnt && h->pcnt_used >= kProfCountSlots)) {
     h->prof_overflow = true;
-    CK(rounds_launch(h->N, lut, what, R, G, setup_pass, st));
+    CK(rounds_launch(h->N, lut, what, R, G, pass, st));
     return 0;
   }
   if (cnt) {
@@ -459,7 +459,7 @@ int launch_kernel(b200chem_reactor* h, int lut, int what, int prof_kind, const R
     CK(cudaMemcpyAsync(h->h_pcnt + rec.slot, cnt, sizeof(int), cudaMemcpyDeviceToHost, st));
   }
   CK(cudaEventRecord(rec.e0, st));
-  CK(rounds_launch(h->N, lut, what, R, G, setup_pass, st));
+  CK(rounds_launch(h->N, lut, what, R, G, pass, st));
   CK(cudaEventRecord(rec.e1, st));
   h->prof.push_back(rec);
   return 0;
@@ -477,39 +477,44 @@ struct RoundLists {
 // Newton correction and step of those that keep their Newton matrix; Jacobian
 // and inverse of the others, then their step; the control kernel for whatever
 // the step kernel passed on.  Every kernel appends to the lists of the next
-// round, whose counters the right-hand-side kernel clears.  side (may be st):
-// the Jacobian and the inverse need nothing of this round's other kernels and
-// share no data with them before the step of their cells, so in the captured
-// graph they run on a branch of their own: a round of few cells is a chain of
-// kernels of 5 to 20 us each, and this takes two of the six off it.
+// round, whose counters the right-hand-side kernel clears.
+// side (when not st): the Jacobian and the inverse need nothing of this round's
+// other kernels, so in the captured graph of few cells they run on a branch
+// beside the right-hand sides.  Such a round is a chain of kernels of 5 to 50 us,
+// whatever they process.  Up to 32 components the branch is as short as the
+// right-hand sides, and one launch of the step kernel takes all cells behind
+// both (an 8^3 H2 box: 2.40 ms, 2.79 with two launches, 3.0 without the branch);
+// with 54 it is longer, and the cells that keep their matrix go ahead (dodecane
+// 20^3: 180 ms, 192 with one launch, 266 without the branch).
 int enqueue_round(b200chem_reactor* h, int lut, RoundsParams R, const RoundsGrids& G, const RoundLists& Ls, int cur,
                   cudaStream_t st, cudaStream_t side) {
   const int* cnt = Ls.cnt[cur];
   R.cnt_next = Ls.cnt[1 - cur];
   for (int k = 0; k < kRoundLists; ++k) R.list[k] = Ls.lst[1 - cur][k];
-  const struct { int what, kind, setup_pass, in; const int* c; const int* list; } seq[6] = {
-      {kRoundsRhs, B200CHEM_PROF_RHS, 0, kRlRhs, cnt, Ls.lst[cur][kRlRhs]},
-      {kRoundsStep, B200CHEM_PROF_CTRL, 0, kRlRhs, cnt, Ls.lst[cur][kRlRhs]},
-      {kRoundsJac, B200CHEM_PROF_JAC, 0, kRlJac, cnt, Ls.lst[cur][kRlJac]},
-      {kRoundsGj, B200CHEM_PROF_GJ, 0, kRlSetup, cnt, Ls.lst[cur][kRlSetup]},
-      {kRoundsStep, B200CHEM_PROF_CTRL_SETUP, 1, kRlSetup, cnt, Ls.lst[cur][kRlSetup]},
-      {kRoundsCtrl, B200CHEM_PROF_CTRL_RARE, 0, kRlCtrl, R.cnt_next, Ls.lst[1 - cur][kRlCtrl]}};
-  if (side != st) {
+  auto launch = [&](int what, int kind, int pass, int in, const int* c, const int* list, cudaStream_t s) {
+    R.list_in = list;
+    R.cnt_in = c + in;
+    return launch_kernel(h, lut, what, kind, R, G, pass, R.cnt_in, 0, s);
+  };
+  int* const* lst = Ls.lst[cur];
+  const bool fork = side != st, one_step = fork && h->n <= 32;
+  int err = 0;
+  if (fork) {
     CK(cudaEventRecord(h->cap_ev[0], st));
     CK(cudaStreamWaitEvent(side, h->cap_ev[0], 0));
   }
-  for (const auto& k : seq) {
-    R.list_in = k.list;
-    R.cnt_in = k.c + k.in;
-    const bool setup = k.what == kRoundsJac || k.what == kRoundsGj;
-    if (side != st && k.setup_pass) {
-      CK(cudaEventRecord(h->cap_ev[1], side));
-      CK(cudaStreamWaitEvent(st, h->cap_ev[1], 0));
-    }
-    const int err = launch_kernel(h, lut, k.what, k.kind, R, G, k.setup_pass, R.cnt_in, 0, setup ? side : st);
-    if (err) return err;
+  if ((err = launch(kRoundsRhs, B200CHEM_PROF_RHS, 0, kRlRhs, cnt, lst[kRlRhs], st))) return err;
+  if (!one_step && (err = launch(kRoundsStep, B200CHEM_PROF_CTRL, kStepKept, kRlRhs, cnt, lst[kRlRhs], st))) return err;
+  if ((err = launch(kRoundsJac, B200CHEM_PROF_JAC, 0, kRlJac, cnt, lst[kRlJac], side))) return err;
+  if ((err = launch(kRoundsGj, B200CHEM_PROF_GJ, 0, kRlSetup, cnt, lst[kRlSetup], side))) return err;
+  if (fork) {
+    CK(cudaEventRecord(h->cap_ev[1], side));
+    CK(cudaStreamWaitEvent(st, h->cap_ev[1], 0));
   }
-  return 0;
+  err = one_step ? launch(kRoundsStep, B200CHEM_PROF_CTRL, kStepAll, kRlRhs, cnt, lst[kRlRhs], st)
+                 : launch(kRoundsStep, B200CHEM_PROF_CTRL_SETUP, kStepSetup, kRlSetup, cnt, lst[kRlSetup], st);
+  if (err) return err;
+  return launch(kRoundsCtrl, B200CHEM_PROF_CTRL_RARE, 0, kRlCtrl, R.cnt_next, Ls.lst[1 - cur][kRlCtrl], st);
 }
 
 // Captures `rounds` rounds (an even number: the two sets of lists swap roles
@@ -661,7 +666,7 @@ int launch_rounds(b200chem_reactor* h, const ReactParams& P, cudaStream_t st, in
           if (err) return err;
         }
       }
-      h->launches += 6LL * per_check;
+      h->launches += (graph && cls > 0 && h->n <= 32 ? 5LL : 6LL) * per_check;
       // per_check is even: the live cells are back in the first list
       CK(cudaMemcpyAsync(h->h_rcnt, Ls.cnt[0] + kRlRhs, sizeof(int), cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));

@@ -162,6 +162,7 @@ struct RoundsSetupLayout {
 // Jacobian is recomputed, and the cells the control kernel takes this round.
 enum { kRlRhs = 0, kRlSetup, kRlJac, kRlCtrl, kRoundLists };
 constexpr int kSetupFlag = 1 << 30;
+enum { kStepKept = 0, kStepSetup, kStepAll };  // which cells a launch of the step kernel takes
 // slot lists of a chunk: the first three of the above twice (read and written
 // in turn) and the control kernel's
 constexpr int kRoundSlotLists = 2 * kRlCtrl + 1;
@@ -220,7 +221,7 @@ long long rounds_state_bytes_per_cell(int N, int lut_bytes);
 rounds::RState rounds_carve(void* base, long long cap, int N, int lut_bytes);
 cudaError_t rounds_grids_for(int N, int R, int gen, int lut_bytes, const RoundsSetupLayout& SL, int sm_count,
                              RoundsGrids* G);
-cudaError_t rounds_launch(int N, int lut_bytes, int what, const RoundsParams& R, const RoundsGrids& G, int setup_pass,
+cudaError_t rounds_launch(int N, int lut_bytes, int what, const RoundsParams& R, const RoundsGrids& G, int pass,
                           cudaStream_t st);
 
 // ------------------------------------------- packed constant-memory table

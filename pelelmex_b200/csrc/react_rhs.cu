@@ -177,22 +177,39 @@ __device__ __forceinline__ void rhs_warp(const DevMech& m, const View& v, double
   }
   __syncwarp();
   double Ctot = 0.0, rcp = 0.0;
+#pragma unroll 9
   for (int k = 0; k < NS; ++k) {
     Ctot = __dadd_rn(Ctot, sC[k]);
     rcp = fma(sC[k], sP[k], rcp);
   }
   for (int j = lane; j < R; j += 32) {
+    // a reaction's table entries all at once: one memory latency, not one per slot
     const int type = __ldg(m.rtype + j), flags = __ldg(m.rflags + j);
+    int sp[8], nu[8];
+#pragma unroll
+    for (int sl = 0; sl < 8; ++sl) {
+      sp[sl] = __ldg(m.sp + sl * R + j);
+      nu[sl] = __ldg(m.nu + sl * R + j);
+    }
     auto arrh = [&](const double* p) {
       return fma(-__ldg(p + 2 * R + j), invT, fma(__ldg(p + R + j), lnT, __ldg(p + j)));
     };
     double kf[1] = {arrh(m.arr)};
+    const int e0 = __ldg(m.eff_ptr + j), e1 = __ldg(m.eff_ptr + j + 1);
     pexp(kf);
     double M = 0.0;
     if (type != 0) {
       M = Ctot;
-      const int e0 = __ldg(m.eff_ptr + j), e1 = __ldg(m.eff_ptr + j + 1);
-      for (int q = e0; q < e1; ++q) M = fma(__ldg(m.eff_m1 + q), sC[__ldg(m.eff_sp + q)], M);
+      for (int q = e0; q < e1; q += 4) {
+        double em[4], c[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          em[t] = q + t < e1 ? __ldg(m.eff_m1 + q + t) : 0.0;
+          c[t] = q + t < e1 ? sC[__ldg(m.eff_sp + q + t)] : 0.0;
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) M = fma(em[t], c[t], M);  // a padded term adds nothing
+      }
     }
     if (type >= 2) {
       double k0[1] = {arrh(m.arr_lo)};
@@ -213,21 +230,21 @@ __device__ __forceinline__ void rhs_warp(const DevMech& m, const View& v, double
     double pf = 1.0, pr = 1.0, fac = 1.0;
 #pragma unroll
     for (int sl = 4; sl < 8; ++sl) {
-      const int k = __ldg(m.sp + sl * R + j);
-      if (k >= 0)
-        for (int e = __ldg(m.nu + sl * R + j); e > 0; --e) {
-          pr = __dmul_rn(pr, sC[k]);
-          fac = __dmul_rn(fac, sE[k]);
-        }
+      if (sp[sl] < 0) continue;
+      const double c = sC[sp[sl]], x = sE[sp[sl]];
+      for (int e = nu[sl]; e > 0; --e) {
+        pr = __dmul_rn(pr, c);
+        fac = __dmul_rn(fac, x);
+      }
     }
 #pragma unroll
     for (int sl = 0; sl < 4; ++sl) {
-      const int k = __ldg(m.sp + sl * R + j);
-      if (k >= 0)
-        for (int e = -__ldg(m.nu + sl * R + j); e > 0; --e) {
-          pf = __dmul_rn(pf, sC[k]);
-          fac = __dmul_rn(fac, sI[k]);
-        }
+      if (sp[sl] < 0) continue;
+      const double c = sC[sp[sl]], x = sI[sp[sl]];
+      for (int e = -nu[sl]; e > 0; --e) {
+        pf = __dmul_rn(pf, c);
+        fac = __dmul_rn(fac, x);
+      }
     }
     double q;
     if (flags & 2) {
@@ -249,13 +266,23 @@ __device__ __forceinline__ void rhs_warp(const DevMech& m, const View& v, double
   for (int k = lane; k < NS; k += 32) {
     double w = 0.0;
     const int p0 = __ldg(m.inc_ptr + k), p1 = __ldg(m.inc_ptr + k + 1);
-    for (int p = p0; p < p1; ++p) w = fma(__ldg(m.inc_nu + p), sq[__ldg(m.inc_rxn + p)], w);
+    for (int p = p0; p < p1; p += 8) {
+      double a[8], q[8];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        a[t] = p + t < p1 ? __ldg(m.inc_nu + p + t) : 0.0;
+        q[t] = p + t < p1 ? sq[__ldg(m.inc_rxn + p + t)] : 0.0;
+      }
+#pragma unroll
+      for (int t = 0; t < 8; ++t) w = fma(a[t], q[t], w);
+    }
     const double yd = fma(w, __ldg(m.mw + k), v.F(k));
     v.set_f(k, yd);
     sP[k] = yd;
   }
   __syncwarp();
   double hs = 0.0;
+#pragma unroll 9
   for (int k = 0; k < NS; ++k) hs = fma(sH[k], sP[k], hs);
   if (lane == 0) v.set_f(NS, fma(-T, hs, v.F(NS)) / __dmul_rn(kRu, rcp));
   __syncwarp();  // the scratch is free again
@@ -284,9 +311,11 @@ __global__ void __launch_bounds__(kRoundsRhsBlock, 6) rk_rhs(RoundsParams R) {
   }
 }
 
-// Generated right-hand sides for few live cells, one warp per cell.  A thread takes 60 us and
-// more for a cell however few there are, mostly waiting for its 100 KB of code;
-// the warp form is a few loops over the tables.
+// Generated right-hand sides for few live cells, one warp per cell.  A thread
+// takes 60 us (21 species) to 200 us (53) for a cell however few there are, mostly
+// waiting for its code; the warp form, a few loops over the tables, 15 to 43.  It
+// is bound by the latency of the table reads, so a reaction's entries are read
+// together (53 species: 57 us a launch with one read after the other).
 constexpr int kRhsWarpBlock = 128;
 template <int NS>
 __global__ void __launch_bounds__(kRhsWarpBlock, 8) rk_rhs_warp(RoundsParams R) {
@@ -376,9 +405,10 @@ int rhs_warp_smem(int R) { return kRhsWarpBlock / 32 * rhs_warp_doubles<NS>(R) *
 
 // Most cells for which the warp form is used, in cells per warp of a grid that
 // fills the GPU (4736 warps).  2 for the smaller mechanisms: 32^3 H2 spends
-// 1.35 ms in right-hand sides with it, 1.64 with 4 and 3.6 with 8.  8 for 53
-// species, whose thread form spills: six boxes of 571,824 cells take 20 ms with
-// 8 or 16 (26 with one that used the thread form from 3500 cells on).
+// 1.37 ms in right-hand sides with it, 1.64 with 4 and 3.6 with 8; 61x43x37 CH4
+// 12.7 and 12.9 ms with 2 and 4.  8 for 53 species, whose thread form spills: six
+// boxes of 571,824 cells take 18 ms (26 with one that took the thread form from
+// 3500 cells on).
 constexpr int rhs_warp_waves(int NS) { return NS <= 32 ? 2 : 8; }
 
 template <int NS>

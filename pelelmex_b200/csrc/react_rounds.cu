@@ -326,11 +326,12 @@ __device__ __forceinline__ void step_cell(const RoundsParams& R, bool live, int 
   warp_append_lists(gl == 0 ? which : 0, slot, rhs_val, R);
 }
 
-// Newton correction and step of the cells of list_in, G lanes per cell.
-// setup_pass: the cells whose Newton matrix this round's setup kernels
-// rebuilt; otherwise the others (those entries, flagged, are passed over).
+// Newton correction and step of the cells of list_in, G lanes per cell.  pass
+// kStepKept: the cells that keep their Newton matrix (the flagged entries of the
+// others are passed over); kStepSetup: a list of those this round's setup
+// kernels rebuilt it for; kStepAll: both kinds from the first list.
 template <int NS, typename LUT>
-__global__ void __launch_bounds__(128, step_min_ctas(NS + 1)) rk_step(RoundsParams R, int setup_pass) {
+__global__ void __launch_bounds__(128, step_min_ctas(NS + 1)) rk_step(RoundsParams R, int pass) {
   constexpr int n = NS + 1;
   constexpr int G = ctrl_group(n);
   constexpr int GPW = 32 / G;  // cells per warp
@@ -343,8 +344,9 @@ __global__ void __launch_bounds__(128, step_min_ctas(NS + 1)) rk_step(RoundsPara
   const int nw = (gridDim.x * blockDim.x) >> 5;
   for (int base = wid * GPW; base < cnt; base += nw * GPW) {
     const int idx = base + gi;
-    const int entry = idx < cnt ? R.list_in[idx] : kSetupFlag;
-    step_cell<NS, G, LUT>(R, !(entry & kSetupFlag), entry & ~kSetupFlag, sm, gl, gm);
+    const int entry = idx < cnt ? R.list_in[idx] : 0;
+    const bool live = idx < cnt && (pass != kStepKept || !(entry & kSetupFlag));
+    step_cell<NS, G, LUT>(R, live, entry & ~kSetupFlag, sm, gl, gm);
   }
 }
 
@@ -882,7 +884,7 @@ __device__ __forceinline__ void team_jac(const DevMech& m, const GrpScratch& s, 
   for (int sl = tid >> 5; sl < m.jt_slices; sl += W) {
     const int t0 = __ldg(m.jt_off + sl), t1 = __ldg(m.jt_off + sl + 1);
     double v = 0.0;
-#pragma unroll 4
+#pragma unroll 8
     for (int t = t0; t < t1; ++t) {
       const unsigned term = __ldg(m.jt_term + t * 32 + lane);
       v += __ldg(m.jt_coef + (term & (kJtCoefs - 1))) * D[term >> kJtCoefBits];
@@ -1151,7 +1153,7 @@ cudaError_t rounds_grids(int R, int gen, const RoundsSetupLayout& SL, int sm_cou
 }
 
 template <int NS, typename LUT>
-cudaError_t rounds_launch_t(int what, const RoundsParams& R, const RoundsGrids& G, int setup_pass, cudaStream_t st) {
+cudaError_t rounds_launch_t(int what, const RoundsParams& R, const RoundsGrids& G, int pass, cudaStream_t st) {
   constexpr int n = NS + 1;
   switch (what) {
     case kRoundsStart:
@@ -1160,7 +1162,7 @@ cudaError_t rounds_launch_t(int what, const RoundsParams& R, const RoundsGrids& 
     case kRoundsRhs:
       return rhs_launch(NS, R, G.rhs_by_warp ? G.rhs.warp : G.rhs.thread, G.rhs_by_warp, st);
     case kRoundsStep:
-      rk_step<NS, LUT><<<G.step, 128, step_smem<n>(), st>>>(R, setup_pass);
+      rk_step<NS, LUT><<<G.step, 128, step_smem<n>(), st>>>(R, pass);
       break;
     case kRoundsCtrl:
       rk_ctrl<NS><<<G.ctrl, 128, 0, st>>>(R);
@@ -1226,17 +1228,17 @@ cudaError_t rounds_grids_for(int N, int R, int gen, int lut_bytes, const RoundsS
   return cudaErrorInvalidValue;
 }
 
-cudaError_t rounds_launch(int N, int lut_bytes, int what, const RoundsParams& R, const RoundsGrids& G, int setup_pass,
+cudaError_t rounds_launch(int N, int lut_bytes, int what, const RoundsParams& R, const RoundsGrids& G, int pass,
                           cudaStream_t st) {
   if (N == 9)
-    return lut_bytes == 4 ? rounds_launch_t<9, float>(what, R, G, setup_pass, st)
-                          : rounds_launch_t<9, double>(what, R, G, setup_pass, st);
+    return lut_bytes == 4 ? rounds_launch_t<9, float>(what, R, G, pass, st)
+                          : rounds_launch_t<9, double>(what, R, G, pass, st);
   if (N == 21)
-    return lut_bytes == 4 ? rounds_launch_t<21, float>(what, R, G, setup_pass, st)
-                          : rounds_launch_t<21, double>(what, R, G, setup_pass, st);
+    return lut_bytes == 4 ? rounds_launch_t<21, float>(what, R, G, pass, st)
+                          : rounds_launch_t<21, double>(what, R, G, pass, st);
   if (N == 53)
-    return lut_bytes == 4 ? rounds_launch_t<53, float>(what, R, G, setup_pass, st)
-                          : rounds_launch_t<53, double>(what, R, G, setup_pass, st);
+    return lut_bytes == 4 ? rounds_launch_t<53, float>(what, R, G, pass, st)
+                          : rounds_launch_t<53, double>(what, R, G, pass, st);
   return cudaErrorInvalidValue;
 }
 
