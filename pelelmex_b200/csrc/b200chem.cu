@@ -221,9 +221,14 @@ struct StagedBuf {
   cudaEvent_t ev = nullptr;
 };
 
-// Launch shapes of a round by how many cells are live: many (right-hand sides
-// by thread), few (by warp), and so few that the grids shrink to them.
-constexpr int kRoundClasses = 3;
+// Launch shapes of a round by how many cells are live: many (kernels in a row,
+// right-hand sides by thread), fewer (setup kernels on a branch), few
+// (right-hand sides by warp as well), and so few that the grids shrink to them.
+// The branch pays up to 131072 cells (32^3 H2: 4.56 ms, 5.03 without it above
+// the warp form's 9472 cells; 61x43x37 CH4: 44.3 and 45.8) and costs 10 % with
+// two million, whose kernels contend for L2.
+constexpr int kRoundClasses = 4;
+constexpr int kForkCells = 131072;
 constexpr int kTinyCells = 1024;
 
 struct b200chem_reactor {
@@ -637,14 +642,10 @@ int launch_rounds(b200chem_reactor* h, const ReactParams& P, cudaStream_t st, in
     if (err) return err;
     h->launches++;
     // the launch shape follows the live cells, which only become fewer
-    bool captured[kRoundClasses] = {};
-    long long live = R.nchunk;
-    for (long long round = 0;; round += per_check) {
-      if (round >= max_rounds) return set_err(B200CHEM_EINTEGRATE, "round-based integrator did not finish");
-      const int cls = live <= kTinyCells ? 2 : live <= G.rhs.warp_cells ? 1 : 0;
+    auto shape = [&](int cls) {
       RoundsGrids Gc = G;
-      Gc.rhs_by_warp = R.gen_mech && live <= G.rhs.warp_cells;
-      if (cls == 2) {
+      Gc.rhs_by_warp = R.gen_mech && cls >= 2;
+      if (cls == 3) {
         const int per_cta = 128 / rounds::ctrl_group(h->n);
         const int need = (kTinyCells + per_cta - 1) / per_cta;
         Gc.step = std::min(G.step, need);
@@ -653,22 +654,31 @@ int launch_rounds(b200chem_reactor* h, const ReactParams& P, cudaStream_t st, in
         Gc.rhs.warp = std::min(G.rhs.warp, kTinyCells / 4);
         Gc.rhs.thread = std::min(G.rhs.thread, kTinyCells / kRoundsRhsBlock);
       }
+      return Gc;
+    };
+    bool captured[kRoundClasses] = {};
+    auto capture = [&](int cls) {
+      captured[cls] = true;
+      return capture_rounds(h, lut, R, shape(cls), per_check, Ls, cls);
+    };
+    long long live = R.nchunk;
+    for (long long round = 0;; round += per_check) {
+      if (round >= max_rounds) return set_err(B200CHEM_EINTEGRATE, "round-based integrator did not finish");
+      const int cls = live <= kTinyCells ? 3 : live <= G.rhs.warp_cells ? 2 : live <= kForkCells ? 1 : 0;
       if (graph) {
-        if (!captured[cls]) {
-          err = capture_rounds(h, lut, R, Gc, per_check, Ls, cls);
-          if (err) return err;
-          captured[cls] = true;
-        }
+        if (!captured[cls] && (err = capture(cls))) return err;
         CK(cudaGraphLaunch(h->rgraph[cls], st));
       } else {
         for (int r = 0; r < per_check; ++r) {
-          err = enqueue_round(h, lut, R, Gc, Ls, r & 1, st, st);
+          err = enqueue_round(h, lut, R, shape(cls), Ls, r & 1, st, st);
           if (err) return err;
         }
       }
       h->launches += (graph && cls > 0 && h->n <= 32 ? 5LL : 6LL) * per_check;
       // per_check is even: the live cells are back in the first list
       CK(cudaMemcpyAsync(h->h_rcnt, Ls.cnt[0] + kRlRhs, sizeof(int), cudaMemcpyDeviceToHost, st));
+      // the next class's graph is made while this one runs
+      if (graph && cls + 1 < kRoundClasses && !captured[cls + 1] && (err = capture(cls + 1))) return err;
       CK(cudaStreamSynchronize(st));
       live = *h->h_rcnt;
       if (live == 0) break;

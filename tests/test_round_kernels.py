@@ -24,8 +24,10 @@ def _field(name, n):
 
 
 # the large batch starts with the thread form (more than the 2 x 4736 cells, or
-# 8 x 4736 with 53 species, that take the warp form), the small ones do not
-@pytest.mark.parametrize("name,big", [("synth_h2_9", 60000), ("synth_ch4_21", 60000), ("synth_c12_53", 40000)])
+# 8 x 4736 with 53 species, that take the warp form), the small ones do not;
+# above 131072 cells the kernels of a round run in a row, below on two branches
+@pytest.mark.parametrize("name,big", [("synth_h2_9", 60000), ("synth_ch4_21", 60000), ("synth_c12_53", 40000),
+                                      ("synth_ch4_21", 131073), ("synth_c12_53", 131073)])
 @pytest.mark.parametrize("small", [1, 33, 257])
 def test_result_of_a_cell_is_independent_of_its_batch(name, big, small):
     f = _field(name, big)
