@@ -115,10 +115,11 @@ def kernel_bytes(kind: str, n_species: int, lut_bytes: int = 4) -> float:
     write, each once):
 
     * rhs: list slot, read y and the forcing (2n), write f (n)
-    * ctrl / ctrl_setup (one Newton iteration): the step-control record read
-      and written, read zn[1], acor, ftemp, f, ewt, scaling (6n) and write
+    * ctrl / ctrl_setup (rk_step, one Newton iteration): the step-control
+      record read and written, read zn[1], acor, f, ewt, scaling (5n) and write
       acor (n), read the FP64 Jacobian (n^2) for the refinement residual and
-      the inverse (n^2 at lut_bytes)
+      the inverse (n^2 at lut_bytes); the Nordsieck columns of a completed
+      step are not counted
     * jac (only the setups whose Jacobian is stale reach it): list slot,
       read y and f (2n), write J (n^2)
     * gj: list slot and gamma, read J (n^2) and ewt (n), write the scaling
@@ -128,7 +129,7 @@ def kernel_bytes(kind: str, n_species: int, lut_bytes: int = 4) -> float:
     if kind == "rhs":
         return 4 + 8 * 3 * n
     if kind in ("ctrl", "ctrl_setup"):
-        return 4 + 2 * RCELL_BYTES + 8 * 7 * n + 8 * n * n + lut_bytes * n * n
+        return 4 + 2 * RCELL_BYTES + 8 * 6 * n + 8 * n * n + lut_bytes * n * n
     if kind == "jac":
         return 4 + jac_refresh_bytes(n_species)
     if kind == "gj":
