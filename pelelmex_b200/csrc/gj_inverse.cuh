@@ -115,6 +115,7 @@ __device__ __forceinline__ int reg_gj_inverse(const double* J, const double* dsc
     for (int j = 1; j < n; ++j) a[j - 1] = fma(-gi, pr[j], a[j]);
     a[n - 1] = (lane == p) ? inv : -gi;
   }
+  __syncwarp();  // the pivot-row buffers lie in Xs
   if (row) {
 #pragma unroll
     for (int j = 0; j < n; ++j) Xs[lane * ldl + j] = a[j];
