@@ -755,10 +755,17 @@ __global__ void __launch_bounds__(128, gj_min_ctas<NS + 1, LUT>()) rk_gj(RoundsP
 // ------------------------------------------------------------ host side
 namespace {
 
+// Most shared memory of a Jacobian CTA that keeps two of them on an SM; the
+// teams' parts are rounded up to 16 bytes each.
+constexpr int kJacSmemCta = 100 * 1024, kJacSmemMax = kJacSmemCta + 4 * 16;
+
+// The limit of dynamic shared memory is a property of the function and not of a
+// handle: it is what any mechanism of this species count may need, so that
+// handles of different mechanisms do not take it from one another.
 template <int NS, typename LUT>
 cudaError_t rounds_setup_attrs(const RoundsSetupLayout& SL) {
   constexpr int n = NS + 1;
-  cudaError_t e = cudaFuncSetAttribute(rk_jac<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SL.jac_smem);
+  cudaError_t e = cudaFuncSetAttribute(rk_jac<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, kJacSmemMax);
   if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(rk_step<NS, LUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, step_smem<n>());
   if (e != cudaSuccess) return e;
@@ -829,11 +836,12 @@ RoundsSetupLayout rounds_setup_layout(int N, int lut_bytes, int jac_nd) {
   L.Npad = ((n + 31) / 32) * 32;
   L.ldl = n | 1;
   // scratch of a Jacobian team; the reactions' derivatives move to device
-  // memory where they would leave fewer than two CTAs on an SM
+  // memory where they would leave fewer than two CTAs on an SM (what is left,
+  // 8 to 27 KB a CTA, fits)
   const int teams = 4 / jac_warps(n);
   const long long fixed = 8LL * (4 * L.Npad + n * jac_ld(n) + 2 * N + n), dbytes = 8LL * jac_nd;
   L.jac_nd = jac_nd;
-  L.jac_d_global = teams * (fixed + dbytes) > 100 * 1024;
+  L.jac_d_global = teams * (fixed + dbytes) > kJacSmemCta;
   L.jac_smem_per_team = (int)((fixed + (L.jac_d_global ? 0 : dbytes) + 15) & ~15LL);
   L.jac_smem = teams * L.jac_smem_per_team;
   L.gbytes_per_cta = L.jac_d_global ? teams * dbytes : 0;
