@@ -1,7 +1,8 @@
 """Mechanisms of one species count and different numbers of reactions: reactors of
-two of them used in turn in one process.  The long mechanisms are the bundled ones
-with every reaction written `times` over and its rate divided by that, so their
-solution is the plain one's."""
+two of them used in turn in one process, and one whose reactions' derivatives do
+not fit the Jacobian kernel's shared memory.  The long mechanisms are the bundled
+ones with every reaction written `times` over and its rate divided by that, so
+their solution is the plain one's."""
 import copy
 
 import numpy as np
@@ -12,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 from pelelmex_b200 import mechanism as M, workloads as W  # noqa: E402
 from pelelmex_b200.reactor import ReactorB200  # noqa: E402
-from test_gpu_parity import DEV, T_RTOL, _dev  # noqa: E402
+from test_gpu_parity import DEV, T_RTOL, Y_ATOL, _dev  # noqa: E402
 
 
 def _repeated(name, times):
@@ -55,5 +56,30 @@ def test_reactors_of_two_mechanisms_in_turn(name, times):
     again = _react(a, f)
     assert np.array_equal(first[0], again[0]) and np.array_equal(first[1], again[1])
     assert np.abs(first[1] - plain[1]).max() <= T_RTOL * plain[1].max()
+    a.close()
+    b.close()
+
+# above 100 KB a CTA the derivatives go to device memory
+@pytest.mark.parametrize("name,times", [("synth_h2_9", 28), ("synth_ch4_21", 6), ("synth_c12_53", 8)])
+@pytest.mark.parametrize("lu_fp64", [False, True])
+def test_derivatives_in_device_memory(name, times, lu_fp64):
+    f = _field(name, 300)
+    a, b = _reactor(_repeated(name, times), lu_fp64), _reactor(M.builtin(name), lu_fp64)
+    (y, T, st), (yp, Tp, sp) = _react(a, f), _react(b, f)
+    assert st["n_failed"] == 0 and sp["n_failed"] == 0
+    assert np.abs(T - Tp).max() <= T_RTOL * Tp.min()
+    rho, err = f.rhoY.sum(axis=0), Y_ATOL
+    if name == "synth_c12_53":
+        # step decisions that flip at round-off move a cell by the integrator's own
+        # error, which is that of the plain mechanism against a tight solve
+        c = _reactor(M.builtin(name), True, 1e-12, 1e-20)
+        yt = _react(c, f)[0]
+        c.close()
+        err, yp = 3.0 * (np.abs(yp - yt).max(axis=0) / rho).max() + 1e-9, yt
+    assert (np.abs(y - yp).max(axis=0) / rho).max() <= err
+    # a wrong Jacobian costs Newton iterations first; step decisions that flip at
+    # round-off move the counts of the 53-species field by a few per cent
+    for k in ("nst", "nfe", "nje", "nlu"):
+        assert abs(st[k] - sp[k]) <= (3e-2 if name == "synth_c12_53" else 2e-3) * sp[k] + 2, k
     a.close()
     b.close()
