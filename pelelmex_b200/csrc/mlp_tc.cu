@@ -823,6 +823,15 @@ int make_operand_map(CUtensorMap* map, const void* base, int cols, int rows, lon
   return r == CUDA_SUCCESS ? 0 : -1;
 }
 
+// Sets the limit of a kernel's dynamic shared memory, which belongs to the
+// function, to the most that any call may use: with each call setting its own
+// size, another thread's launch could come between the two and be refused.
+// optin: the device's opt-in maximum, of which 2 KB are left for static arrays.
+template <typename Kernel>
+bool allow_smem(Kernel kernel, int optin) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 2048) == cudaSuccess;
+}
+
 }  // namespace
 
 extern "C" int b200chem_mlp_gemm_bf16(const void* A, long long lda, const void* B, long long ldb, int M, int N, int K,
@@ -865,17 +874,16 @@ extern "C" int b200chem_mlp_gemm_bf16(const void* A, long long lda, const void* 
     g.vec_ok = (cal && aal) ? 1 : 0;
   }
   const bool resident = (K <= 256 && N <= 256);
-  int dev = 0, sms = 0;
+  int dev = 0, sms = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (resident && (K <= 64 || K % 64 == 0)) {
     // warp-specialised pipeline: TMA producer, MMA issuer, epilogue warps
     CUtensorMap ta, tb;
     if (make_operand_map(&ta, A, arep * K, M, lda, kTileM) || make_operand_map(&tb, B, K, N, ldb, N)) return -2;
     const int KC = K <= 64 ? K : 64;
-    int optin = 0;
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const int b_bytes = (N * K * 2 + 1023) & ~1023, stage_bytes = kTileM * KC * 2;
     // as many A stages as fit beside B (2 KB left for the static barriers and bias)
     int stages = (optin - 2048 - b_bytes) / stage_bytes;
@@ -884,8 +892,7 @@ extern "C" int b200chem_mlp_gemm_bf16(const void* A, long long lda, const void* 
     g.stages = stages;
     int smem = b_bytes + stages * stage_bytes;
     if (smem < kWsMinSmem) smem = kWsMinSmem;
-    if (cudaFuncSetAttribute(gemm_bf16_ws, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return -2;
+    if (!allow_smem(gemm_bf16_ws, optin)) return -2;
     const int tiles = M / kTileM;
     const int grid = tiles < sms ? tiles : sms;
     gemm_bf16_ws<<<grid, kWsThreads, smem, st>>>(g, ta, tb);
@@ -898,16 +905,14 @@ extern "C" int b200chem_mlp_gemm_bf16(const void* A, long long lda, const void* 
   if (epi == kEpiF32 && !resident && K % kSplitKC == 0 && K >= 2 * kSplit * kSplitKC &&
       2 * (M / kTileM) * ((N + 255) / 256) < sms) {
     const int nt = split_nt(N), ssm = split_smem(nt);
-    if (cudaFuncSetAttribute(gemm_bf16_splitk, cudaFuncAttributeMaxDynamicSharedMemorySize, ssm) != cudaSuccess)
-      return -2;
+    if (!allow_smem(gemm_bf16_splitk, optin)) return -2;
     gemm_bf16_splitk<<<(M / kTileM) * (N / nt) * kSplit, kThreads, ssm, st>>>(g, nt);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }
   const int NT = N <= 256 ? N : 256;
   const int KC = resident ? K : 64;
   const int smem = kTileM * KC * 2 + NT * KC * 2;
-  cudaError_t e = cudaFuncSetAttribute(gemm_bf16_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return -2;
+  if (!allow_smem(gemm_bf16_tc, optin)) return -2;
   const int tiles = (M / kTileM) * ((N + NT - 1) / NT);
   const int grid = tiles < sms ? tiles : sms;
   gemm_bf16_tc<<<grid, kThreads, smem, st>>>(g);
