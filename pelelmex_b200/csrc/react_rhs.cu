@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(128) rk_t_from_hy(DevMech m, const double* __r
       w[k] = y * __ldg(m.inv_mw + k);
     }
     const double h = rhoH[c] * (1.0e4 / kRu);  // J/m^3 -> erg/g kg/m^3, over Ru
-    double t = T[c];
+    double t = rho == 0.0 ? nan("") : T[c];  // an empty cell (covered, say) has no temperature
     for (int it = 0; it < 100; ++it) {
       const double invT = 1.0 / t;
       double hs = 0.0, cs = 0.0;
