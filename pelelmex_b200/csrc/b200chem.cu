@@ -16,6 +16,7 @@
 #include "common.cuh"
 #include "jac_table.h"
 #include "react_group.cuh"
+#include "round_loop.h"
 
 using namespace b200;
 
@@ -220,16 +221,6 @@ struct StagedBuf {
   bool pending = false;
   cudaEvent_t ev = nullptr;
 };
-
-// Launch shapes of a round by how many cells are live: many (kernels in a row,
-// right-hand sides by thread), fewer (setup kernels on a branch), few
-// (right-hand sides by warp as well), and so few that the grids shrink to them.
-// The branch pays up to 131072 cells (32^3 H2: 4.56 ms, 5.03 without it above
-// the warp form's 9472 cells; 61x43x37 CH4: 44.3 and 45.8) and costs 10 % with
-// two million, whose kernels contend for L2.
-constexpr int kRoundClasses = 4;
-constexpr int kForkCells = 131072;
-constexpr int kTinyCells = 1024;
 
 struct b200chem_reactor {
   int device = 0;
@@ -656,33 +647,37 @@ int launch_rounds(b200chem_reactor* h, const ReactParams& P, cudaStream_t st, in
       }
       return Gc;
     };
-    bool captured[kRoundClasses] = {};
-    auto capture = [&](int cls) {
-      captured[cls] = true;
-      return capture_rounds(h, lut, R, shape(cls), per_check, Ls, cls);
-    };
-    long long live = R.nchunk;
-    for (long long round = 0;; round += per_check) {
-      if (round >= max_rounds) return set_err(B200CHEM_EINTEGRATE, "round-based integrator did not finish");
-      const int cls = live <= kTinyCells ? 3 : live <= G.rhs.warp_cells ? 2 : live <= kForkCells ? 1 : 0;
-      if (graph) {
-        if (!captured[cls] && (err = capture(cls))) return err;
-        CK(cudaGraphLaunch(h->rgraph[cls], st));
-      } else {
-        for (int r = 0; r < per_check; ++r) {
-          err = enqueue_round(h, lut, R, shape(cls), Ls, r & 1, st, st);
-          if (err) return err;
+    struct Ops {
+      b200chem_reactor* h;
+      const RoundsParams& R;
+      const RoundLists& Ls;
+      decltype(shape)& grids;
+      int lut, per_check;
+      bool graph;
+      cudaStream_t st;
+      int capture(int cls) { return capture_rounds(h, lut, R, grids(cls), per_check, Ls, cls); }
+      int launch(int cls) {
+        if (graph) {
+          CK(cudaGraphLaunch(h->rgraph[cls], st));
+        } else {
+          for (int r = 0; r < per_check; ++r) {
+            const int err = enqueue_round(h, lut, R, grids(cls), Ls, r & 1, st, st);
+            if (err) return err;
+          }
         }
+        h->launches += (graph && cls > 0 && h->n <= 32 ? 5LL : 6LL) * per_check;
+        // per_check is even: the live cells are back in the first list
+        CK(cudaMemcpyAsync(h->h_rcnt, Ls.cnt[0] + kRlRhs, sizeof(int), cudaMemcpyDeviceToHost, st));
+        return 0;
       }
-      h->launches += (graph && cls > 0 && h->n <= 32 ? 5LL : 6LL) * per_check;
-      // per_check is even: the live cells are back in the first list
-      CK(cudaMemcpyAsync(h->h_rcnt, Ls.cnt[0] + kRlRhs, sizeof(int), cudaMemcpyDeviceToHost, st));
-      // the next class's graph is made while this one runs
-      if (graph && cls + 1 < kRoundClasses && !captured[cls + 1] && (err = capture(cls + 1))) return err;
-      CK(cudaStreamSynchronize(st));
-      live = *h->h_rcnt;
-      if (live == 0) break;
-    }
+      int wait(long long* live) {
+        CK(cudaStreamSynchronize(st));
+        *live = *h->h_rcnt;
+        return 0;
+      }
+      int timed_out() { return set_err(B200CHEM_EINTEGRATE, "round-based integrator did not finish"); }
+    } ops{h, R, Ls, shape, lut, per_check, graph, st};
+    if ((err = run_rounds(ops, R.nchunk, G.rhs.warp_cells, max_rounds, per_check, graph))) return err;
   }
   return 0;
 }

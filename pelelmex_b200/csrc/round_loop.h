@@ -1,0 +1,51 @@
+// round_loop.h -- the host side of a chunk's rounds: which launch shape they take,
+// and the loop that launches them until no cell is live.
+#pragma once
+
+namespace b200 {
+
+// Launch shapes of a round by how many cells are live: many (kernels in a row,
+// right-hand sides by thread), fewer (setup kernels on a branch), few
+// (right-hand sides by warp as well), and so few that the grids shrink to them.
+// The branch pays up to 131072 cells (32^3 H2: 4.56 ms, 5.03 without it above
+// the warp form's 9472 cells; 61x43x37 CH4: 44.3 and 45.8) and costs 10 % with
+// two million, whose kernels contend for L2.
+constexpr int kRoundClasses = 4;
+constexpr int kForkCells = 131072;
+constexpr int kTinyCells = 1024;
+
+// Shape of a round with `live` cells; warp_cells: most cells that take the warp
+// form of the right-hand sides.
+inline int round_class(long long live, long long warp_cells) {
+  return live <= kTinyCells ? 3 : live <= warp_cells ? 2 : live <= kForkCells ? 1 : 0;
+}
+
+// Launches per_check rounds at a time until none of the `live` cells is left.
+// Ops: capture(cls) makes the graph of a shape, launch(cls) enqueues per_check
+// rounds of it and the read of the live count, wait(&live) waits for both;
+// timed_out() reports max_rounds.  All but timed_out return 0 or an error.
+// The next shape's graph is made while the rounds of this one run.  Should that
+// fail it is tried again when the shape is needed and nothing is running: the
+// loop never returns while the GPU still works on the caller's arrays.
+template <class Ops>
+int run_rounds(Ops& ops, long long live, long long warp_cells, long long max_rounds, int per_check, bool graph) {
+  bool captured[kRoundClasses] = {};
+  for (long long round = 0; live > 0; round += per_check) {
+    if (round >= max_rounds) return ops.timed_out();
+    const int cls = round_class(live, warp_cells);
+    int err = 0;
+    if (graph && !captured[cls]) {
+      err = ops.capture(cls);
+      captured[cls] = err == 0;
+    }
+    if (!err) err = ops.launch(cls);
+    if (!err && graph && cls + 1 < kRoundClasses && !captured[cls + 1]) captured[cls + 1] = ops.capture(cls + 1) == 0;
+    long long left = 0;
+    const int werr = ops.wait(&left);
+    if (err || werr) return err ? err : werr;
+    live = left;
+  }
+  return 0;
+}
+
+}  // namespace b200
