@@ -20,6 +20,14 @@ inline int round_class(long long live, long long warp_cells) {
   return live <= kTinyCells ? 3 : live <= warp_cells ? 2 : live <= kForkCells ? 1 : 0;
 }
 
+// The shape after cls that a call comes to next, or kRoundClasses: a mechanism
+// without a warp form (warp_cells 0) has no class 2.
+inline int next_round_class(int cls, long long warp_cells) {
+  for (++cls; cls < kRoundClasses; ++cls)
+    if (cls == 1 ? warp_cells < kForkCells : cls == 2 ? warp_cells > kTinyCells : true) break;
+  return cls;
+}
+
 // Launches per_check rounds at a time until none of the `live` cells is left.
 // Ops: capture(cls) makes the graph of a shape, launch(cls) enqueues per_check
 // rounds of it and the read of the live count, wait(&live) waits for both;
@@ -39,7 +47,8 @@ int run_rounds(Ops& ops, long long live, long long warp_cells, long long max_rou
       captured[cls] = err == 0;
     }
     if (!err) err = ops.launch(cls);
-    if (!err && graph && cls + 1 < kRoundClasses && !captured[cls + 1]) captured[cls + 1] = ops.capture(cls + 1) == 0;
+    const int next = next_round_class(cls, warp_cells);
+    if (!err && graph && next < kRoundClasses && !captured[next]) captured[next] = ops.capture(next) == 0;
     long long left = 0;
     const int werr = ops.wait(&left);
     if (err || werr) return err ? err : werr;

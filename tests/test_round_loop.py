@@ -36,6 +36,13 @@ def test_shapes_follow_the_live_cells(run):
     assert run(200000, LEFT, graph=0) == (0, "l0 w l0 w l1 w l2 w l3 w".split())
 
 
+def test_no_graph_of_a_shape_that_cannot_come(run):
+    # no warp form (no generated code): class 2 is empty; one that reaches beyond
+    # the cells of class 1 leaves that one empty
+    assert run(200000, [90000, 3000, 300, 0], warp_cells=0) == (0, "c0 l0 c1 w l1 c3 w l1 w l3 w".split())
+    assert run(200000, [90000, 3000, 300, 0], warp_cells=140000) == (0, "c0 l0 c2 w l2 c3 w l2 w l3 w".split())
+
+
 def test_graph_made_ahead_that_fails_is_tried_again_when_needed(run):
     # class 2 fails beside the rounds of class 1, and again with nothing running
     assert run(200000, LEFT, fail_capture=2) == (-7, "c0 l0 c1 w l0 w l1 c2 w c2 w".split())
