@@ -549,11 +549,13 @@ def run_b200(args, rank, world, local_rank, field):
     # the first launch of rk_step passes over the cells of the second (their
     # entries are in its list): what it works on is the rest
     prof["ctrl"]["cells"] -= prof["ctrl_setup"]["cells"]
-    for k in ("start", "rhs", "ctrl", "jac", "gj", "ctrl_setup"):
+    for k in ("start", "rhs", "ctrl", "jac", "gj", "ctrl_setup", "ctrl_rare"):
         v = prof[k]
+        kernels[k] = dict(v, share=v["ms"] / tot_ms if tot_ms else None)
+        if k == "ctrl_rare":  # the state machine: no bytes a cell cannot do without
+            continue
         b = perfmodel.kernel_bytes(k, N) * v["cells"]
-        kernels[k] = dict(v, share=v["ms"] / tot_ms if tot_ms else None,
-                          algorithmic_gbs=(b / (v["ms"] * 1e-3) / 1e9) if v["ms"] else None, bytes=b)
+        kernels[k].update(algorithmic_gbs=(b / (v["ms"] * 1e-3) / 1e9) if v["ms"] else None, bytes=b)
     # dominant kernel: rk_step (both of its launches per round)
     c_ms = kernels["ctrl"]["ms"] + kernels["ctrl_setup"]["ms"]
     c_launch = kernels["ctrl"]["launches"] + kernels["ctrl_setup"]["launches"]

@@ -350,7 +350,8 @@ int b200chem_selftest_bounded_wait(int* err, int polls, void* stream);
 enum {
   B200CHEM_PROF_START = 0,       /* rk_start: load, validate, initialise   */
   B200CHEM_PROF_RHS = 1,         /* rk_rhs: right-hand sides               */
-  B200CHEM_PROF_CTRL = 2,        /* rk_step after the right-hand sides     */
+  B200CHEM_PROF_CTRL = 2,        /* rk_step after the right-hand sides; its list holds the cells of
+                                    PROF_CTRL_SETUP as well, which it passes over                  */
   B200CHEM_PROF_JAC = 3,         /* rk_jac: analytic Jacobians             */
   B200CHEM_PROF_GJ = 4,          /* rk_gj: Newton-matrix inverses          */
   B200CHEM_PROF_CTRL_SETUP = 5,  /* rk_step after a setup                  */

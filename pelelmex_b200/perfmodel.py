@@ -121,7 +121,7 @@ def kernel_bytes(kind: str, n_species: int, lut_bytes: int = 4) -> float:
       the inverse (n^2 at lut_bytes); the Nordsieck columns of a completed
       step are not counted
     * jac (only the setups whose Jacobian is stale reach it): list slot,
-      read y and f (2n), write J (n^2)
+      read y and the forcing (2n), write J (n^2)
     * gj: list slot and gamma, read J (n^2) and ewt (n), write the scaling
       (n) and the inverse (n^2 at lut_bytes)
     """
@@ -140,7 +140,7 @@ def kernel_bytes(kind: str, n_species: int, lut_bytes: int = 4) -> float:
 
 
 def jac_refresh_bytes(n_species: int) -> float:
-    """HBM bytes of one analytic-Jacobian refresh: read y and f (2n), write
-    J (n^2)."""
+    """HBM bytes of one analytic-Jacobian refresh: read y and the forcing
+    (2n), write J (n^2)."""
     n = n_species + 1
     return 8 * 2 * n + 8 * n * n

@@ -232,7 +232,10 @@ class ReactorB200:
 
     def profile_end(self) -> dict:
         """{kind: {"launches", "cells", "ms"}} since profile_begin, kinds
-        start / rhs / ctrl / jac / gj / ctrl_setup; plus "complete"."""
+        start / rhs / ctrl / jac / gj / ctrl_setup / ctrl_rare; plus "complete".
+        cells are list entries: ctrl's list holds the cells of ctrl_setup too, which
+        its launch passes over, so it works on the difference.  ctrl_rare is the
+        control kernel (starts, failures, ends of cells)."""
         self._need()
         p = _lib.KernelProfile()
         _lib.check(_lib.load().b200chem_profile_end(self._h, ctypes.byref(p)))
