@@ -51,6 +51,7 @@ def _d(x: float) -> str:
 
 
 KRU = 8.31446261815324e7  # erg/mol/K, as in the device code
+PATM = 1013250.0  # dyn/cm^2
 # largest magnitude of an exponential's argument in the generated code (its
 # exponential has no overflow or underflow handling)
 EXP_LIMIT = 690.0
@@ -65,19 +66,28 @@ def _nasa_g(nasa, T):
 
 def temperature_range(flat) -> tuple:
     """Widest range of temperatures around 1000 K in which every exponential of
-    the generated right-hand side, and every product of species exponentials,
-    stays within EXP_LIMIT; outside it the table form is used."""
+    the generated right-hand side (Troe's may underflow, not overflow) and every
+    product of species exponentials, after each of its factors, stay within
+    EXP_LIMIT; outside it the table form is used."""
     a = flat.arrays
     nu, sp = a["nu"], a["sp"]
 
     def fine(T):
         g = _nasa_g(a["nasa"], T)
         ok = np.abs(g).max() <= EXP_LIMIT
+        lnu = np.log(T * KRU / PATM)
         for j in range(flat.n_reactions):
             for key in ("arr", "arr_lo", "arr_rev"):
                 ok &= abs(a[key][j][0] + a[key][j][1] * np.log(T) - a[key][j][2] / T) <= EXP_LIMIT
-            side = [sum(int(nu[j, s]) * g[sp[j, s]] for s in r if sp[j, s] >= 0) for r in (range(4), range(4, 8))]
-            ok &= max(abs(side[0]), abs(side[1]), abs(side[1] - side[0])) <= EXP_LIMIT
+            if a["rtype"][j] == 3:
+                _, t3, t1, t2 = a["troe"][j]
+                ok &= max(-T / t3, -T / t1, -t2 / T if a["rflags"][j] & 4 else 0.0) <= EXP_LIMIT
+            # exponents of the factors in the order of the product: products,
+            # reactants, powers of the standard concentration
+            sides = [[sp[j, s] for s in r if sp[j, s] >= 0 for _ in range(int(nu[j, s]))] for r in (range(4), range(4, 8))]
+            dn = len(sides[1]) - len(sides[0])
+            e = np.concatenate([g[sides[1]], -g[sides[0]], np.full(abs(dn), np.sign(dn) * lnu)])
+            ok &= np.abs(np.cumsum(e)).max() <= EXP_LIMIT
         return bool(ok)
 
     lo, hi = 1000.0, 1000.0
