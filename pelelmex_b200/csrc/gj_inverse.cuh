@@ -31,24 +31,21 @@ __device__ __forceinline__ void store_inverse_row(const LUT* src, const int* pin
   }
 }
 
-// In-place Gauss-Jordan inverse of the scaled Newton matrix D (I - gamma J)
-// D^-1 (FP32, D = diag(dsc)) or I - gamma J (FP64) with partial pivoting, one
-// warp per cell, lane i holding row i in registers (n <= 32).  Rows are never
-// exchanged: step k takes as pivot the unused row p_k with the largest
-// |a[., k]|, and at the end the inverse is (A^-1)[k][j] = X[p_k][q_j] with
-// q_j the step at which row j was the pivot; that permutation is applied
-// while the result is written to Ar (mat_idx order).  Xs, prow, pinv: per-warp
-// shared scratch.  Returns 0, or k+1 when no usable pivot is left at step k.
-template <int n, typename LUT>
-__device__ __forceinline__ int reg_gj_inverse(const double* J, const double* dsc, double gamma, LUT* Xs, int ldl,
-                                              int* prow, int* pinv, LUT* Ar, int lane) {
+// In-place Gauss-Jordan inverse of the Newton matrix I - gamma J with partial
+// pivoting, in FP64 (n <= 32): one warp per cell, lane i holding row i in
+// registers.  Rows are never exchanged: step k takes as pivot the unused row p_k
+// with the largest |a[., k]|, and at the end the inverse is (A^-1)[k][j] =
+// X[p_k][q_j] with q_j the step at which row j was the pivot; that permutation is
+// applied while the result is written to Ar (mat_idx order).  Xs, prow, pinv:
+// per-warp shared scratch.  Returns 0, or k+1 when no usable pivot is left at
+// step k.
+template <int n>
+__device__ __forceinline__ int reg_gj_inverse(const double* J, double gamma, double* Xs, int ldl, int* prow, int* pinv,
+                                              double* Ar, int lane) {
   constexpr int G = ctrl_group(n);
-  static_assert(n <= 32, "one row per lane");
-  constexpr bool kScaled = sizeof(LUT) == 4;
+  static_assert(n <= 32 && n % 2 == 0, "one row per lane, no column padding");
   const bool row = lane < n;
-  const double di = row ? dsc[lane] : 1.0;
-  const double rdi = 1.0 / di;
-  LUT a[n];
+  double a[n];
 #pragma unroll
   for (int jb = 0; jb < n / kVJ; ++jb) {
     double2 jv = make_double2(0.0, 0.0);
@@ -56,39 +53,27 @@ __device__ __forceinline__ int reg_gj_inverse(const double* J, const double* dsc
 #pragma unroll
     for (int e = 0; e < kVJ; ++e) {
       const int j = jb * kVJ + e;
-      const double rdj = __shfl_sync(kAllLanes, rdi, j);
-      const double mij = ((lane == j) ? 1.0 : 0.0) - gamma * (e ? jv.y : jv.x);
-      a[j] = row ? (LUT)(kScaled ? mij * di * rdj : mij) : (LUT)0;
+      a[j] = row ? ((lane == j) ? 1.0 : 0.0) - gamma * (e ? jv.y : jv.x) : 0.0;
     }
   }
-  // Pivot search by one warp reduction: key = the bits of |a[k]| (FP32; the
-  // high word for FP64) with the low 5 bits replaced by (31 - lane), so the
-  // maximum picks the largest magnitude (to 2^-18 relative in FP32, 2^-15 in
-  // FP64) and, among equals, the lowest lane.
+  // Pivot search by one warp reduction: key = the high word of |a[k]| with the
+  // low 5 bits replaced by (31 - lane), so the maximum picks the largest
+  // magnitude (to 2^-15 relative) and, among equals, the lowest lane.
   // The pivot row goes through shared memory (two buffers, alternating per
   // step, 16-byte chunks) and every row, the pivot row included, is updated
   // by one FMA per column: a_ij -= g_i * a_pj with g_i = a_ik / a_pk off the
   // pivot row and g_p = 1 - 1 / a_pk on it (which scales the pivot row by
   // 1 / a_pk); column k is set last (1 / a_pk on the pivot row, -g_i off it).
   // The columns rotate by one register per step, so that column k is always
-  // a[0] and the loop needs no unrolling (unrolled, the 54-step form is 150 KB
-  // of code and waits for instructions: 766,122 inverses 38 ms, now 26).
-  constexpr int kVec = 16 / (int)sizeof(LUT);      // LUTs per 16-byte chunk
-  constexpr int kChunks = (n + kVec - 1) / kVec;
-  constexpr int kBuf = 32;                         // LUTs per row buffer (>= kChunks * kVec)
-  static_assert(kChunks * kVec <= kBuf, "row buffer");
+  // a[0] and the loop needs no unrolling.
+  constexpr int kBuf = 32;  // entries per row buffer
   unsigned used = 0;
   int mystep = -1;
 #pragma unroll 1
   for (int k = 0; k < n; ++k) {
-    LUT* buf = Xs + (k & 1) * kBuf;
+    double* buf = Xs + (k & 1) * kBuf;
     unsigned key = 0u;
-    if (row && !((used >> lane) & 1u)) {
-      unsigned bits;
-      if constexpr (sizeof(LUT) == 4) bits = __float_as_uint(fabsf((float)a[0]));
-      else bits = (unsigned)__double2hiint(fabs((double)a[0]));
-      key = (bits & ~31u) | (unsigned)(31 - lane);
-    }
+    if (row && !((used >> lane) & 1u)) key = ((unsigned)__double2hiint(fabs(a[0])) & ~31u) | (unsigned)(31 - lane);
     const unsigned kmax = __reduce_max_sync(kAllLanes, key);
     if ((kmax >> 5) == 0u) return k + 1;  // no nonzero candidate: singular (warp-uniform)
     const int p = 31 - (int)(kmax & 31u);
@@ -96,21 +81,20 @@ __device__ __forceinline__ int reg_gj_inverse(const double* J, const double* dsc
     if (lane == p) {
       mystep = k;
 #pragma unroll
-      for (int c = 0; c < kChunks; ++c) {
-        LUT t[kVec];
-#pragma unroll
-        for (int e = 0; e < kVec; ++e) t[e] = (c * kVec + e < n) ? a[c * kVec + e] : (LUT)0;
-        *reinterpret_cast<uint4*>(buf + c * kVec) = *reinterpret_cast<const uint4*>(t);
-      }
+      for (int c = 0; c < n / 2; ++c) reinterpret_cast<double2*>(buf)[c] = make_double2(a[2 * c], a[2 * c + 1]);
     }
     __syncwarp();
-    LUT pr[kChunks * kVec];
+    double pr[n];
 #pragma unroll
-    for (int c = 0; c < kChunks; ++c) *reinterpret_cast<uint4*>(pr + c * kVec) = *reinterpret_cast<const uint4*>(buf + c * kVec);
-    const LUT pv = pr[0];
-    if (!(fabs(pv) > (LUT)0) || isnan(pv)) return k + 1;  // zero or NaN pivot (warp-uniform)
-    const LUT inv = (LUT)1 / pv;
-    const LUT gi = (lane == p) ? (LUT)1 - inv : a[0] * inv;
+    for (int c = 0; c < n / 2; ++c) {
+      const double2 t = reinterpret_cast<const double2*>(buf)[c];
+      pr[2 * c] = t.x;
+      pr[2 * c + 1] = t.y;
+    }
+    const double pv = pr[0];
+    if (!(fabs(pv) > 0.0) || isnan(pv)) return k + 1;  // zero or NaN pivot (warp-uniform)
+    const double inv = 1.0 / pv;
+    const double gi = (lane == p) ? 1.0 - inv : a[0] * inv;
 #pragma unroll
     for (int j = 1; j < n; ++j) a[j - 1] = fma(-gi, pr[j], a[j]);
     a[n - 1] = (lane == p) ? inv : -gi;
@@ -123,13 +107,14 @@ __device__ __forceinline__ int reg_gj_inverse(const double* J, const double* dsc
     prow[mystep] = lane;
   }
   __syncwarp();
-  if (lane < n) store_inverse_row<n, LUT>(Xs + prow[lane] * ldl, pinv, Ar, lane);
+  if (row) store_inverse_row<n, double>(Xs + prow[lane] * ldl, pinv, Ar, lane);
   __syncwarp();
   return 0;
 }
 
-// The same inverse for n <= 32 in FP32 by a group of G lanes per cell, lane g
-// holding rows g, g + G, ... in registers: a pivot step costs its search, its
+// The inverse of the scaled matrix D (I - gamma J) D^-1, D = diag(dsc), the same
+// way for n <= 32 in FP32 by a group of G lanes per cell, lane g holding rows g,
+// g + G, ... in registers: a pivot step costs its search, its
 // exchange and its reciprocal once for the 32 / G cells of a warp, and a row
 // chunk read from shared memory feeds every row of the lane.  All lanes of the
 // warp call it; a group without a cell (live false) works on zeros.  Xs: two
@@ -253,20 +238,22 @@ __device__ __forceinline__ int grp_reg_gj_inverse(const double* J, bool live, co
   return ier;
 }
 
-// The same inverse for 32 < n <= 64 in FP32: lane l holds rows l and l + 32
-// in registers.  The pivot key carries the row index (6 bits) instead of the
-// lane; the pivot row's owner writes it to shared memory and every lane
-// updates both of its rows from 16-byte reads of it.
-template <int n, typename LUT>
-__device__ __forceinline__ int reg_gj_inverse2(const double* J, const double* dsc, double gamma, LUT* Xs, int ldl,
-                                               int* prow, int* pinv, LUT* Ar, int lane) {
+// The inverse of the scaled matrix for 32 < n <= 64 in FP32: lane l of a warp
+// holds rows l and l + 32 in registers.  The pivot key carries the row index (6
+// bits) instead of the lane; the pivot row's owner writes it to shared memory and
+// every lane updates both of its rows from 16-byte reads of it.  Unrolled, the 54
+// steps are 150 KB of code that waits for instructions: 766,122 inverses took 38
+// ms and take 26 in the rolled loop.
+template <int n>
+__device__ __forceinline__ int reg_gj_inverse2(const double* J, const double* dsc, double gamma, float* Xs, int ldl,
+                                               int* prow, int* pinv, float* Ar, int lane) {
   constexpr int G = ctrl_group(n);
-  static_assert(n > 32 && n <= 64 && sizeof(LUT) == 4, "two FP32 rows per lane");
+  static_assert(n > 32 && n <= 64, "two rows per lane");
   const int r1 = lane + 32;
   const bool row1 = r1 < n;
   const double d0 = dsc[lane], d1 = row1 ? dsc[r1] : 1.0;
   const double rd0 = 1.0 / d0, rd1 = 1.0 / d1;
-  LUT a0[n], a1[n];
+  float a0[n], a1[n];
 #pragma unroll
   for (int jb = 0; jb < n / kVJ; ++jb) {
     const double2 j0 = *reinterpret_cast<const double2*>(J + mat_vec<n, G, kVJ>(lane / G, lane % G, jb));
@@ -278,8 +265,8 @@ __device__ __forceinline__ int reg_gj_inverse2(const double* J, const double* ds
       const double rdj = (j < 32) ? __shfl_sync(kAllLanes, rd0, j) : __shfl_sync(kAllLanes, rd1, j - 32);
       const double m0 = ((lane == j) ? 1.0 : 0.0) - gamma * (e ? j0.y : j0.x);
       const double m1 = row1 ? ((r1 == j) ? 1.0 : 0.0) - gamma * (e ? j1.y : j1.x) : 0.0;
-      a0[j] = (LUT)(m0 * d0 * rdj);
-      a1[j] = row1 ? (LUT)(m1 * d1 * rdj) : (LUT)0;
+      a0[j] = (float)(m0 * d0 * rdj);
+      a1[j] = row1 ? (float)(m1 * d1 * rdj) : 0.f;
     }
   }
   constexpr int kChunks = (n + 3) / 4;
@@ -288,7 +275,7 @@ __device__ __forceinline__ int reg_gj_inverse2(const double* J, const double* ds
   int step0 = -1, step1 = -1;
 #pragma unroll 1
   for (int k = 0; k < n; ++k) {
-    LUT* buf = Xs + (k & 1) * kBuf;
+    float* buf = Xs + (k & 1) * kBuf;
     unsigned key = 0u;
     if (!((used0 >> lane) & 1u)) key = (__float_as_uint(fabsf(a0[0])) & ~63u) | (unsigned)(63 - lane);
     if (row1 && !((used1 >> lane) & 1u)) {
@@ -327,11 +314,11 @@ __device__ __forceinline__ int reg_gj_inverse2(const double* J, const double* ds
       }
     }
     __syncwarp();
-    const LUT pv = buf[0];
+    const float pv = buf[0];
     if (!(fabsf(pv) > 0.f) || isnan(pv)) return k + 1;  // zero or NaN pivot (warp-uniform)
-    const LUT inv = 1.f / pv;
-    const LUT g0 = (p == lane) ? 1.f - inv : a0[0] * inv;
-    const LUT g1 = (p == r1) ? 1.f - inv : a1[0] * inv;
+    const float inv = 1.f / pv;
+    const float g0 = (p == lane) ? 1.f - inv : a0[0] * inv;
+    const float g1 = (p == r1) ? 1.f - inv : a1[0] * inv;
 #pragma unroll
     for (int c = 0; c < kChunks; ++c) {
       const float4 q = reinterpret_cast<const float4*>(buf)[c];
@@ -364,7 +351,7 @@ __device__ __forceinline__ int reg_gj_inverse2(const double* J, const double* ds
   __syncwarp();
   for (int h = 0; h < 2; ++h) {
     const int i = lane + 32 * h;
-    if (i < n) store_inverse_row<n, LUT>(Xs + prow[i] * ldl, pinv, Ar, i);
+    if (i < n) store_inverse_row<n, float>(Xs + prow[i] * ldl, pinv, Ar, i);
   }
   __syncwarp();
   return 0;

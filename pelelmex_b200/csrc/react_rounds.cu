@@ -729,9 +729,9 @@ __global__ void __launch_bounds__(128, gj_min_ctas<NS + 1, LUT>()) rk_gj(RoundsP
       __syncwarp();
       int ier;
       if constexpr (WCPL == 1) {
-        ier = reg_gj_inverse<n, LUT>(J, Dsc, gamma, A, SL.ldl, ipiv, ipiv2, Ar, lane);
+        ier = reg_gj_inverse<n>(J, gamma, A, SL.ldl, ipiv, ipiv2, Ar, lane);
       } else if constexpr (WCPL == 2 && sizeof(LUT) == 4) {
-        ier = reg_gj_inverse2<n, LUT>(J, Dsc, gamma, A, SL.ldl, ipiv, ipiv2, Ar, lane);
+        ier = reg_gj_inverse2<n>(J, Dsc, gamma, A, SL.ldl, ipiv, ipiv2, Ar, lane);
       } else {
         static_assert(sizeof(LUT) == 8, "the unscaled matrix");
         constexpr int G = ctrl_group(n);

@@ -24,9 +24,9 @@ int invert(const double* J, const double* dsc, double gamma, int order, double* 
   for (int g = 0; g < GPW; ++g) std::fill(Ar[g], Ar[g] + n * ((n + V - 1) / V) * V, (LUT)0);
   warp_host::run([&](int lane) {
     if constexpr (form == 0) {
-      ier[lane] = reg_gj_inverse<n, LUT>(Jr, dl, gamma, Xs[0], ldl, prow[0], pinv[0], Ar[0], lane);
+      ier[lane] = reg_gj_inverse<n>(Jr, gamma, Xs[0], ldl, prow[0], pinv[0], Ar[0], lane);
     } else if constexpr (form == 1) {
-      ier[lane] = reg_gj_inverse2<n, LUT>(Jr, dl, gamma, Xs[0], ldl, prow[0], pinv[0], Ar[0], lane);
+      ier[lane] = reg_gj_inverse2<n>(Jr, dl, gamma, Xs[0], ldl, prow[0], pinv[0], Ar[0], lane);
     } else {
       const int gi = lane / G, gl = lane % G;
       const bool live = gi + 1 < GPW;
