@@ -43,7 +43,7 @@ enum Label : int {
   kLAfterRestart,  // f(y) after an order-1 restart
   kLAfterSetup,    // f(predicted y) evaluated and Newton matrix rebuilt (setup_ier holds its status)
   // internal labels
-  kLStart, kLBeginStep, kLAttempt, kLNlsAttempt, kLNlsRecover, kLNlsFail1, kLNlsFail2, kLNlsSuccess,
+  kLStart, kLAttempt, kLNlsAttempt, kLNlsRecover, kLNlsFail1, kLNlsFail2, kLNlsSuccess,
   kLStall
 };
 
@@ -57,14 +57,14 @@ enum Need : int { kNeedRhs = 0, kNeedSetup = 1, kDone = 2, kNeedSetupJac = 3 };
 // multiple of 16 bytes so that it moves as 16-byte vectors.
 struct alignas(16) RCell {
   double tau[kZn + 2], tq[6], l[kZn];
-  double h, hprime, hscale, eta, etamax, tn, gamma, gammap, gamrat, crate, acnrm, rl1, saved_tq5, gamma_lu;
+  double h, hscale, eta, etamax, tn, gamma, gammap, gamrat, crate, acnrm, rl1, saved_tq5, gamma_lu;
   double dt, saved_t, delp, hg, hub, hlb;
-  int q, qprime, L, qwait, nstlp, nstlj, jcur, ncf, nef, nflag, convfail, callSetup, jbad, mnewt, attempt;
+  int q, L, qwait, nstlp, nstlj, jcur, ncf, nef, nflag, convfail, callSetup, jbad, mnewt, attempt;
   int count1, hnewOK, nstloc, qmax, max_steps, setup_conv, label, setup_ier;
   CellCounters cnt;
   float refine_ratio;  // WRMS of the last FP64 refinement step over its correction (kRefineUnknown: none since
                        // the last setup)
-  int pad_;
+  int pad_[4];  // 448 bytes in all, which keep a warp's cells apart in the banks
 };
 static_assert(sizeof(RCell) % 16 == 0, "RCell moves as 16-byte vectors");
 
@@ -119,8 +119,8 @@ __device__ __forceinline__ unsigned char* rec_of(const RState& S, long long slot
 // Field-by-field copies (no address of the local RCell is taken, so its
 // fields can live in registers).
 #define B200_RCELL_SCALARS(X)                                                                              \
-  X(h) X(hprime) X(hscale) X(eta) X(etamax) X(tn) X(gamma) X(gammap) X(gamrat) X(crate) X(acnrm) X(rl1)    \
-  X(saved_tq5) X(gamma_lu) X(dt) X(saved_t) X(delp) X(hg) X(hub) X(hlb) X(q) X(qprime) X(L) X(qwait)      \
+  X(h) X(hscale) X(eta) X(etamax) X(tn) X(gamma) X(gammap) X(gamrat) X(crate) X(acnrm) X(rl1)    \
+  X(saved_tq5) X(gamma_lu) X(dt) X(saved_t) X(delp) X(hg) X(hub) X(hlb) X(q) X(L) X(qwait)      \
   X(nstlp) X(nstlj) X(jcur) X(ncf) X(nef) X(nflag) X(convfail) X(callSetup) X(jbad) X(mnewt) X(attempt)    \
   X(count1) X(hnewOK) X(nstloc) X(qmax) X(max_steps) X(setup_conv) X(label) X(setup_ier) X(cnt.nst)       \
   X(cnt.nfe) X(cnt.nje) X(cnt.nlu) X(cnt.netf) X(cnt.ncfn) X(cnt.nni) X(refine_ratio)
@@ -308,42 +308,6 @@ __device__ __forceinline__ void r_set_bdf(RCell& c) {
 }
 
 template <int n, int G>
-__device__ __forceinline__ void r_increase(RCell& c, const RVec<n>& v, int gl) {
-  const int q = c.q;
-#pragma unroll
-  for (int i = 0; i < kZn; ++i)
-    if (i <= c.qmax) c.l[i] = 0.0;
-  double alpha1 = 1.0, prod = 1.0, xiold = 1.0, alpha0 = -1.0, hsum = c.hscale;
-  c.l[2] = 1.0;
-#pragma unroll
-  for (int j = 1; j < kZn - 1; ++j) {
-    if (j < q) {
-      hsum += c.tau[j + 1];
-      const double xi = hsum / c.hscale;
-      prod *= xi;
-      alpha0 -= 1.0 / (j + 1);
-      alpha1 += 1.0 / xi;
-#pragma unroll
-      for (int i = j + 2; i >= 2; --i)
-        if (i < kZn) c.l[i] = c.l[i] * xiold + c.l[i - 1];
-      xiold = xi;
-    }
-  }
-  const double A1 = (-alpha0 - alpha1) / prod;
-  const int qm = c.qmax;
-  double lj[kZn];
-#pragma unroll
-  for (int j = 0; j < kZn; ++j) lj[j] = c.l[j];
-  each<n, G>(gl, [&](int i) {
-    const double z = A1 * v.zn(qm, i);
-    v.zn(q + 1, i) = z;
-#pragma unroll
-    for (int j = 2; j < kZn; ++j)
-      if (j <= q) v.zn(j, i) += lj[j] * z;
-  });
-}
-
-template <int n, int G>
 __device__ __forceinline__ void r_decrease(RCell& c, const RVec<n>& v, int gl) {
   const int q = c.q;
 #pragma unroll
@@ -375,60 +339,6 @@ __device__ __forceinline__ void r_decrease(RCell& c, const RVec<n>& v, int gl) {
 template <int n, int G>
 __device__ __forceinline__ void r_set_ewt(const RVec<n>& v, const double* atolv, double rtol, int gl) {
   each<n, G>(gl, [&](int i) { v.ewt(i) = 1.0 / (rtol * fabs(v.zn(0, i)) + __ldg(atolv + i)); });
-}
-
-template <int n, int G>
-__device__ __forceinline__ void r_prepare_next(RCell& c, const RVec<n>& v, double dsm, int gl, unsigned gm) {
-  if (c.etamax == 1.0) {
-    c.qwait = c.qwait > 2 ? c.qwait : 2;
-    c.qprime = c.q;
-    c.hprime = c.h;
-    c.eta = 1.0;
-    return;
-  }
-  const double etaq = 1.0 / (pow(kBIAS2 * dsm, 1.0 / c.L) + kADDON);
-  if (c.qwait != 0) {
-    c.eta = etaq;
-    c.qprime = c.q;
-  } else {
-    c.qwait = 2;
-    double etaqm1 = 0.0, etaqp1 = 0.0;
-    if (c.q > 1) {
-      const int q = c.q;
-      const double ddn = r_wrms<n, G>(v, gl, gm, [&](int i) { return v.zn(q, i); }) * c.tq[1];
-      etaqm1 = 1.0 / (pow(kBIAS1 * ddn, 1.0 / c.q) + kADDON);
-    }
-    if (c.q != c.qmax && c.saved_tq5 != 0.0) {
-      const double cquot = (c.tq[5] / c.saved_tq5) * pow(c.h / c.tau[2], (double)c.L);
-      const int qm = c.qmax;
-      const double dup =
-          r_wrms<n, G>(v, gl, gm, [&](int i) { return v.acor(i) - cquot * v.zn(qm, i); }) * c.tq[3];
-      etaqp1 = 1.0 / (pow(kBIAS3 * dup, 1.0 / (c.L + 1)) + kADDON);
-    }
-    const double etam = fmax(etaqm1, fmax(etaq, etaqp1));
-    if (etam < kTHRESH) {
-      c.eta = 1.0;
-      c.qprime = c.q;
-    } else if (etam == etaq) {
-      c.eta = etaq;
-      c.qprime = c.q;
-    } else if (etam == etaqm1) {
-      c.eta = etaqm1;
-      c.qprime = c.q - 1;
-    } else {
-      c.eta = etaqp1;
-      c.qprime = c.q + 1;
-      const int qm = c.qmax;
-      each<n, G>(gl, [&](int i) { v.zn(qm, i) = v.acor(i); });
-    }
-  }
-  if (c.eta < kTHRESH) {
-    c.eta = 1.0;
-    c.hprime = c.h;
-  } else {
-    c.eta = fmin(c.eta, c.etamax);
-    c.hprime = c.h * c.eta;
-  }
 }
 
 // Internal status of a cell stopped for the FP64 retry (never reported).
@@ -716,8 +626,6 @@ __device__ __forceinline__ int g_finish_step(const RCell& c, RCell& o, const RVe
     }
   }
   o.saved_t = c.tn;
-  o.qprime = qprime;
-  o.hprime = hprime;
   o.eta = eta;
   o.q = q;
   o.L = L;
@@ -916,31 +824,12 @@ __device__ __forceinline__ int r_advance(RCell& c, const RVec<n>& v, int lab, co
       }
       case kLStart: {
         const double h0 = c.h;
-        c.hscale = c.hprime = h0;
+        c.hscale = h0;
         each<n, G>(gl, [&](int i) { v.zn(1, i) *= h0; });
         c.nstloc = 0;
-        lab = kLBeginStep;
-        break;
-      }
-      case kLBeginStep: {
-        if (c.cnt.nst > 0) r_set_ewt<n, G>(v, atolv, rtol, gl);
-        if (c.nstloc >= c.max_steps) {
-          *status = -1;
-          return kDone;
-        }
         c.saved_t = c.tn;
         c.ncf = c.nef = 0;
         c.nflag = kFirstCall;
-        if (c.cnt.nst > 0 && c.hprime != c.h) {
-          if (c.qprime != c.q) {
-            if (c.qprime - c.q == 1) r_increase<n, G>(c, v, gl);
-            else if (c.qprime - c.q == -1) r_decrease<n, G>(c, v, gl);
-            c.q = c.qprime;
-            c.L = c.q + 1;
-            c.qwait = c.L;
-          }
-          r_rescale<n, G>(c, v, gl);
-        }
         lab = kLAttempt;
         break;
       }
@@ -998,16 +887,10 @@ __device__ __forceinline__ int r_advance(RCell& c, const RVec<n>& v, int lab, co
       case kLNlsSuccess: {
         const double dsm = c.acnrm * c.tq[2];
         if (dsm <= 1.0) {
-          // complete the step
+          // the last step of the cell, at dt or at the limit of steps (the step
+          // kernel completes every other): its state is all that is still needed
           c.cnt.nst++;
-#pragma unroll
-          for (int i = kZn + 1; i >= 2; --i)
-            if (i <= c.q) c.tau[i] = c.tau[i - 1];
-          if (c.q == 1 && c.cnt.nst > 1) c.tau[2] = c.tau[1];
-          c.tau[1] = c.h;
           const int q = c.q;
-          const bool save = (c.qwait - 1 == 1 && q != c.qmax);
-          const int qm = c.qmax;
           double lj[kZn];
 #pragma unroll
           for (int j = 0; j < kZn; ++j) lj[j] = c.l[j];
@@ -1016,19 +899,9 @@ __device__ __forceinline__ int r_advance(RCell& c, const RVec<n>& v, int lab, co
 #pragma unroll
             for (int j = 0; j < kZn; ++j)
               if (j <= q) v.zn(j, i) += lj[j] * ac;
-            if (save) v.zn(qm, i) = ac;
           });
-          c.qwait--;
-          if (save) c.saved_tq5 = c.tq[5];
-          r_prepare_next<n, G>(c, v, dsm, gl, gm);
-          c.etamax = (c.cnt.nst <= kSMALL_NST) ? kETAMX2 : kETAMX3;
-          c.nstloc++;
-          if (c.tn - c.dt >= 0.0) {
-            *status = 0;
-            return kDone;
-          }
-          lab = kLBeginStep;
-          break;
+          *status = (c.tn - c.dt >= 0.0) ? 0 : -1;
+          return kDone;
         }
         c.nef++;
         c.cnt.netf++;
@@ -1090,7 +963,7 @@ __device__ __forceinline__ void r_begin(RCell& c, const RVec<n>& v, const double
   c.cnt = CellCounters{0, 0, 0, 0, 0, 0, 0};
   c.refine_ratio = kRefineUnknown;
   c.nstlp = c.nstlj = 0;
-  c.q = c.qprime = 1;
+  c.q = 1;
   c.L = 2;
   c.qwait = c.L;
   c.etamax = kETAMX1;
@@ -1102,7 +975,7 @@ __device__ __forceinline__ void r_begin(RCell& c, const RVec<n>& v, const double
   c.gamma_lu = 1.0;
   c.qmax = qmax;
   c.max_steps = max_steps;
-  c.h = c.hprime = c.hscale = c.eta = 1.0;
+  c.h = c.hscale = c.eta = 1.0;
   c.acnrm = c.rl1 = c.saved_t = c.delp = c.hg = c.hub = c.hlb = 0.0;
   c.ncf = c.nef = c.nflag = c.convfail = c.callSetup = c.jbad = c.mnewt = c.attempt = 0;
   c.count1 = c.hnewOK = c.nstloc = c.setup_conv = c.setup_ier = 0;

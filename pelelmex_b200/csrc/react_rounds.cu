@@ -295,8 +295,8 @@ __device__ __forceinline__ void step_cell(const RoundsParams& R, bool live, int 
         c.refine_ratio = ratio;
         if (step) {
 #define B200_ST(f) c.f = o.f;
-          B200_ST(h) B200_ST(hprime) B200_ST(hscale) B200_ST(eta) B200_ST(etamax) B200_ST(tn) B200_ST(gamma)
-          B200_ST(gamrat) B200_ST(rl1) B200_ST(saved_tq5) B200_ST(saved_t) B200_ST(q) B200_ST(qprime) B200_ST(L)
+          B200_ST(h) B200_ST(hscale) B200_ST(eta) B200_ST(etamax) B200_ST(tn) B200_ST(gamma)
+          B200_ST(gamrat) B200_ST(rl1) B200_ST(saved_tq5) B200_ST(saved_t) B200_ST(q) B200_ST(L)
           B200_ST(qwait) B200_ST(nstlj) B200_ST(jcur) B200_ST(ncf) B200_ST(nef) B200_ST(nflag) B200_ST(convfail)
           B200_ST(callSetup) B200_ST(jbad) B200_ST(attempt) B200_ST(nstloc) B200_ST(setup_conv) B200_ST(label)
           B200_ST(cnt.nst) B200_ST(cnt.nje)
