@@ -299,7 +299,8 @@ int64_t b200chem_kernel_launches(b200chem_handle h);
  * shape at compile time.  Zero fields take the defaults. */
 typedef struct b200chem_tuning {
   int32_t rhs_ctas_per_sm;   /* CTAs per SM of the right-hand-side kernel (0: as many as fit) */
-  int32_t ctrl_ctas_per_sm;  /* ... of the step-control / Newton kernel                      */
+  int32_t ctrl_ctas_per_sm;  /* ... of the step kernel (Newton) and of the control kernel,
+                              * of which 2 to 4 and 3 fit                                    */
   int32_t jac_ctas_per_sm;   /* ... of the Jacobian kernel                                   */
   int32_t gj_ctas_per_sm;    /* ... of the iteration-matrix inversion kernel                 */
   int32_t rounds_per_check;  /* rounds between two reads of the live-cell count: 2, 4, 8

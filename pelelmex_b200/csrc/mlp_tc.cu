@@ -900,8 +900,8 @@ extern "C" int b200chem_mlp_gemm_bf16(const void* A, long long lda, const void* 
   }
   if (arep != 1) return -1;  // two-term A operands need the warp-specialised kernel
   // Split K where the tiles would leave most SMs idle: 16 chunks of K and more
-  // (each of the cluster's CTAs gets at least two) with fewer 128 x 256 tiles
-  // than half the SMs.
+  // (two for each of the cluster's CTAs; the ranges are rounded up, so that the
+  // last CTAs may have fewer or none) with fewer 128 x 256 tiles than half the SMs.
   if (epi == kEpiF32 && !resident && K % kSplitKC == 0 && K >= 2 * kSplit * kSplitKC &&
       2 * (M / kTileM) * ((N + 255) / 256) < sms) {
     const int nt = split_nt(N), ssm = split_smem(nt);

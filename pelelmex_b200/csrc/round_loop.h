@@ -7,9 +7,12 @@ namespace b200 {
 // Launch shapes of a round by how many cells are live: many (kernels in a row,
 // right-hand sides by thread), fewer (setup kernels on a branch), few
 // (right-hand sides by warp as well), and so few that the grids shrink to them.
-// The branch pays up to 131072 cells (32^3 H2: 4.56 ms, 5.03 without it above
-// the warp form's 9472 cells; 61x43x37 CH4: 44.3 and 45.8) and costs 10 % with
-// two million, whose kernels contend for L2.
+// With the branch against without it, ms a react: 32^3 H2 4.56 and 5.03, 61x43x37
+// CH4 44.3 and 45.8; above the line 64^3 H2 23.2 and 26.2, 64^3 CH4 54.2 and 55.8,
+// 80^3 CH4 96.7 and 99.4, 80^3 dodecane 391 and 392, 96^3 H2 72.9 and 74.1, 96^3
+// CH4 160.6 and 163.1; 128^3 CH4 445 and 408, where the kernels contend for L2.  So
+// the two cross between one and two million cells, and the line lies at the
+// largest size that was measured when it was drawn.
 constexpr int kRoundClasses = 4;
 constexpr int kForkCells = 131072;
 constexpr int kTinyCells = 1024;

@@ -1,5 +1,5 @@
 """GEMMs with few tiles and a long K (the weight gradients), which a cluster of
-CTAs shares: edges of the K ranges (fewer chunks than an even split, a last CTA
+CTAs shares: edges of the K ranges (fewer chunks than an even split, last CTAs
 without any), N tiles of 16 to 64, partial output columns, the same bits twice."""
 import pytest
 
@@ -11,8 +11,8 @@ from pelelmex_b200.surrogate import gemm  # noqa: E402
 DEV = "cuda:0"
 
 
-# K = 1024: 2 chunks of 64 for each of 8 CTAs; 1088: 17 chunks, so 3 each and
-# the last two CTAs get 2 and none; 16384: the training batch
+# K = 1024: 2 chunks of 64 for each of 8 CTAs; 1088: 17 chunks, so 3 for the
+# first five, 2 for the sixth and none for the last two; 16384: the training batch
 @pytest.mark.parametrize("M,N,K,n_valid", [(128, 16, 1024, 0), (256, 32, 1088, 22), (128, 48, 1216, 0),
                                            (256, 256, 1024, 0), (256, 80, 2112, 70), (256, 512, 4096, 0),
                                            (256, 256, 16384, 0), (128, 256, 16384, 255)])
