@@ -41,7 +41,7 @@ __global__ void __launch_bounds__(kRoundsRhsBlock, rhs_min_ctas(NS)) rk_rhs_gen(
 
 // Mass production rates at (rhoY, T), one thread per cell.
 template <int NS>
-__global__ void __launch_bounds__(kRoundsRhsBlock, rhs_min_ctas(NS)) rk_rates(const __grid_constant__ DevMech m, InstView<NS> v, const double* __restrict__ T) {
+__global__ void __launch_bounds__(kRoundsRhsBlock, rhs_min_ctas(NS)) rk_rates(const __grid_constant__ DevMech m, InstView<NS> v) {
   extern __shared__ __align__(16) unsigned char dsm[];
   double* sd = reinterpret_cast<double*>(dsm);
   const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
@@ -50,7 +50,6 @@ __global__ void __launch_bounds__(kRoundsRhsBlock, rhs_min_ctas(NS)) rk_rates(co
   for (v.c = t0; v.c < v.n; v.c += nt) {
     double y[NS + 1], f[NS + 1];
     const double F[NS + 1] = {};
-    v.t = T[v.c];
 #pragma unroll
     for (int k = 0; k <= NS; ++k) y[k] = v.yev(k);
     if (!gen_covers<NS>(y[NS])) cold_inst<NS>(&m, y, f);
@@ -88,7 +87,7 @@ cudaError_t rates_t(const DevMech& m, const double* rhoY, const double* T, doubl
                     cudaStream_t st) {
   const long long need = (ncells + kRoundsRhsBlock - 1) / kRoundsRhsBlock;
   rk_rates<NS><<<(int)std::min<long long>(need, grid), kRoundsRhsBlock, gen_smem<NS>(), st>>>(
-      m, InstView<NS>{rhoY, dot, ncells, 0, 0.0}, T);
+      m, InstView<NS>{rhoY, T, dot, ncells, 0});
   return cudaGetLastError();
 }
 

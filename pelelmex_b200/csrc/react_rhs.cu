@@ -336,104 +336,99 @@ __global__ void __launch_bounds__(kRhsWarpBlock, 8) rk_rhs_warp(RoundsParams R) 
   }
 }
 
-// T from (h, Y) by Newton on h(T) = sum Y_k h_k(T) from the given T (MKS;
-// getTfromHY of the C ABI), one thread per cell, or one warp that solves the
-// rates of the cell as well; both give the same bits.
-template <int NS>
-__device__ __forceinline__ void cp_h(const DevMech& m, int k, double t, double invT, double& cp, double& h) {
-  const double* a = m.nasa + (t < __ldg(m.nasa + k) ? 1 : 8) * NS + k;
-  const double a0 = __ldg(a), a1 = __ldg(a + NS), a2 = __ldg(a + 2 * NS), a3 = __ldg(a + 3 * NS), a4 = __ldg(a + 4 * NS);
-  cp = gen::nasa_cp(a0, a1, a2, a3, a4, t);
-  h = gen::nasa_h(a0, __dmul_rn(a1, 0.5), __dmul_rn(a2, 1.0 / 3.0), __dmul_rn(a3, 0.25), __dmul_rn(a4, 0.2),
-                  __ldg(a + 5 * NS), t, invT);
-}
-
-// Newton iteration from t; sums(t, invT, hs, cs) gives sum w h/R(T) / T and sum
-// w cp/R, w = rhoY / W; H = rhoH in erg/g kg/m^3, over Ru.
-template <class Sums>
-__device__ __forceinline__ double newton_t(double t, double H, Sums sums) {
-  for (int it = 0; it < 100; ++it) {
-    double hs = 0.0, cs = 0.0;
-    sums(t, 1.0 / t, hs, cs);
-    const double dT = fma(-hs, t, H) / cs;
-    t = __dadd_rn(t, dT);
-    if (fabs(dT) <= 1e-12 * t) break;
-  }
-  return t;
-}
-constexpr double kHScale = 1.0e4 / kRu;  // J/m^3 -> erg/g kg/m^3, over Ru
-
+// T from (h, Y) by Newton on h(T) = sum Y_k h_k(T) from the given T, one
+// thread per cell (MKS, component-major; getTfromHY of the C ABI).
 template <int NS>
 __global__ void __launch_bounds__(128) rk_t_from_hy(DevMech m, const double* __restrict__ rhoY,
                                                     const double* __restrict__ rhoH, double* __restrict__ T,
                                                     long long ncells) {
   for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < ncells;
        c += (long long)gridDim.x * blockDim.x) {
-    double w[NS], rho = 0.0;
+    double w[NS];
 #pragma unroll
-    for (int k = 0; k < NS; ++k) {
-      const double y = rhoY[(long long)k * ncells + c];
-      rho += y;
-      w[k] = __dmul_rn(y, __ldg(m.inv_mw + k));
+    for (int k = 0; k < NS; ++k) w[k] = rhoY[(long long)k * ncells + c] * __ldg(m.inv_mw + k);
+    const double h = rhoH[c] * (1.0e4 / kRu);  // J/m^3 -> erg/g kg/m^3, over Ru
+    double t = T[c];
+    for (int it = 0; it < 100; ++it) {
+      const double invT = 1.0 / t;
+      double hs = 0.0, cs = 0.0;
+#pragma unroll
+      for (int k = 0; k < NS; ++k) {
+        const double* a = m.nasa + (t < __ldg(m.nasa + k) ? 1 : 8) * NS + k;
+        const double a0 = __ldg(a), a1 = __ldg(a + NS), a2 = __ldg(a + 2 * NS), a3 = __ldg(a + 3 * NS),
+                     a4 = __ldg(a + 4 * NS);
+        cs += w[k] * (a0 + t * (a1 + t * (a2 + t * (a3 + t * a4))));
+        hs += w[k] * (a0 + t * (a1 * 0.5 + t * (a2 * (1.0 / 3.0) + t * (a3 * 0.25 + t * (a4 * 0.2)))) +
+                      __ldg(a + 5 * NS) * invT);
+      }
+      const double dT = (h - hs * t) / cs;
+      t += dT;
+      // a cell without mass (a covered one, say) has no temperature: its infinite
+      // step is not a converged one, and the next is NaN, which ends the loop
+      if (!(fabs(dT) >= 1e-12 * t)) break;
     }
-    // an empty cell (covered, say) has no temperature
-    T[c] = newton_t(rho == 0.0 ? nan("") : T[c], __dmul_rn(rhoH[c], kHScale),
-                    [&](double t, double invT, double& hs, double& cs) {
-#pragma unroll
-                      for (int k = 0; k < NS; ++k) {
-                        double cp, h;
-                        cp_h<NS>(m, k, t, invT, cp, h);
-                        cs = fma(w[k], cp, cs);
-                        hs = fma(w[k], h, hs);
-                      }
-                    });
+    T[c] = t;
   }
 }
 
-// T of cell c by a warp, lane per species; sums run in species order on every
-// lane, as the thread form adds them.  s: 3 NS doubles of the warp's shared memory.
+// The same by a warp, lane per species; sums run in species order on every lane,
+// as the thread form adds them.  s: 3 NS doubles of the warp's shared memory.
 template <int NS>
 __device__ __forceinline__ double t_warp(const DevMech& m, const InstView<NS>& v, const double* rhoH, double* s, int lane) {
   double *sw = s, *sc = s + NS, *sh = s + 2 * NS;
-  for (int k = lane; k < NS; k += 32) {
-    const double y = v.rhoY[(long long)k * v.n + v.c];
-    sw[k] = __dmul_rn(y, __ldg(m.inv_mw + k));
-    sc[k] = y;
-  }
-  __syncwarp();
-  double rho = 0.0;
-#pragma unroll 9
-  for (int k = 0; k < NS; ++k) rho += sc[k];
-  __syncwarp();
-  return newton_t(rho == 0.0 ? nan("") : v.t, __dmul_rn(rhoH[v.c], kHScale), [&](double t, double invT, double& hs, double& cs) {
-    for (int k = lane; k < NS; k += 32) cp_h<NS>(m, k, t, invT, sc[k], sh[k]);
-    __syncwarp();
-#pragma unroll 9
-    for (int k = 0; k < NS; ++k) {
-      cs = fma(sw[k], sc[k], cs);
-      hs = fma(sw[k], sh[k], hs);
+  for (int k = lane; k < NS; k += 32) sw[k] = v.rhoY[(long long)k * v.n + v.c] * __ldg(m.inv_mw + k);
+  const double h = rhoH[v.c] * (1.0e4 / kRu);
+  double t = v.T[v.c];
+  for (int it = 0; it < 100; ++it) {
+    const double invT = 1.0 / t;
+    for (int k = lane; k < NS; k += 32) {
+      const double* a = m.nasa + (t < __ldg(m.nasa + k) ? 1 : 8) * NS + k;
+      const double a0 = __ldg(a), a1 = __ldg(a + NS), a2 = __ldg(a + 2 * NS), a3 = __ldg(a + 3 * NS),
+                   a4 = __ldg(a + 4 * NS);
+      sc[k] = a0 + t * (a1 + t * (a2 + t * (a3 + t * a4)));
+      sh[k] = a0 + t * (a1 * 0.5 + t * (a2 * (1.0 / 3.0) + t * (a3 * 0.25 + t * (a4 * 0.2)))) + __ldg(a + 5 * NS) * invT;
     }
     __syncwarp();
-  });
+    double hs = 0.0, cs = 0.0;
+#pragma unroll 9
+    for (int k = 0; k < NS; ++k) {
+      cs += sw[k] * sc[k];
+      hs += sw[k] * sh[k];
+    }
+    __syncwarp();
+    const double dT = (h - hs * t) / cs;
+    t += dT;
+    if (!(fabs(dT) >= 1e-12 * t)) break;
+  }
+  return t;
 }
+
+// InstView of the warp form, which has its T at hand.
+template <int NS>
+struct InstViewT : InstView<NS> {
+  double t;
+  __device__ __forceinline__ double yev(int k) const { return k < NS ? InstView<NS>::yev(k) : t; }
+};
 
 // Mass production rates at (rhoY, T) with the generated right-hand side
 // (reactionRateRhoY of the C ABI): one thread per cell, and for few cells one
 // warp per cell with the same bits, which solves for T first when rhoH is given.
 // dot = nullptr: T only.
 template <int NS>
-__global__ void __launch_bounds__(kRhsWarpBlock, 8) rk_rates_warp(DevMech m, InstView<NS> v, const double* rhoH, double* T) {
+__global__ void __launch_bounds__(kRhsWarpBlock, 8) rk_rates_warp(DevMech m, InstView<NS> view, const double* rhoH, double* T) {
   extern __shared__ __align__(16) unsigned char dsm[];
   __shared__ DevMech s_mech;
   if (threadIdx.x == 0) s_mech = m;
   __syncthreads();
   const int lane = threadIdx.x & 31;
   double* sw = reinterpret_cast<double*>(dsm) + (threadIdx.x >> 5) * rhs_warp_doubles<NS>(s_mech.R);
+  InstViewT<NS> v{view, 0.0};
   for (v.c = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; v.c < v.n; v.c += (gridDim.x * blockDim.x) >> 5) {
-    v.t = T[v.c];
     if (rhoH) {
       v.t = t_warp<NS>(s_mech, v, rhoH, sw, lane);
       if (lane == 0) T[v.c] = v.t;
+    } else {
+      v.t = v.T[v.c];
     }
     if (!v.dot) continue;
     if (gen_covers<NS>(v.t)) {
@@ -493,15 +488,15 @@ cudaError_t rhs_launch_t(const RoundsParams& R, int grid, int by_warp, cudaStrea
 // Most cells whose T and rates one launch takes, a warp per cell: about a wave of
 // the GPU's 4736 warps for the smaller mechanisms, half of one for 53 species.  A
 // call (T and rates, host included) takes 16 / 19 / 37 us at 512 cells of 9 / 21 /
-// 53 species, 20 / 29 / 50 with T by thread in a launch of its own; 21 / 29 against
-// 23 / 35 at 4096 cells of 9 and 21, where 9000 cells of 21 species already need 21
-// against 15 us for T alone; 46 against 56 at 2048 of 53, 64 and 66 at 4096.
+// 53 species, 20 / 29 / 50 with T by thread in a launch of its own; 20 / 29 against
+// 23 / 35 at 4096 cells of 9 and 21, where T alone of 9000 cells of 21 species
+// already takes 21 against 15; 46 against 56 at 2048 of 53, 64 and 66 at 4096.
 constexpr int inst_warp_cells(int NS) { return NS <= 32 ? 4096 : 2048; }
 
 template <int NS>
 cudaError_t inst_launch_t(const DevMech& m, const double* rhoY, const double* rhoH, double* T, double* dot,
                           long long ncells, int sm_count, cudaStream_t st) {
-  const InstView<NS> v{rhoY, dot, ncells, 0, 0.0};
+  const InstView<NS> v{rhoY, T, dot, ncells, 0};
   const int smem = rhs_warp_smem<NS>(m.R), per = kRhsWarpBlock / 32;
   cudaError_t e = cudaFuncSetAttribute(rk_rates_warp<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;

@@ -152,12 +152,11 @@ __device__ __noinline__ void cold_inst(const DevMech* m, const double* y, double
 // forcing, the rate of T not wanted.
 template <int NS>
 struct InstView {
-  const double* rhoY;
+  const double *rhoY, *T;
   double* dot;
-  long long n, c;  // cells, and this one
-  double t;        // its temperature
+  long long n, c;
   __device__ __forceinline__ double yev(int k) const {
-    return k < NS ? rhoY[(long long)k * n + c] * 1.0e-3 : t;  // kg/m^3 -> g/cm^3
+    return k < NS ? rhoY[(long long)k * n + c] * 1.0e-3 : T[c];  // kg/m^3 -> g/cm^3
   }
   __device__ __forceinline__ double F(int) const { return 0.0; }
   __device__ __forceinline__ void set_f(int k, double v) const {
