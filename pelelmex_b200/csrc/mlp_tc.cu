@@ -27,6 +27,7 @@
 #include <stdint.h>
 
 #include "../../include/b200chem.h"
+#include "split_rule.h"
 
 namespace b200 {
 namespace mlp {
@@ -431,17 +432,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_bf16_tc(GemmArgs g) {
 // and adds the partial sums through distributed shared memory in rank order
 // (the same bits every time); NT is at most 64, so the 256 x 256 case runs on
 // 64 SMs.  FP32 output without activation.
-constexpr int kSplit = 8;
-constexpr int kSplitStages = 4;
-constexpr int kSplitKC = 64;
-
-// N tile: the largest multiple of 16 up to 64 that divides N.
-inline int split_nt(int N) {
-  for (int nt = 64; nt > 16; nt -= 16)
-    if (N % nt == 0) return nt;
-  return 16;
-}
-inline int split_smem(int NT) { return kSplitStages * (kTileM + NT) * kSplitKC * 2; }
+static_assert(kSplitTileM == kTileM, "one tile height");
 
 __global__ void __cluster_dims__(kSplit, 1, 1) __launch_bounds__(kThreads) gemm_bf16_splitk(GemmArgs g, int NT) {
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -899,11 +890,7 @@ extern "C" int b200chem_mlp_gemm_bf16(const void* A, long long lda, const void* 
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
   }
   if (arep != 1) return -1;  // two-term A operands need the warp-specialised kernel
-  // Split K where the tiles would leave most SMs idle: 16 chunks of K and more
-  // (two for each of the cluster's CTAs; the ranges are rounded up, so that the
-  // last CTAs may have fewer or none) with fewer 128 x 256 tiles than half the SMs.
-  if (epi == kEpiF32 && !resident && K % kSplitKC == 0 && K >= 2 * kSplit * kSplitKC &&
-      2 * (M / kTileM) * ((N + 255) / 256) < sms) {
+  if (epi == kEpiF32 && !resident && split_pays(M, N, K, sms)) {
     const int nt = split_nt(N), ssm = split_smem(nt);
     if (!allow_smem(gemm_bf16_splitk, optin)) return -2;
     gemm_bf16_splitk<<<(M / kTileM) * (N / nt) * kSplit, kThreads, ssm, st>>>(g, nt);
