@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(kRoundsRhsBlock, rhs_min_ctas(NS)) rk_rhs_gen(
   for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < cnt; idx += gridDim.x * blockDim.x) {
     const int slot = R.list_in[idx] & ~kSetupFlag;
     const RVec<n> v{reinterpret_cast<double*>(rec_of(R.S, slot) + R.S.L.off_vec)};
-    if (!gen_covers<NS>(v.yev(NS))) cold_rhs<NS>(&R.P.mech, v.b);
+    if (!gen_covers<NS>(v.yev(NS))) cold_rhs<NS>(&R.P.mech, RecView<NS>{v}, sE, sI, kRoundsRhsBlock, &v.fv(0), 1);
     else if constexpr (NS == 9) gen::gen_rhs_synth_h2_9(&v.yev(0), &v.F(0), &v.fv(0), sE, sI, kRoundsRhsBlock);
     else if constexpr (NS == 21) gen::gen_rhs_synth_ch4_21(&v.yev(0), &v.F(0), &v.fv(0), sE, sI, kRoundsRhsBlock);
     else if constexpr (NS == 53) gen::gen_rhs_synth_c12_53(&v.yev(0), &v.F(0), &v.fv(0), sE, sI, kRoundsRhsBlock);
@@ -48,12 +48,15 @@ __global__ void __launch_bounds__(kRoundsRhsBlock, rhs_min_ctas(NS)) rk_rates(co
   double* sE = sd + threadIdx.x;
   double* sI = sE + NS * kRoundsRhsBlock;
   for (v.c = t0; v.c < v.n; v.c += nt) {
+    if (!gen_covers<NS>(v.T[v.c])) {
+      cold_rhs<NS>(&m, v, sE, sI, kRoundsRhsBlock, v.dot + v.c, v.n);
+      continue;
+    }
     double y[NS + 1], f[NS + 1];
     const double F[NS + 1] = {};
 #pragma unroll
     for (int k = 0; k <= NS; ++k) y[k] = v.yev(k);
-    if (!gen_covers<NS>(y[NS])) cold_inst<NS>(&m, y, f);
-    else if constexpr (NS == 9) gen::gen_rhs_synth_h2_9(y, F, f, sE, sI, kRoundsRhsBlock);
+    if constexpr (NS == 9) gen::gen_rhs_synth_h2_9(y, F, f, sE, sI, kRoundsRhsBlock);
     else if constexpr (NS == 21) gen::gen_rhs_synth_ch4_21(y, F, f, sE, sI, kRoundsRhsBlock);
     else if constexpr (NS == 53) gen::gen_rhs_synth_c12_53(y, F, f, sE, sI, kRoundsRhsBlock);
 #pragma unroll

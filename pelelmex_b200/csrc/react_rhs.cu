@@ -138,15 +138,6 @@ __device__ __forceinline__ void cm_rhs(const RVec<NS + 1>& v, double* sC, double
 template <int NS>
 constexpr int rhs_warp_doubles(int R) { return 5 * NS + R; }
 
-// The cell of the round integrator: its record.
-template <int NS>
-struct RecView {
-  RVec<NS + 1> v;
-  __device__ __forceinline__ double yev(int k) const { return v.yev(k); }
-  __device__ __forceinline__ double F(int k) const { return v.F(k); }
-  __device__ __forceinline__ void set_f(int k, double x) const { v.fv(k) = x; }
-};
-
 // The generated right-hand side's arithmetic (mechgen.generate), one warp per
 // cell from the tables: lane per species, then per reaction, then per species;
 // sums over species run in species order on every lane, as the generated code
@@ -307,7 +298,7 @@ __global__ void __launch_bounds__(kRoundsRhsBlock, 6) rk_rhs(RoundsParams R) {
     const int slot = R.list_in[idx] & ~kSetupFlag;
     const RVec<n> v{reinterpret_cast<double*>(rec_of(R.S, slot) + R.S.L.off_vec)};
     if (R.const_mech) cm_rhs<NS>(v, sC, sG, sW, blockDim.x);
-    else r_rhs<NS>(s_mech, v, sC, sG, sW, blockDim.x);
+    else r_rhs<NS>(s_mech, RecView<NS>{v}, sC, sG, (int)blockDim.x, sW, (int)blockDim.x);
   }
 }
 
@@ -331,8 +322,12 @@ __global__ void __launch_bounds__(kRhsWarpBlock, 8) rk_rhs_warp(RoundsParams R) 
   for (int idx = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; idx < cnt; idx += nw) {
     const int slot = R.list_in[idx] & ~kSetupFlag;
     const RVec<n> v{reinterpret_cast<double*>(rec_of(R.S, slot) + R.S.L.off_vec)};
-    if (gen_covers<NS>(v.yev(NS))) rhs_warp<NS>(s_mech, RecView<NS>{v}, sw, lane);
-    else if (lane == 0) cold_rhs<NS>(&s_mech, v.b);
+    if (gen_covers<NS>(v.yev(NS))) {
+      rhs_warp<NS>(s_mech, RecView<NS>{v}, sw, lane);
+    } else {
+      if (lane == 0) cold_rhs<NS>(&s_mech, RecView<NS>{v}, sw, sw + NS, 1, sw + 2 * NS, 1);
+      __syncwarp();
+    }
   }
 }
 
@@ -433,13 +428,10 @@ __global__ void __launch_bounds__(kRhsWarpBlock, 8) rk_rates_warp(DevMech m, Ins
     if (!v.dot) continue;
     if (gen_covers<NS>(v.t)) {
       rhs_warp<NS>(s_mech, v, sw, lane);
-    } else if (lane == 0) {
-      double y[NS + 1], f[NS + 1];
-      for (int k = 0; k <= NS; ++k) y[k] = v.yev(k);
-      cold_inst<NS>(&s_mech, y, f);
-      for (int k = 0; k < NS; ++k) v.set_f(k, f[k]);
+    } else {
+      if (lane == 0) cold_rhs<NS>(&s_mech, v, sw, sw + NS, 1, sw + 2 * NS, 1);
+      __syncwarp();
     }
-    __syncwarp();
   }
 }
 

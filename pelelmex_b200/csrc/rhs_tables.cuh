@@ -75,10 +75,20 @@ __device__ __forceinline__ double r_progress(const DevMech& m, int j, double T, 
   return q;
 }
 
-// HP right-hand side at v.yev (forcing v.F) into v.fv, thread per cell.
+// The cell of the round integrator: its record.
 template <int NS>
-__device__ __forceinline__ void r_rhs(const DevMech& m, const RVec<NS + 1>& v, double* sC, double* sG, double* sW,
-                                      int ss) {
+struct RecView {
+  RVec<NS + 1> v;
+  __device__ __forceinline__ double yev(int k) const { return v.yev(k); }
+  __device__ __forceinline__ double F(int k) const { return v.F(k); }
+  __device__ __forceinline__ void set_f(int k, double x) const { v.fv(k) = x; }
+};
+
+// HP right-hand side at v.yev (forcing v.F) into v.set_f, thread per cell.  sC,
+// sG: scratch of stride ss; sW of stride ws, which may be where set_f writes.
+template <int NS, class View, class Stride>
+__device__ __forceinline__ void r_rhs(const DevMech& m, const View& v, double* sC, double* sG, int ss, double* sW,
+                                      Stride ws) {
   const double T = v.yev(NS);
   const double lnT = log(T), invT = 1.0 / T;
   double Ctot = 0.0, rcp = 0.0;
@@ -91,7 +101,7 @@ __device__ __forceinline__ void r_rhs(const DevMech& m, const RVec<NS + 1>& v, d
     const double Ck = yk * iw;
     sC[k * ss] = Ck;
     sG[k * ss] = hRT - sR;
-    sW[k * ss] = 0.0;
+    sW[k * ws] = 0.0;
     Ctot += Ck;
     rcp += yk * cpR * kRu * iw;
   }
@@ -104,7 +114,7 @@ __device__ __forceinline__ void r_rhs(const DevMech& m, const RVec<NS + 1>& v, d
     for (int sl = 0; sl < 8; ++sl) {
       const int k = __ldg(m.sp + sl * R + j);
       if (k >= 0) {
-        sW[k * ss] += (double)__ldg(m.nu + sl * R + j) * q;
+        sW[k * ws] += (double)__ldg(m.nu + sl * R + j) * q;
       }
     }
   }
@@ -113,19 +123,20 @@ __device__ __forceinline__ void r_rhs(const DevMech& m, const RVec<NS + 1>& v, d
   for (int k = 0; k < NS; ++k) {
     double cpR, hRT, sR, dcpR;
     nasa7(m, k, T, lnT, cpR, hRT, sR, dcpR);
-    const double yd = sW[k * ss] * __ldg(m.mw + k) + v.F(k);
-    v.fv(k) = yd;
+    const double yd = sW[k * ws] * __ldg(m.mw + k) + v.F(k);
+    v.set_f(k, yd);
     hs += hRT * kRu * T * __ldg(m.inv_mw + k) * yd;
   }
-  v.fv(NS) = (v.F(NS) - hs) / rcp;
+  v.set_f(NS, (v.F(NS) - hs) / rcp);
 }
 
-// Right-hand side of a cell outside the generated code's temperatures (never
-// in a healthy integration): the table form in one thread's local memory.
-template <int NS>
-__device__ __noinline__ void cold_rhs(const DevMech* m, double* b) {
-  double sC[NS], sG[NS], sW[NS];
-  r_rhs<NS>(*m, RVec<NS + 1>{b}, sC, sG, sW, 1);
+// Right-hand side of a cell outside the generated code's temperatures (never in a
+// healthy integration): the table form, out of line and in the caller's scratch,
+// because an array of its own would be local memory for every thread the GPU can
+// hold (1.2 GB with 53 species).
+template <int NS, class View>
+__device__ __noinline__ void cold_rhs(const DevMech* m, View v, double* sC, double* sG, int ss, double* sW, long long ws) {
+  r_rhs<NS>(*m, v, sC, sG, ss, sW, ws);
 }
 
 template <int NS>
@@ -133,19 +144,6 @@ __device__ __forceinline__ bool gen_covers(double T) {
   if constexpr (NS == 9) return T >= gen::kGenTlo_synth_h2_9 && T <= gen::kGenThi_synth_h2_9;
   else if constexpr (NS == 21) return T >= gen::kGenTlo_synth_ch4_21 && T <= gen::kGenThi_synth_ch4_21;
   else return T >= gen::kGenTlo_synth_c12_53 && T <= gen::kGenThi_synth_c12_53;
-}
-
-// The rates of one cell outside the generated code's temperatures.
-template <int NS>
-__device__ __noinline__ void cold_inst(const DevMech* m, const double* y, double* f) {
-  double b[kVecs * (NS + 1)];
-  const RVec<NS + 1> v{b};
-  for (int k = 0; k <= NS; ++k) {
-    v.yev(k) = y[k];
-    v.F(k) = 0.0;
-  }
-  cold_rhs<NS>(m, b);
-  for (int k = 0; k <= NS; ++k) f[k] = v.fv(k);
 }
 
 // The cell of the rates kernels: MKS state in component-major arrays, no
