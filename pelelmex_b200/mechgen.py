@@ -91,9 +91,9 @@ def temperature_range(flat) -> tuple:
         return bool(ok)
 
     lo, hi = 1000.0, 1000.0
-    while lo > 150.0 and fine(lo - 5.0):
+    while lo > 50.0 and fine(lo - 5.0):
         lo -= 5.0
-    while hi < 8000.0 and fine(hi + 50.0):
+    while hi < 20000.0 and fine(hi + 50.0):
         hi += 50.0
     return lo, hi
 
