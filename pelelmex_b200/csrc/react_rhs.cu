@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(kRhsWarpBlock, 8) rk_rhs_warp(RoundsParams R) 
     if (gen_covers<NS>(v.yev(NS))) {
       rhs_warp<NS>(s_mech, RecView<NS>{v}, sw, lane);
     } else {
-      if (lane == 0) cold_rhs<NS>(&s_mech, RecView<NS>{v}, sw, sw + NS, 1, sw + 2 * NS, 1);
+      if (lane == 0) cold_rhs_lane<NS>(&s_mech, v.b, sw);
       __syncwarp();
     }
   }

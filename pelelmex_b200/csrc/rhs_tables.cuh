@@ -138,6 +138,13 @@ template <int NS, class View>
 __device__ __noinline__ void cold_rhs(const DevMech* m, View v, double* sC, double* sG, int ss, double* sW, long long ws) {
   r_rhs<NS>(*m, v, sC, sG, ss, sW, ws);
 }
+// The same for a record (vectors at b) by one lane of the warp form, in its scratch
+// s.  Few arguments: with those of the other the loop around the call spills (20^3
+// dodecane flame: 54.8 ms in right-hand sides, 52.7 so).
+template <int NS>
+__device__ __noinline__ void cold_rhs_lane(const DevMech* m, double* b, double* s) {
+  r_rhs<NS>(*m, RecView<NS>{{b}}, s, s + NS, 1, s + 2 * NS, 1);
+}
 
 template <int NS>
 __device__ __forceinline__ bool gen_covers(double T) {
