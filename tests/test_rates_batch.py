@@ -18,9 +18,11 @@ from test_round_kernels import _field  # noqa: E402
                                           ("synth_c12_53", 2048, 40000)])
 def test_cell_is_independent_of_its_batch(name, lim, big):
     f = _field(name, big)
-    T = np.resize(np.array([0.9, 1.0, 1.1]), big) * f.T  # first guess; the ends of the generated code's temperatures too
-    T[:8] = [120.0, 179.0, 181.0, 999.9, 1000.1, 7990.0, 8100.0, 300.0]
-    rhoH = f.rhoY.sum(axis=0) * M.mix_h_mass(M.builtin(name), np.where(np.arange(big) < 8, T, f.T), (f.rhoY / f.rhoY.sum(axis=0)).T)
+    T = np.resize(np.array([0.9, 1.0, 1.1]), big) * f.T  # first guess
+    ends = np.array([60.0, 94.0, 96.0, 139.0, 141.0, 179.0, 181.0, 12500.0, 12600.0, 17300.0, 17400.0, 17850.0, 18000.0])
+    T[:ends.size] = ends  # around the ends of the generated code's temperatures
+    state = np.where(np.arange(big) < ends.size, T, f.T)
+    rhoH = f.rhoY.sum(axis=0) * M.mix_h_mass(M.builtin(name), state, (f.rhoY / f.rhoY.sum(axis=0)).T)
     r = ReactorB200(name).init()
     ref = {}
     for n in (big, lim + 1, lim, 33, 1):

@@ -1,7 +1,7 @@
 """The round integrator's kernels where their forms meet: right-hand sides by
 warp and by thread (chosen by how many cells are live) give the same bits, so a
 cell's result does not depend on what is integrated with it; the generated
-rates at the ends of their temperature range; and the work counters of the
+rates over a wide range of temperatures; and the work counters of the
 dense-direct BDF, which a wrong Jacobian or inverse would change first."""
 import numpy as np
 import pytest
@@ -41,9 +41,10 @@ def test_result_of_a_cell_is_independent_of_its_batch(name, big, small):
 @pytest.mark.parametrize("name", ["synth_h2_9", "synth_ch4_21", "synth_c12_53"])
 @pytest.mark.parametrize("n", [9, 40000])
 def test_generated_rates_over_their_temperatures(name, n, orc_cache):
-    """Rates around the NASA midpoint, at and beyond both ends of the generated
-    code's temperatures (the table form takes over there), by warp and by thread,
-    against the oracle: sums of R products of 64-bit terms, 1e-11 of the largest."""
+    """Rates around the NASA midpoint and from 120 to 8100 K (the table form takes
+    over at 120 K with 21 and 53 species; the ends of the generated code's range:
+    test_generated_range.py), by warp and by thread, against the oracle: sums of R
+    products of 64-bit terms, 1e-11 of the largest."""
     f = _field(name, n)
     mech = M.builtin(name)
     T = np.resize(np.array([120.0, 179.0, 181.0, 300.0, 999.9, 1000.0, 1000.1, 3500.0, 7990.0, 8100.0]), n)
